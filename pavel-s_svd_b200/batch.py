@@ -197,14 +197,16 @@ class UnevenBatch:
                                            self.launch_choice.flags, int(xt))
         self.workspace = torch.empty(max(int(ws), 256), dtype=torch.uint8, device=dev)
         # Persistent kernels per solve (after a memset of the work tickets): one
-        # per precision phase, two when the register path splits the batch
-        # into size classes (widths above and up to 32 columns run in CTAs of
-        # different sizes; the library does this for batches wider than 32
-        # that fit the register tiles: max(m, n) <= 128, min(m, n) <= 64).
+        # per precision phase; on the register path (max(m, n) <= 128, min(m, n)
+        # <= 64) a mixed solve takes four (precondition, refine, and the FP32
+        # and FP64 register kernels for what these leave), an FP32 one two when
+        # the batch is wider than 32 (widths above and up to 32 columns run in
+        # CTAs of different sizes).
         phases = 2 if self.precision == N.PREC_MIXED else 1
-        split = (not self.launch_choice.flags & (N.ROUND_ROBIN | N.BLOCK_WIDTH_8) and self.max_m <= 128
-                 and 32 < self.max_n <= 64)
-        self.kernels_per_solve = phases * (2 if split else 1)
+        register = (not self.launch_choice.flags & (N.ROUND_ROBIN | N.BLOCK_WIDTH_8) and self.max_m <= 128
+                    and self.max_n <= 64)
+        split = self.max_n > 32 and not self.launch_choice.flags & N.ONE_SIZE_CLASS
+        self.kernels_per_solve = phases * (2 if register and (phases == 2 or split) else 1)
 
     # -- solving ----------------------------------------------------------------
     def launch(self, a_flat: torch.Tensor, stream=None):

@@ -102,6 +102,8 @@ struct Params {
     int xchg;                     // register FP32 kernels: tile exchange area (tile_x) ...
     size_t xchg_off;              // ... at this byte offset in the work area (after W / V; it may share the
                                   //     warm-start staging of A, which is dead once the sweeps start)
+    int *n_pending;               // mixed solve: matrices the refinement left (jb_mixed.cuh)
+    int pending;                  // register kernels: solve only those
 };
 
 __device__ inline jb_matrix_desc desc_of(const Params &p, int64_t mat) {
@@ -492,6 +494,10 @@ __device__ __forceinline__ bool unpack_handoff(int w, int &ns, int &e) {
     return true;
 }
 
+}  // namespace jb
+#include "jb_mixed.cuh"
+namespace jb {
+
 // K1: FP32 sweeps.  MIXED: store the FP32 V (nt x nt) in the scratch for K2;
 // else run the epilogue and write U, S, Vh.  THREADS / MR / MRV: the CTA size
 // and the register tile (rows per lane of W and V); rb32_kernel is the
@@ -504,6 +510,7 @@ __global__ void __launch_bounds__(THREADS, (BW == kB32 && MR <= kMaxR) ? 512 / T
     Aux ax = carve_aux(smem, p.maxd);
     unsigned char *region = smem + aux_bytes(p.maxd);
     float *xbuf = p.xchg ? (float *)(region + p.xchg_off) : nullptr;   // tile exchange area
+    if (p.pending && *p.n_pending == 0) return;
     for (;;) {
         int64_t idx;
         next_ticket(p.counter, s_idx, idx);
@@ -511,6 +518,7 @@ __global__ void __launch_bounds__(THREADS, (BW == kB32 && MR <= kMaxR) ? 512 / T
         const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
         const jb_matrix_desc d = desc_of(p, mat);
         if (!class_takes(d, p.cls)) continue;  // the other size class's launch solves it
+        if (p.pending && p.status[mat] != kPending) continue;
         if (threadIdx.x < 4) ax.flag[threadIdx.x] = 0;
         __syncthreads();
         int ns = 0, st = JB_ST_OK, e_in = 0;
@@ -580,7 +588,7 @@ __global__ void __launch_bounds__(THREADS, (BW == kB32 && MR <= kMaxR) ? 512 / T
             }
         }
         if (threadIdx.x == 0) {
-            if (p.status) p.status[mat] = st;
+            if (p.status) p.status[mat] = p.pending && st == JB_ST_OK ? kHanded : st;
             // Mixed, register tiles: the FP64 phase (rb64_kernel) takes over a
             // matrix this launch solved; the sweeps word then also carries the
             // input's scale exponent, so that rb64 need not scan the input again.
@@ -604,6 +612,7 @@ __global__ void __launch_bounds__(THREADS, kT64 / THREADS) rb64_kernel(Params p)
     __shared__ int s_idx;
     Aux ax = carve_aux(smem, p.maxd);
     unsigned char *region = smem + aux_bytes(p.maxd);
+    if (p.pending && *p.n_pending == 0) return;
     for (;;) {
         int64_t idx;
         next_ticket(MIXED ? p.counter2 : p.counter, s_idx, idx);
@@ -621,7 +630,7 @@ __global__ void __launch_bounds__(THREADS, kT64 / THREADS) rb64_kernel(Params p)
         __syncthreads();
         if (threadIdx.x == 0) ax.flag[2] = 0;
         __syncthreads();
-        if (prev != JB_ST_OK) continue;  // K1 already reported this matrix
+        if (prev != (p.pending ? kHanded : JB_ST_OK)) continue;  // already reported
         int ns = s1, st = JB_ST_OK;
         if (!rdesc_fits(d, kB64, 8, p, MIXED)) {
             st = JB_ST_BAD_DESC;
@@ -1084,10 +1093,32 @@ static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsign
     }
     // Shapes are known on the host only for a uniform batch, whose matrices
     // share one class: the split applies to descriptor (uneven) batches.
-    const bool split = pl.split && p.descs != nullptr;
-    if (cudaMemsetAsync(ws, 0, 4 * sizeof(int), st) != cudaSuccess) return JB_ECUDA;
+    bool split = pl.split && p.descs != nullptr;
+    if (cudaMemsetAsync(ws, 0, 8 * sizeof(int), st) != cudaSuccess) return JB_ECUDA;
     int64_t grid;
     int rc;
+    // Mixed solve: precondition and refine; the register kernels below then
+    // take what these left (usually nothing: they read one word and return).
+    // Not with a warm start or another block width, which are choices of the
+    // register kernels, nor for full bases, which the refinement does not
+    // complete.
+    if (mixed && !p.vstart && pl.bw == kB32 &&
+        (p.descs || !(p.uflags & JB_FULL_MATRICES) || p.um == p.un)) {
+        p.n_pending = (int *)ws + 4;
+        p.maxd = pl.d32;
+        p.region_cap = pl.reg32;
+        const size_t s1 = pre_smem(pl.d.mt, pl.d.nt), s2 = ref_smem(pl.d.mt, pl.d.nt);
+        if ((rc = occupancy_grid(precondition_kernel, kPreT, s1, p.count, grid))) return rc;
+        precondition_kernel<<<(unsigned)grid, kPreT, s1, st>>>(p);
+        if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
+        if ((rc = occupancy_grid(refine_kernel, kRefT, s2, p.count, grid))) return rc;
+        refine_kernel<<<(unsigned)grid, kRefT, s2, st>>>(p);
+        if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
+        p.pending = 1;
+        p.counter = (int *)ws + 5;
+        p.counter2 = (int *)ws + 6;
+        split = false;
+    }
     if (elem == 4) {
         // block width 4: 8 warps of 256 threads for 64 columns; 8: 4 warps of 128
         auto k1 = pl.bw == 8 ? (mixed ? rb32_kernel_t<true, 128, 8, kMaxR, kMaxRV>

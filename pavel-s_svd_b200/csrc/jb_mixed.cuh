@@ -1,0 +1,884 @@
+// jb_mixed.cuh - the mixed-precision solve of float32 matrices up to 128 x 64
+// (tall view): a preconditioned FP32 Jacobi, then an FP64 refinement made of
+// matrix products.
+//
+//   precondition_kernel (64 threads a matrix)
+//     G = A^T A in FP64 (mma f64), pivoted Cholesky P^T G P = L L^T in FP64,
+//     one-sided Jacobi of L rounded to FP32.  A = Q L^T P^T, so the left
+//     singular vectors of L are the right singular vectors of A: the rotated
+//     and normalised columns are V, and no V is accumulated.  L is n x n and
+//     its columns start out graded (Veselic and Hari; Drmac and Veselic), so
+//     a sweep moves n instead of m + n rows a column and fewer sweeps are
+//     needed (128 x 64 with singular values over three decades: 7 instead of
+//     13).
+//   refine_kernel (256 threads a matrix)
+//     repeat: E = V^T V - I, W = A V from the exact input, H = W^T W (FP64);
+//     done when every pair ratio |h_pq| / sqrt(h_pp h_qq) is <= tol -- the
+//     reference's convergence test on the current W (primitives.py:334-339,
+//     352-353) -- and V is orthogonal to 1e-8; else V <- V (I + N), N = K -
+//     E / 2 with K the skew matrix of all Jacobi angles of H at once
+//     (primitives.py:340-346), which leaves the square of the errors (the
+//     refinement of Ogita and Aishima).  Usually one correction.
+//
+// Measured (B200, 8192 matrices n ~ U[8,64], m ~ U[n,2n]): 1.62 + 1.27 ms a
+// batch, against 4.55 + 3.03 ms of the register kernels' FP32 and FP64 phases
+// from V = I; 4096 x 128 x 64 over three decades 3.4 against 12.9 ms.  U is
+// also closer to LAPACK's (1.4e-7 against 1.4e-6: all pairs are corrected,
+// not only those above tol).
+//
+// A matrix that this does not suit -- numerically rank-deficient, full bases
+// wanted, no convergence within its passes -- is marked kPending and solved by
+// the launches that follow (rb32_kernel_t, rb64_kernel).
+#pragma once
+#include "jb_device.cuh"
+
+namespace jb {
+
+constexpr int kPending = -1;   // status: left to the register kernels
+constexpr int kHanded = -2;    // status: FP32 sweeps done by rb32, FP64 phase due
+constexpr int kPreT = 64, kRefT = 256;
+constexpr int kPreN = 64, kPreM = 128;
+// A pivot below kPivotCut times the largest diagonal of G (a singular value
+// ratio of about 3e-6) is left to the register kernels: FP64 rounding of G
+// no longer resolves it well enough for a start.
+constexpr double kPivotCut = 1e-11;
+constexpr int kRefPasses = 6;
+constexpr double kRefOrth = 1e-8;
+
+__host__ __device__ inline int round8(int x) { return (x + 7) & ~7; }
+// Smallest 4 * odd >= x: with it as a leading dimension in doubles (or the
+// row stride in floats) the 8 x 4 lane pattern of the f64 mma fragments hits
+// every bank once; 8 * odd does so for floats along the other index.
+__host__ __device__ inline int ld4odd(int x) { const int q = (x + 3) >> 2; return 4 * (q | 1); }
+__host__ __device__ inline int ld8odd(int x) { const int q = (x + 7) >> 3; return 8 * (q | 1); }
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+
+// The tall view of A as FP32 in shared memory, zero-padded to m8 x n8:
+// element (i, k) at i * sr + k * sk, the fast index as in the input, so that
+// reads of the input are coalesced and stores conflict-free.
+struct Stage { int sr, sk; };
+__host__ __device__ inline Stage stage_of(bool wide, int m8, int n8) {
+    return wide ? Stage{1, ld8odd(m8)} : Stage{ld4odd(n8), 1};
+}
+__host__ __device__ inline size_t stage_floats(int m8, int n8) {
+    const size_t a = (size_t)m8 * ld4odd(n8), b = (size_t)n8 * ld8odd(m8);
+    return a > b ? a : b;
+}
+template <int THREADS>
+__device__ void stage_input(const float *A, int rows, int cols, int rows8, int cols8, int ld, float *As) {
+    // input rows x cols (row-major), padded with zeros; the thread's column
+    // and row advance by a fixed step
+    const int step_r = THREADS / cols8, step_c = THREADS - step_r * cols8;
+    int r = threadIdx.x / cols8, c = threadIdx.x - r * cols8;
+    while (r < rows8) {
+        float v[8];
+        int at[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            at[u] = r < rows8 ? r * ld + c : -1;
+            v[u] = (r < rows && c < cols) ? A[(size_t)r * cols + c] : 0.f;
+            r += step_r;
+            c += step_c;
+            if (c >= cols8) { c -= cols8; ++r; }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (at[u] >= 0) As[at[u]] = v[u];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP32 Jacobi with 8 lanes a block pair: lane gl of a group owns R rows of
+// the 2B columns of its two blocks.  Compared with a whole warp a pair
+// (jb_regblock.cuh) a step's fixed cost -- the reductions, the rotation
+// parameters, the broadcasts -- is shared by four pairs of blocks a warp:
+// about 10 instead of 39 instructions a column pair at 64 rows.  Eight
+// groups hold all columns, so a matrix needs two warps.
+// ---------------------------------------------------------------------------
+constexpr int kGL = 8;
+
+template <int NV>
+__device__ __forceinline__ void group_reduce_scatter(float (&x)[NV], int lane) {
+    constexpr int L = Log2<NV>::value;
+#pragma unroll
+    for (int s = 0; s < L; ++s) {
+        const int h = NV >> (s + 1);
+        const int o = (kGL / 2) >> s;
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const float send = up ? x[k] : x[k + h];
+            const float keep = up ? x[k + h] : x[k];
+            x[k] = keep + __shfl_xor_sync(FULL, send, o);
+        }
+    }
+#pragma unroll
+    for (int o = (kGL / 2) >> L; o >= 1; o >>= 1) x[0] += __shfl_xor_sync(FULL, x[0], o);
+}
+
+template <int B, int R>
+struct GTile {
+    float w[2 * B][R];
+    float nx, ny;   // squared norms of the lane's pair (x_i, y_i), i = lane's position in the group / (8 / B)
+};
+
+template <int R>
+__device__ __forceinline__ float gdot(const float (&x)[R], const float (&y)[R]) {
+    float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+    for (int r = 0; r < R; r += 2) fma2(a0, a1, x[r], x[r + 1], y[r], y[r + 1]);
+    return a0 + a1;
+}
+template <int R>
+__device__ __forceinline__ void grot(float (&x)[R], float (&y)[R], float c, float s) {
+    const Rot2 g(c, s);
+#pragma unroll
+    for (int r = 0; r < R; r += 2) rot2(x[r], x[r + 1], y[r], y[r + 1], g);
+}
+
+// B pairs of the group's columns: INTRA pairs columns inside each block with
+// exact norms; otherwise x_i with y_i, norms kept and updated by the lanes
+// of pair i (rot_params' shift).
+template <bool INTRA, int B, int R>
+__device__ __forceinline__ void gstep(GTile<B, R> &t, float tol2, float ex2, int &fl, int lane) {
+    constexpr int LB = Log2<B>::value;
+    float pc[B];
+#pragma unroll
+    for (int i = 0; i < B; ++i) pc[i] = gdot(t.w[pair_p<INTRA, B>(i)], t.w[pair_q<INTRA, B>(i)]);
+    group_reduce_scatter(pc, lane);
+    float app, aqq;
+    if constexpr (INTRA) {
+        float pa[B], pb[B];
+#pragma unroll
+        for (int i = 0; i < B; ++i) {
+            const int p = pair_p<INTRA, B>(i), q = pair_q<INTRA, B>(i);
+            pa[i] = gdot(t.w[p], t.w[p]);
+            pb[i] = gdot(t.w[q], t.w[q]);
+        }
+        group_reduce_scatter(pa, lane);
+        group_reduce_scatter(pb, lane);
+        app = pa[0];
+        aqq = pb[0];
+    } else {
+        app = t.nx;
+        aqq = t.ny;
+    }
+    float c, s, sh;
+    const int f = rot_params<float>(app, aqq, pc[0], tol2, 0.f, ex2, 0.f, c, s, &sh);
+    fl |= f;
+    if (!__any_sync(FULL, f != 0)) return;
+    if constexpr (!INTRA) {
+        t.nx = app - sh;
+        t.ny = aqq + sh;
+    }
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+        const int src = (lane & ~(kGL - 1)) | (i << (3 - LB));
+        const float ci = __shfl_sync(FULL, c, src), si = __shfl_sync(FULL, s, src);
+        grot(t.w[pair_p<INTRA, B>(i)], t.w[pair_q<INTRA, B>(i)], ci, si);
+    }
+}
+
+template <int B, int R>
+__device__ __forceinline__ void gcircle(GTile<B, R> &t) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int o = half * B;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float last = t.w[o + B - 1][r];
+#pragma unroll
+            for (int i = B - 1; i >= 2; --i) t.w[o + i][r] = t.w[o + i - 1][r];
+            if (B > 1) t.w[o + 1][r] = last;
+        }
+    }
+}
+template <int B, int R>
+__device__ __forceinline__ void gshift_y(GTile<B, R> &t, int lane) {
+    t.ny = __shfl_sync(FULL, t.ny, (lane & ~(kGL - 1)) | ((lane + kGL / B) & (kGL - 1)));
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const float f = t.w[B][r];
+#pragma unroll
+        for (int i = 0; i < B - 1; ++i) t.w[B + i][r] = t.w[B + i + 1][r];
+        t.w[2 * B - 1][r] = f;
+    }
+}
+
+// Row of register r of lane gl: chunks of 4 (then 2) consecutive rows, chunk
+// by chunk over the lanes, so that a group's vector access to a column in the
+// exchange area is one run of 128 (64) bytes.
+template <int R>
+__device__ __forceinline__ int grow(int r, int gl) {
+    return r < (R & ~3) ? (r >> 2) * 4 * kGL + gl * 4 + (r & 3) : (R & ~3) * kGL + gl * (R & 3) + (r - (R & ~3));
+}
+template <int B, int R, bool STORE>
+__device__ __forceinline__ void gtile_x(GTile<B, R> &t, float *xw, int X, int Y, int gl) {
+#pragma unroll
+    for (int c = 0; c < 2 * B; ++c) {
+        float *col = xw + (c < B ? X * B + c : Y * B + (c - B)) * (kGL * R);
+#pragma unroll
+        for (int k = 0; k < R / 4; ++k) {
+            float4 *p = (float4 *)(col + k * 4 * kGL) + gl;
+            if (STORE) *p = make_float4(t.w[c][4 * k], t.w[c][4 * k + 1], t.w[c][4 * k + 2], t.w[c][4 * k + 3]);
+            else {
+                const float4 v = *p;
+                t.w[c][4 * k] = v.x; t.w[c][4 * k + 1] = v.y; t.w[c][4 * k + 2] = v.z; t.w[c][4 * k + 3] = v.w;
+            }
+        }
+        if (R & 2) {
+            float2 *p = (float2 *)(col + (R & ~3) * kGL) + gl;
+            if (STORE) *p = make_float2(t.w[c][R - 2], t.w[c][R - 1]);
+            else {
+                const float2 v = *p;
+                t.w[c][R - 2] = v.x; t.w[c][R - 1] = v.y;
+            }
+        }
+    }
+}
+
+// Sweeps over L (column c = G[prow[c] * ld + row], scaled by scl) until no pair
+// ratio of a sweep exceeds exit_ratio; then the normalised columns to x (n x
+// n, column-major).  G's memory becomes the exchange area.  Returns the
+// sweeps, or max_sweeps + 1.
+template <int B, int R>
+__device__ int precondition_sweeps(double *G, int ld, const int *prow, double scl, int n, float exit_ratio,
+                                   int max_sweeps, float *x) {
+    constexpr int LB = Log2<B>::value;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (kGL - 1);
+    const int group = threadIdx.x / kGL;
+    const int nb = 2 * ((n + 2 * B - 1) / (2 * B));
+    const bool act = group < nb / 2, wact = warp * (32 / kGL) < nb / 2;
+    const int li = gl >> (3 - LB);
+    float *xb = (float *)G, *xn = xb + nb * B * kGL * R;
+    GTile<B, R> t;
+    int X = act ? group : 0, Y = act ? nb - 1 - group : 0;
+#pragma unroll
+    for (int c = 0; c < 2 * B; ++c) {
+        const int col = c < B ? X * B + c : Y * B + (c - B);
+        const double *g = G + (size_t)(act && col < n ? prow[col] : 0) * ld;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int row = grow<R>(r, gl);
+            t.w[c][r] = act && col < n && row < n ? (float)(g[row] * scl) : 0.f;
+        }
+    }
+    const float tol = 10.f * Lim<float>::eps();
+    const float tol2 = tol * tol, ex2 = exit_ratio * exit_ratio;
+    int sweep = 1;
+    __syncthreads();
+    for (; sweep <= max_sweeps; ++sweep) {
+        int fl = 0;
+        if (wact) {
+            if constexpr (B > 1) {
+#pragma unroll
+                for (int j = 0; j < B - 1; ++j) {
+                    gstep<true>(t, tol2, ex2, fl, lane);
+                    gcircle(t);
+                }
+            }
+            // exact norms: column j of the 2B on lanes j * 8 / 2B ...
+            float nrm[2 * B];
+#pragma unroll
+            for (int c = 0; c < 2 * B; ++c) nrm[c] = gdot(t.w[c], t.w[c]);
+            group_reduce_scatter(nrm, lane);
+            const int base = lane & ~(kGL - 1);
+            t.nx = __shfl_sync(FULL, nrm[0], base | (li << (2 - LB)));
+            t.ny = __shfl_sync(FULL, nrm[0], base | ((B + li) << (2 - LB)));
+        }
+        for (int br = 0; br < nb - 1; ++br) {
+            if (br > 0 || sweep > 1) {
+                if (act) {
+                    gtile_x<B, R, true>(t, xb, X, Y, gl);
+                    if ((gl & (kGL / B - 1)) == 0) {
+                        xn[X * B + li] = t.nx;
+                        xn[Y * B + li] = t.ny;
+                    }
+                }
+                __syncthreads();
+                if (act) {
+                    if (X > 0) X = X == 1 ? nb - 1 : X - 1;
+                    Y = Y == 1 ? nb - 1 : Y - 1;
+                    gtile_x<B, R, false>(t, xb, X, Y, gl);
+                    t.nx = xn[X * B + li];
+                    t.ny = xn[Y * B + li];
+                }
+            }
+            if (wact) {
+#pragma unroll
+                for (int j = 0; j < B; ++j) {
+                    gstep<false>(t, tol2, ex2, fl, lane);
+                    gshift_y(t, lane);
+                }
+            }
+        }
+        if (!__syncthreads_or(fl & 4)) break;
+    }
+    if (sweep > max_sweeps) return sweep;
+    if (wact) {
+        float nrm[2 * B];
+#pragma unroll
+        for (int c = 0; c < 2 * B; ++c) nrm[c] = gdot(t.w[c], t.w[c]);
+        group_reduce_scatter(nrm, lane);
+        const int base = lane & ~(kGL - 1);
+#pragma unroll
+        for (int c = 0; c < 2 * B; ++c) {
+            const float inv = 1.f / sqrtf(__shfl_sync(FULL, nrm[0], base | (c << (2 - LB))));
+            const int col = c < B ? X * B + c : Y * B + (c - B);
+            if (act && col < n) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int row = grow<R>(r, gl);
+                    if (row < n) x[(size_t)col * n + row] = t.w[c][r] * inv;
+                }
+            }
+        }
+    }
+    return sweep;
+}
+
+// Pivoted Cholesky of G (n x n, both triangles, ld), thread i = row i: step
+// k takes the largest remaining diagonal p and leaves column k of L in row p
+// of G (rows chosen before: zero), p in prow[k].  The pivot is found on FP32
+// keys that carry the row (redux); one barrier a step.  False when a pivot is
+// <= cut.
+__device__ __forceinline__ bool pivoted_cholesky(double *G, int ld, int n, double cut, double scl, int *prow,
+                                                 double *sd, unsigned *skey) {
+    const int i = threadIdx.x, warp = i >> 5, lane = i & 31;
+    const bool mine = i < n;
+    double d = mine ? G[(size_t)i * ld + i] : 0.0;
+    bool taken = !mine;
+    if (mine) sd[i] = d;
+    for (int k = 0; k < n; ++k) {
+        const unsigned key = taken ? 0u : ((__float_as_uint(fmaxf((float)(d * scl), 0.f)) & ~63u) | (63 - i)) + 64u;
+        const unsigned kw = __reduce_max_sync(FULL, key);
+        if (lane == 0) skey[2 * (k & 1) + warp] = kw;
+        __syncthreads();
+        const unsigned kk = max(skey[2 * (k & 1)], skey[2 * (k & 1) + 1]);
+        const int p = 63 - (int)(kk & 63u);
+        const double dp = sd[p];
+        if (!(dp > cut)) return false;
+        const double rs = rsqrt(dp);
+        double *gp = G + (size_t)p * ld;
+        if (i < ld) {
+            double v[4] = {gp[i], 0.0, 0.0, 0.0};
+            int j = 0;
+            for (; j + 4 <= k; j += 4) {
+                const int4 r4 = *(const int4 *)(prow + j);
+                v[0] = fma(-G[r4.x * ld + i], G[r4.x * ld + p], v[0]);
+                v[1] = fma(-G[r4.y * ld + i], G[r4.y * ld + p], v[1]);
+                v[2] = fma(-G[r4.z * ld + i], G[r4.z * ld + p], v[2]);
+                v[3] = fma(-G[r4.w * ld + i], G[r4.w * ld + p], v[3]);
+            }
+            for (; j < k; ++j) v[0] = fma(-G[prow[j] * ld + i], G[prow[j] * ld + p], v[0]);
+            const double l = taken ? 0.0 : (i == p ? dp * rs : ((v[0] + v[1]) + (v[2] + v[3])) * rs);
+            gp[i] = l;
+            if (i == p) taken = true;
+            d = fma(-l, l, d);
+            if (mine && !taken) sd[i] = d;
+        }
+        if (i == 0) prow[k] = p;
+    }
+    __syncthreads();
+    return true;
+}
+
+__host__ __device__ inline int pre_ld(int n8) { return n8; }
+// Shared memory: prow (64 ints), sd (64 doubles), skey (4), then G (n8 x n8
+// doubles), the staged input and the exchange area in one place.
+__host__ __device__ inline size_t pre_smem(int mt, int nt) {
+    const int m8 = round8(mt), n8 = round8(nt);
+    const size_t g = (size_t)n8 * pre_ld(n8) * 8, a = stage_floats(m8, n8) * 4;
+    const size_t x = ((size_t)64 * 64 + 64) * 4 * (nt > 32 ? 4 : nt > 16 ? 1 : 1) / 4;   // npb x 8 R floats + norms
+    size_t r = g > a ? g : a;
+    r = r > x ? r : x;
+    return 64 * 4 + 64 * 8 + 16 + r;
+}
+
+template <int JOBS>
+__device__ __forceinline__ void gram_tiles(const float *As, Stage st, int m8, int nt8, double *G, int ld) {
+    // lower tiles of G in jobs of 4 x 2 (32 rows, 16 columns) over two warps; all
+    // sums stay in registers until the staged input is no longer needed
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    double acc[JOBS][4][2][2];
+#pragma unroll
+    for (int j = 0; j < JOBS; ++j)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) acc[j][a][b][0] = acc[j][a][b][1] = 0.0;
+    // jobs 0, 1: rows 0..31, columns 16 j; jobs 2..5: rows 32..63
+    auto job_row = [](int job) { return job < 2 ? 0 : 4; };
+    auto job_col = [](int job) { return job < 2 ? 2 * job : 2 * (job - 2); };
+    for (int k0 = 0; k0 < m8; k0 += 4) {
+        const float *a0 = As + (k0 + lk) * st.sr;
+#pragma unroll
+        for (int j = 0; j < JOBS; ++j) {
+            const int job = 2 * j + warp, tr = job_row(job), tc = job_col(job);
+            if (tr >= nt8 || tc >= nt8) continue;
+            double fa[4], fb[2];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) fa[a] = tr + a < nt8 ? (double)a0[((tr + a) * 8 + lr) * st.sk] : 0.0;
+#pragma unroll
+            for (int b = 0; b < 2; ++b) fb[b] = tc + b < nt8 ? (double)a0[((tc + b) * 8 + lr) * st.sk] : 0.0;
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) dmma(acc[j][a][b], fa[a], fb[b]);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < JOBS; ++j) {
+        const int job = 2 * j + warp, tr = job_row(job), tc = job_col(job);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                if (tr + a >= nt8 || tc + b > tr + a) continue;
+                const int r = (tr + a) * 8 + lr, c = (tc + b) * 8 + 2 * lk;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    G[(size_t)r * ld + c + e] = acc[j][a][b][e];
+                    if (tc + b < tr + a) G[(size_t)(c + e) * ld + r] = acc[j][a][b][e];
+                }
+            }
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kPreT, 7) precondition_kernel(Params p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_idx;
+    int *prow = (int *)smem;
+    double *sd = (double *)(smem + 64 * 4);
+    unsigned *skey = (unsigned *)(smem + 64 * 4 + 64 * 8);
+    double *G = (double *)(smem + 64 * 4 + 64 * 8 + 16);
+    const float exit_ratio = p.exit_ratio == 0.f ? kMixedExitRatio
+                                                 : (p.exit_ratio < 0.f ? 10.f * Lim<float>::eps() : p.exit_ratio);
+    for (;;) {
+        int64_t idx;
+        next_ticket(p.counter, s_idx, idx);
+        if (idx >= p.count) break;
+        const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
+        const jb_matrix_desc d = desc_of(p, mat);
+        int st = JB_ST_OK, ns = 0;
+        const int mt = d.m > d.n ? d.m : d.n, nt = d.m > d.n ? d.n : d.m;
+        if (!rdesc_fits(d, kB32, 4, p, true)) {
+            st = JB_ST_BAD_DESC;
+        } else if ((d.flags & JB_FULL_MATRICES) && mt > nt) {
+            st = kPending;
+        } else {
+            const bool wide = d.m < d.n;
+            const int m8 = round8(mt), n8 = round8(nt), ld = pre_ld(n8);
+            const Stage sg = stage_of(wide, m8, n8);
+            float *As = (float *)G;
+            const float *A = (const float *)p.A + d.a_off;
+            if (wide) stage_input<kPreT>(A, d.m, d.n, n8, m8, sg.sk, As);
+            else stage_input<kPreT>(A, d.m, d.n, m8, n8, sg.sr, As);
+            __syncthreads();
+            if (nt > 32) gram_tiles<3>(As, sg, m8, n8 >> 3, G, ld);
+            else gram_tiles<1>(As, sg, m8, n8 >> 3, G, ld);
+            // a diagonal of G is not finite exactly when the input is not
+            const double gd = threadIdx.x < nt ? G[(size_t)threadIdx.x * ld + threadIdx.x] : 0.0;
+            const bool bad = __syncthreads_or(!isfinite(gd));
+            // power of two that brings the largest diagonal into [1, 2)
+            const int ex = __reduce_max_sync(FULL, (__double2hiint(fabs(gd)) >> 20) & 0x7ff);
+            if ((threadIdx.x & 31) == 0) prow[threadIdx.x >> 5] = ex;
+            __syncthreads();
+            const int em = max(prow[0], prow[1]);
+            __syncthreads();
+            if (bad) {
+                st = JB_ST_NONFINITE_IN;
+            } else if (em == 0) {
+                st = kPending;   // zero matrix
+            } else {
+                const double gscl = __hiloint2double((2046 - em) << 20, 0);
+                // sqrt of it, within a factor 2, for the columns of L
+                const double lscl = __hiloint2double((1023 - ((em - 1023) >> 1)) << 20, 0);
+                if (!pivoted_cholesky(G, ld, nt, kPivotCut / gscl, gscl, prow, sd, skey)) {
+                    st = kPending;
+                } else {
+                    float *x = p.x32 + d.x_off;
+                    if (nt > 48) ns = precondition_sweeps<4, 8>(G, ld, prow, lscl, nt, exit_ratio, p.max_sweeps32, x);
+                    else if (nt > 32) ns = precondition_sweeps<4, 6>(G, ld, prow, lscl, nt, exit_ratio, p.max_sweeps32, x);
+                    else if (nt > 16) ns = precondition_sweeps<2, 4>(G, ld, prow, lscl, nt, exit_ratio, p.max_sweeps32, x);
+                    else ns = precondition_sweeps<1, 2>(G, ld, prow, lscl, nt, exit_ratio, p.max_sweeps32, x);
+                    if (ns > p.max_sweeps32) st = kPending;
+                }
+            }
+        }
+        if (threadIdx.x == 0) {
+            p.status[mat] = st;
+            p.sweeps[mat] = ns;
+            if (st == kPending) atomicAdd(p.n_pending, 1);
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 refinement.  Eight warps a matrix; V (n8 x ldv) and W (n8 x ldw,
+// column-major, FP64) in shared memory, the staged input and N in W's place
+// while W is not needed.  Bound by the f64 mma pipe: 3 n^3 + 6 m n^2 flop for
+// the usual one correction and its check.
+// ---------------------------------------------------------------------------
+struct RefGeo {
+    int m8, n8, ldv, ldw;
+};
+__host__ __device__ inline RefGeo ref_geo(int mt, int nt) {
+    RefGeo r;
+    r.m8 = round8(mt);
+    r.n8 = round8(nt);
+    r.ldv = ld4odd(r.n8);
+    r.ldw = ld4odd(r.m8);
+    return r;
+}
+__host__ __device__ inline size_t ref_smem(int mt, int nt) {
+    const RefGeo r = ref_geo(mt, nt);
+    size_t w = (size_t)r.n8 * r.ldw * 8;
+    const size_t a = stage_floats(r.m8, r.n8) * 4;
+    if (a > w) w = a;
+    return (size_t)r.n8 * r.ldv * 8 + w + (size_t)64 * 8 * 3 + 64 * 4;
+}
+
+// W = A V: blocks of 16 x 32 over the warps, at most two a warp (m <= 128, n <= 64).
+__device__ __forceinline__ void ref_w(const float *As, Stage st, const double *V, int ldv, double *W, int ldw, int mt8,
+                                      int nt8) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    const int bm = (mt8 + 1) >> 1, bn = (nt8 + 3) >> 2;
+    double acc[2][2][4][2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) acc[s][a][b][0] = acc[s][a][b][1] = 0.0;
+        const int blk = warp + 8 * s;
+        if (blk >= bm * bn) continue;
+        const int tr = 2 * (blk % bm), tc = 4 * (blk / bm);
+        for (int k0 = 0; k0 < 8 * nt8; k0 += 4) {
+            double fa[2], fb[4];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+                fa[a] = tr + a < mt8 ? (double)As[((tr + a) * 8 + lr) * st.sr + (k0 + lk) * st.sk] : 0.0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) fb[b] = tc + b < nt8 ? V[((tc + b) * 8 + lr) * ldv + k0 + lk] : 0.0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                if (tc + b < nt8) {
+#pragma unroll
+                    for (int a = 0; a < 2; ++a) dmma(acc[s][a][b], fa[a], fb[b]);
+                }
+        }
+    }
+    __syncthreads();   // the staged input gives way to W
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const int blk = warp + 8 * s;
+        if (blk >= bm * bn) continue;
+        const int tr = 2 * (blk % bm), tc = 4 * (blk / bm);
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                if (tr + a < mt8 && tc + b < nt8) {
+                    double *w = W + (size_t)((tc + b) * 8 + 2 * lk) * ldw + (tr + a) * 8 + lr;
+                    w[0] = acc[s][a][b][0];
+                    w[ldw] = acc[s][a][b][1];
+                }
+    }
+}
+
+// Lower 16 x 8 blocks of X^T X (X column-major, ld, rows8 rows): three jobs a warp at most.
+__device__ __forceinline__ void job_place(int job, int &tr, int &tc) {
+    // block row g (16 rows) has 2 g + 2 column tiles
+    int g = 0;
+    while (job >= 2 * g + 2) { job -= 2 * g + 2; ++g; }
+    tr = 2 * g;
+    tc = job;
+}
+__device__ __forceinline__ void ref_gram(const double *X, int ld, int rows8, int tr, int tc, int nt8,
+                                         double (&acc)[2][2]) {
+    const int lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    const double *x0 = X + (size_t)(tr * 8 + lr) * ld + lk;
+    const double *x1 = X + (size_t)((tr + 1 < nt8 ? tr + 1 : tr) * 8 + lr) * ld + lk;
+    const double *y = X + (size_t)(tc * 8 + lr) * ld + lk;
+    acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < rows8; k += 4) {
+        const double b = y[k];
+        dmma(acc[0], x0[k], b);
+        dmma(acc[1], x1[k], b);
+    }
+}
+
+// tan of the Jacobi angle of (d = h_qq - h_pp, h_pq) in FP32 from
+// exponent-scaled inputs: its relative error of 1e-7 is one of the
+// correction only.
+__device__ __forceinline__ double ref_angle(double d, double a) {
+    const double a2 = 2.0 * a;
+    const int ex = (__double2hiint(fmax(fabs(d), fabs(a2))) >> 20) & 0x7ff;
+    if (ex == 0) return 0.0;
+    const double scl = __hiloint2double((2046 - ex) << 20, 0);
+    const float df = fabsf((float)(d * scl)), af = (float)(a2 * scl);
+    const float hf = fmaf(df, df, af * af);
+    const float t = __fdividef(af, df + hf * rsqrtf(hf));
+    return d < 0.0 ? -(double)t : (double)t;
+}
+
+__global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_idx;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    for (;;) {
+        int64_t idx;
+        next_ticket(p.counter2, s_idx, idx);
+        if (idx >= p.count) break;
+        const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
+        const jb_matrix_desc d = desc_of(p, mat);
+        if (p.status[mat] != JB_ST_OK) continue;
+        const bool wide = d.m < d.n;
+        const int mt = wide ? d.n : d.m, nt = wide ? d.m : d.n;
+        const RefGeo g = ref_geo(mt, nt);
+        const int ldv = g.ldv, ldw = g.ldw, nt8 = g.n8 >> 3, mt8 = g.m8 >> 3;
+        double *dh = (double *)smem, *de = dh + 64, *sig = de + 64;   // diagonals of H and E; sigma
+        int *perm = (int *)(sig + 64);
+        double *V = (double *)(perm + 64);
+        double *W = V + (size_t)g.n8 * ldv;
+        double *Nm = W;                       // n8 x ldv
+        float *As = (float *)W;
+        const Stage sg = stage_of(wide, g.m8, g.n8);
+        const float *A = (const float *)p.A + d.a_off;
+        const float *x = p.x32 + d.x_off;
+        for (int k = threadIdx.x; k < g.n8 * g.n8; k += kRefT) {
+            const int c = k / g.n8, i = k - c * g.n8;
+            V[c * ldv + i] = (c < nt && i < nt) ? (double)x[c * nt + i] : 0.0;
+        }
+        const double tol = p.tol > 0 ? (double)(float)p.tol : (double)(10.0f * Lim<float>::eps());
+        const double tol2 = tol * tol;
+        const int nb16 = (nt8 + 1) >> 1, jobs = nb16 * (nb16 + 1);
+        const int most = p.max_sweeps < kRefPasses ? p.max_sweeps : kRefPasses;
+        int pass = 1;
+        bool done = false;
+        for (; pass <= most; ++pass) {
+            if (wide) stage_input<kRefT>(A, d.m, d.n, g.n8, g.m8, sg.sk, As);
+            else stage_input<kRefT>(A, d.m, d.n, g.m8, g.n8, sg.sr, As);
+            __syncthreads();
+            ref_w(As, sg, V, ldv, W, ldw, mt8, nt8);
+            __syncthreads();
+            double h[3][2][2], e[3][2][2];
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const int job = warp + 8 * s;
+                if (job >= jobs) continue;
+                int tr, tc;
+                job_place(job, tr, tc);
+                if (tc >= nt8) continue;
+                ref_gram(W, ldw, g.m8, tr, tc, nt8, h[s]);
+                ref_gram(V, ldv, g.n8, tr, tc, nt8, e[s]);
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+                    if (tr + a == tc) {   // diagonal tile: lanes with column 2 lk or 2 lk + 1 == row lr
+                        const int r = tc * 8 + lr;
+                        if ((lr >> 1) == lk) {
+                            const double ee = (lr & 1 ? e[s][a][1] : e[s][a][0]) - 1.0;
+                            dh[r] = lr & 1 ? h[s][a][1] : h[s][a][0];
+                            de[r] = r < nt ? ee : 0.0;
+                        }
+                    }
+            }
+            __syncthreads();
+            int need = 0;
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const int job = warp + 8 * s;
+                if (job >= jobs) continue;
+                int tr, tc;
+                job_place(job, tr, tc);
+                if (tc >= nt8) continue;
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int r = (tr + a) * 8 + lr, c = tc * 8 + 2 * lk + u;
+                        if (r < nt && c < r) {
+                            if (!(h[s][a][u] * h[s][a][u] <= tol2 * dh[r] * dh[c])) need = 1;
+                            if (!(fabs(e[s][a][u]) <= kRefOrth)) need = 1;
+                        } else if (r < nt && c == r) {
+                            if (!(fabs(de[r]) <= kRefOrth)) need = 1;
+                        }
+                    }
+            }
+            if (!__syncthreads_or(need)) { done = true; break; }
+            if (pass == most) break;
+            // N = K - E / 2, column-major in W's place
+            int wild = 0;
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const int job = warp + 8 * s;
+                if (job >= jobs) continue;
+                int tr, tc;
+                job_place(job, tr, tc);
+                if (tc >= nt8) continue;
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int r = (tr + a) * 8 + lr, c = tc * 8 + 2 * lk + u;
+                        if (tr + a >= nt8 || c > r) continue;
+                        if (r >= nt) {
+                            Nm[r * ldv + c] = 0.0;
+                            Nm[c * ldv + r] = 0.0;
+                        } else if (c == r) {
+                            Nm[c * ldv + r] = -0.5 * de[r];
+                        } else {
+                            // rotation of columns c < r of W: h without what E explains of it
+                            const double ee = e[s][a][u];
+                            const double off = h[s][a][u] - 0.5 * ee * (dh[r] + dh[c]);
+                            const double k = ref_angle(dh[r] * (1.0 - de[r]) - dh[c] * (1.0 - de[c]), off);
+                            if (!(fabs(k) <= 0.25 && fabs(ee) <= 0.1)) wild = 1;
+                            Nm[r * ldv + c] = k - 0.5 * ee;
+                            Nm[c * ldv + r] = -k - 0.5 * ee;
+                        }
+                    }
+            }
+            if (__syncthreads_or(wild)) { pass = most; break; }
+            // second-order term on the diagonal: -sum_i K_ij^2 / 2 (an isolated
+            // close pair has an angle far above all others)
+            for (int j = warp; j < nt; j += kRefT / 32) {
+                double sum = 0.0;
+                for (int i = lane; i < nt; i += 32) {
+                    const double k = 0.5 * (Nm[j * ldv + i] - Nm[i * ldv + j]);
+                    sum = fma(k, k, sum);
+                }
+                sum = warp_sum(sum);
+                if (lane == 0) dh[j] = -0.5 * sum;
+            }
+            __syncthreads();
+            // V <- V + V N: one 16 x 32 block a warp
+            {
+                const int bm = (nt8 + 1) >> 1, bn = (nt8 + 3) >> 2;
+                double acc[2][4][2];
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+                const int tr = 2 * (warp % bm), tc = 4 * (warp / bm);
+                const bool own = warp < bm * bn;
+                if (own) {
+                    for (int k0 = 0; k0 < g.n8; k0 += 4) {
+                        double fa[2], fb[4];
+#pragma unroll
+                        for (int a = 0; a < 2; ++a)
+                            fa[a] = tr + a < nt8 ? V[(k0 + lk) * ldv + (tr + a) * 8 + lr] : 0.0;
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) {
+                            const int c = (tc + b) * 8 + lr;
+                            fb[b] = tc + b < nt8 ? Nm[c * ldv + k0 + lk] + (c == k0 + lk && c < nt ? dh[c] : 0.0) : 0.0;
+                        }
+#pragma unroll
+                        for (int b = 0; b < 4; ++b)
+                            if (tc + b < nt8) {
+#pragma unroll
+                                for (int a = 0; a < 2; ++a) dmma(acc[a][b], fa[a], fb[b]);
+                            }
+                    }
+                }
+                __syncthreads();
+                if (own) {
+#pragma unroll
+                    for (int a = 0; a < 2; ++a)
+#pragma unroll
+                        for (int b = 0; b < 4; ++b)
+                            if (tr + a < nt8 && tc + b < nt8) {
+                                double *v = V + (size_t)((tc + b) * 8 + 2 * lk) * ldv + (tr + a) * 8 + lr;
+                                v[0] += acc[a][b][0];
+                                v[ldv] += acc[a][b][1];
+                            }
+                }
+            }
+        }
+        // sigma, the stable descending order and the cut (primitives.py:356-366)
+        int st = JB_ST_OK;
+        if (done) {
+            if (threadIdx.x < nt) sig[threadIdx.x] = sqrt(dh[threadIdx.x]);
+            __syncthreads();
+            int below = 0;
+            if (threadIdx.x < 4 * nt) {   // four threads count a column's rank
+                const int j = threadIdx.x >> 2;
+                const double sj = sig[j];
+                int rnk = 0;
+                double smax = 0.0;
+                for (int i = threadIdx.x & 3; i < nt; i += 4) {
+                    const double si = sig[i];
+                    rnk += (si > sj) || (si == sj && i < j);
+                    smax = fmax(smax, si);
+                }
+                const unsigned quad = 0xfu << (lane & ~3);
+                rnk += __shfl_xor_sync(quad, rnk, 1);
+                rnk += __shfl_xor_sync(quad, rnk, 2);
+                smax = fmax(smax, __shfl_xor_sync(quad, smax, 1));
+                smax = fmax(smax, __shfl_xor_sync(quad, smax, 2));
+                const int npref = nt + (nt & 1);
+                below = !(sj > Lim<double>::eps() * (mt > npref ? mt : npref) * smax);
+                if ((threadIdx.x & 3) == 0) perm[rnk] = j;
+            }
+            if (__syncthreads_or(below)) done = false;   // columns to complete: not here
+        }
+        if (!done) {
+            st = kPending;
+        } else {
+            float *U = p.U ? (float *)p.U + d.u_off : nullptr;
+            float *Vh = p.Vh ? (float *)p.Vh + d.v_off : nullptr;
+            float *S = (float *)p.S + d.s_off;
+            int bad = 0;
+            if (threadIdx.x < d.rank) {
+                const float o = (float)sig[perm[threadIdx.x]];
+                if (!isfinite(o)) bad = 1;
+                S[threadIdx.x] = o;
+            }
+            if (!(d.flags & JB_VALUES_ONLY)) {
+                if (threadIdx.x < nt) dh[threadIdx.x] = 1.0 / sig[threadIdx.x];
+                __syncthreads();
+                // left factor X (rows x rank, row-major): 8 ranks x 4 rows a warp and step
+                const double *X = wide ? V : W;
+                const int ldl = wide ? ldv : ldw, rows = wide ? nt : mt;
+                const int r8 = (d.rank + 7) >> 3;
+                for (int blk = warp; blk < ((rows + 3) >> 2) * r8; blk += kRefT / 32) {
+                    const int r = (blk % r8) * 8 + (lane & 7), i = (blk / r8) * 4 + (lane >> 3);
+                    if (r < d.rank && i < rows) {
+                        const int c = perm[r];
+                        const float o = (float)(wide ? X[c * ldl + i] : X[c * ldl + i] * dh[c]);
+                        if (!isfinite(o)) bad = 1;
+                        U[(size_t)i * d.rank + r] = o;
+                    }
+                }
+                const double *Y = wide ? W : V;
+                const int ldr = wide ? ldw : ldv, cols = wide ? mt : nt;
+                for (int r = warp; r < d.rank; r += kRefT / 32) {
+                    const int c = perm[r];
+                    const double f = wide ? dh[c] : 1.0;
+                    for (int i = lane; i < cols; i += 32) {
+                        const float o = (float)(Y[c * ldr + i] * f);
+                        if (!isfinite(o)) bad = 1;
+                        Vh[(size_t)r * cols + i] = o;
+                    }
+                }
+            }
+            if (__syncthreads_or(bad)) st = JB_ST_NONFINITE_OUT;
+        }
+        if (threadIdx.x == 0) {
+            p.status[mat] = st;
+            if (st == kPending) atomicAdd(p.n_pending, 1);
+            else p.sweeps[mat] += pass;
+        }
+        __syncthreads();
+    }
+}
+
+}  // namespace jb
