@@ -199,14 +199,16 @@ class UnevenBatch:
         # Persistent kernels per solve (after a memset of the work tickets): one
         # per precision phase; on the register path (max(m, n) <= 128, min(m, n)
         # <= 64) a mixed solve takes four (precondition, refine, and the FP32
-        # and FP64 register kernels for what these leave), an FP32 one two when
-        # the batch is wider than 32 (widths above and up to 32 columns run in
-        # CTAs of different sizes).
+        # and FP64 register kernels for what these leave) after the factor
+        # kernel (one CTA a matrix), an FP32 one two when the batch is wider
+        # than 32 (widths above and up to 32 columns run in CTAs of different
+        # sizes).  launches_per_solve counts every kernel.
         phases = 2 if self.precision == N.PREC_MIXED else 1
         register = (not self.launch_choice.flags & (N.ROUND_ROBIN | N.BLOCK_WIDTH_8) and self.max_m <= 128
                     and self.max_n <= 64)
         split = self.max_n > 32 and not self.launch_choice.flags & N.ONE_SIZE_CLASS
         self.kernels_per_solve = phases * (2 if register and (phases == 2 or split) else 1)
+        self.launches_per_solve = self.kernels_per_solve + (1 if register and phases == 2 else 0)
 
     # -- solving ----------------------------------------------------------------
     def launch(self, a_flat: torch.Tensor, stream=None):

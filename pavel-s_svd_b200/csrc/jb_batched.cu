@@ -918,6 +918,7 @@ __global__ void __launch_bounds__(256) warm_prep_kernel(const float *A, const fl
 // ---------------------------------------------------------------------------
 constexpr size_t kSmemLimit = 227 * 1024;
 constexpr size_t kCounterBytes = 256;
+constexpr int64_t kMaxGrid = 1 << 20;   // CTAs of a launch with one CTA a matrix
 
 struct DevInfo {
     int sms = 0;
@@ -1097,7 +1098,7 @@ static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsign
     if (cudaMemsetAsync(ws, 0, 8 * sizeof(int), st) != cudaSuccess) return JB_ECUDA;
     int64_t grid;
     int rc;
-    // Mixed solve: precondition and refine; the register kernels below then
+    // Mixed solve: factor, precondition and refine; the register kernels below then
     // take what these left (usually nothing: they read one word and return).
     // Not with a warm start or another block width, which are choices of the
     // register kernels, nor for full bases, which the refinement does not
@@ -1107,7 +1108,11 @@ static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsign
         p.n_pending = (int *)ws + 4;
         p.maxd = pl.d32;
         p.region_cap = pl.reg32;
-        const size_t s1 = pre_smem(pl.d.mt, pl.d.nt), s2 = ref_smem(pl.d.mt, pl.d.nt);
+        const size_t s0 = fac_smem(pl.d.mt, pl.d.nt), s1 = pre_smem(pl.d.nt), s2 = ref_smem(pl.d.mt, pl.d.nt);
+        // one CTA a matrix, largest first: no state is kept from one to the next
+        if ((rc = occupancy_grid(factor_kernel, kFacT, s0, p.count, grid))) return rc;
+        factor_kernel<<<(unsigned)(p.count < kMaxGrid ? p.count : kMaxGrid), kFacT, s0, st>>>(p);
+        if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
         if ((rc = occupancy_grid(precondition_kernel, kPreT, s1, p.count, grid))) return rc;
         precondition_kernel<<<(unsigned)grid, kPreT, s1, st>>>(p);
         if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;

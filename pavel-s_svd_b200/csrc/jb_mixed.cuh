@@ -2,11 +2,13 @@
 // (tall view): a preconditioned FP32 Jacobi, then an FP64 refinement made of
 // matrix products.
 //
+//   factor_kernel (128 threads a matrix)
+//     G = A^T A in FP64 (mma f64), pivoted Cholesky P^T G P = L L^T in FP64;
+//     L rounded to FP32.
 //   precondition_kernel (64 threads a matrix)
-//     G = A^T A in FP64 (mma f64), pivoted Cholesky P^T G P = L L^T in FP64,
-//     one-sided Jacobi of L rounded to FP32.  A = Q L^T P^T, so the left
-//     singular vectors of L are the right singular vectors of A: the rotated
-//     and normalised columns are V, and no V is accumulated.  L is n x n and
+//     one-sided FP32 Jacobi of L.  A = Q L^T P^T, so the left singular vectors
+//     of L are the right singular vectors of A: the rotated and normalised
+//     columns are V, and no V is accumulated.  L is n x n and
 //     its columns start out graded (Veselic and Hari; Drmac and Veselic), so
 //     a sweep moves n instead of m + n rows a column and fewer sweeps are
 //     needed (128 x 64 with singular values over three decades: 7 instead of
@@ -20,11 +22,11 @@
 //     (primitives.py:340-346), which leaves the square of the errors (the
 //     refinement of Ogita and Aishima).  Usually one correction.
 //
-// Measured (B200, 8192 matrices n ~ U[8,64], m ~ U[n,2n]): 1.62 + 1.27 ms a
-// batch, against 4.55 + 3.03 ms of the register kernels' FP32 and FP64 phases
-// from V = I; 4096 x 128 x 64 over three decades 3.4 against 12.9 ms.  U is
-// also closer to LAPACK's (1.4e-7 against 1.4e-6: all pairs are corrected,
-// not only those above tol).
+// Measured (B200, 8192 matrices n ~ U[8,64], m ~ U[n,2n]; ms a batch): factor
+// 0.37, precondition 0.86, refine 1.01, against 4.55 + 3.03 of the register
+// kernels' FP32 and FP64 phases from V = I; 4096 x 128 x 64 over three decades
+// 0.44 + 1.00 + 1.03 against 12.9.  U is also closer to LAPACK's (1.4e-7 against
+// 1.4e-6: all pairs are corrected, not only those above tol).
 //
 // A matrix that this does not suit -- numerically rank-deficient, full bases
 // wanted, no convergence within its passes -- is marked kPending and solved by
@@ -36,8 +38,7 @@ namespace jb {
 
 constexpr int kPending = -1;   // status: left to the register kernels
 constexpr int kHanded = -2;    // status: FP32 sweeps done by rb32, FP64 phase due
-constexpr int kPreT = 64, kRefT = 256;
-constexpr int kPreN = 64, kPreM = 128;
+constexpr int kFacT = 128, kPreT = 64, kRefT = 256;
 // A pivot below kPivotCut times the largest diagonal of G (a singular value
 // ratio of about 3e-6) is left to the register kernels: FP64 rounding of G
 // no longer resolves it well enough for a start.
@@ -68,26 +69,47 @@ __host__ __device__ inline size_t stage_floats(int m8, int n8) {
     const size_t a = (size_t)m8 * ld4odd(n8), b = (size_t)n8 * ld8odd(m8);
     return a > b ? a : b;
 }
+// Asynchronous copies (global to shared, zeros past the input): all of a
+// thread's loads are in flight at once.  Rows in quads when the input allows.
+__device__ __forceinline__ void cp_async4(float *dst, const float *src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
+                 :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async16(float *dst, const float *src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
 template <int THREADS>
-__device__ void stage_input(const float *A, int rows, int cols, int rows8, int cols8, int ld, float *As) {
+__device__ __forceinline__ void stage_input(const float *A, int rows, int cols, int rows8, int cols8, int ld,
+                                            float *As) {
     // input rows x cols (row-major), padded with zeros; the thread's column
     // and row advance by a fixed step
-    const int step_r = THREADS / cols8, step_c = THREADS - step_r * cols8;
-    int r = threadIdx.x / cols8, c = threadIdx.x - r * cols8;
+    const bool quads = (cols & 3) == 0 && ((uintptr_t)A & 15) == 0;
+    const int width = quads ? cols8 >> 2 : cols8;
+    const int step_r = THREADS / width, step_c = THREADS - step_r * width;
+    int r = threadIdx.x / width, c = threadIdx.x - r * width;
     while (r < rows8) {
-        float v[8];
-        int at[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            at[u] = r < rows8 ? r * ld + c : -1;
-            v[u] = (r < rows && c < cols) ? A[(size_t)r * cols + c] : 0.f;
-            r += step_r;
-            c += step_c;
-            if (c >= cols8) { c -= cols8; ++r; }
+        if (quads) {
+            const bool in = r < rows && 4 * c < cols;
+            cp_async16(As + r * ld + 4 * c, in ? A + (size_t)r * cols + 4 * c : A, in);
+        } else {
+            const bool in = r < rows && c < cols;
+            cp_async4(As + r * ld + c, in ? A + (size_t)r * cols + c : A, in);
         }
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (at[u] >= 0) As[at[u]] = v[u];
+        r += step_r;
+        c += step_c;
+        if (c >= width) { c -= width; ++r; }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+}
+__device__ __forceinline__ void stage_tall(const float *A, const jb_matrix_desc &d, int m8, int n8, Stage st, float *As,
+                                           int threads) {
+    if (threads == 128) {
+        if (d.m < d.n) stage_input<128>(A, d.m, d.n, n8, m8, st.sk, As);
+        else stage_input<128>(A, d.m, d.n, m8, n8, st.sr, As);
+    } else {
+        if (d.m < d.n) stage_input<256>(A, d.m, d.n, n8, m8, st.sk, As);
+        else stage_input<256>(A, d.m, d.n, m8, n8, st.sr, As);
     }
 }
 
@@ -96,8 +118,11 @@ __device__ void stage_input(const float *A, int rows, int cols, int rows8, int c
 // the 2B columns of its two blocks.  Compared with a whole warp a pair
 // (jb_regblock.cuh) a step's fixed cost -- the reductions, the rotation
 // parameters, the broadcasts -- is shared by four pairs of blocks a warp:
-// about 10 instead of 39 instructions a column pair at 64 rows.  Eight
-// groups hold all columns, so a matrix needs two warps.
+// about 8 instead of 39 instructions a column pair at 64 rows.  Eight
+// groups hold all columns, so a matrix needs two warps.  Issue-bound (62 % of
+// the issue slots at 16 warps an SM, registers the limit); plain instead of
+// scaled rotations, unrolled intra steps and the factor in the same kernel (12
+// warps an SM) took 1.62 ms for factor and sweeps on the uneven batch, 1.22 now.
 // ---------------------------------------------------------------------------
 constexpr int kGL = 8;
 
@@ -120,10 +145,16 @@ __device__ __forceinline__ void group_reduce_scatter(float (&x)[NV], int lane) {
     for (int o = (kGL / 2) >> L; o >= 1; o >>= 1) x[0] += __shfl_xor_sync(FULL, x[0], o);
 }
 
+// The columns are kept scaled, w = scale * (the tile's column): a rotation is
+// then x - a y, y + b x with both columns' scales multiplied by c (Gentleman's
+// square-root-free rotation), half the arithmetic of the plain form.  Scales
+// start at 1 each sweep and shrink by at most sqrt(2) a rotation.
 template <int B, int R>
 struct GTile {
     float w[2 * B][R];
-    float nx, ny;   // squared norms of the lane's pair (x_i, y_i), i = lane's position in the group / (8 / B)
+    // of the lane's pair (x_i, y_i), i = the lane's position in the group / (8 / B):
+    float nx, ny;   // squared norms
+    float dx, dy;   // scales
 };
 
 template <int R>
@@ -133,16 +164,48 @@ __device__ __forceinline__ float gdot(const float (&x)[R], const float (&y)[R]) 
     for (int r = 0; r < R; r += 2) fma2(a0, a1, x[r], x[r + 1], y[r], y[r + 1]);
     return a0 + a1;
 }
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// The rotation of rot_params<float> as its tangent t (with the sign of apq)
+// and c, on approximate reciprocals without denormal handling: the squared
+// norms here are above kPivotCut of the largest, which is about 1.  Returns
+// bit 0: active, bit 2: ratio > the exit ratio.  Inactive: t = 0, c = 1.
+__device__ __forceinline__ int gparams(float app, float aqq, float apq, float tol2, float ex2, float &t, float &c) {
+    const float apq2 = apq * apq, prod = app * aqq;
+    const bool active = apq2 > tol2 * prod && fminf(app, aqq) > 0.f;
+    const float d = aqq - app;
+    const float h = fmaf(d, d, 4.f * apq2);
+    const float tt = 2.f * apq * rcp_ftz(fabsf(d) + h * rsqrt_ftz(h));
+    t = active ? (d < 0.f ? -tt : tt) : 0.f;
+    const float x = fmaf(t, t, 1.f);
+    const float c0 = rsqrt_ftz(x);
+    c = c0 * fmaf(-0.5f * x, c0 * c0, 1.5f);
+    return active ? 1 | (apq2 > ex2 * prod ? 4 : 0) : 0;
+}
+// x <- x - a y, y <- y + b x
 template <int R>
-__device__ __forceinline__ void grot(float (&x)[R], float (&y)[R], float c, float s) {
-    const Rot2 g(c, s);
+__device__ __forceinline__ void grot(float (&x)[R], float (&y)[R], float a, float b) {
+    const float2 na = make_float2(-a, -a), pb = make_float2(b, b);
 #pragma unroll
-    for (int r = 0; r < R; r += 2) rot2(x[r], x[r + 1], y[r], y[r + 1], g);
+    for (int r = 0; r < R; r += 2) {
+        const float2 u = make_float2(x[r], x[r + 1]), v = make_float2(y[r], y[r + 1]);
+        const float2 u2 = __ffma2_rn(na, v, u), v2 = __ffma2_rn(pb, u, v);
+        x[r] = u2.x; x[r + 1] = u2.y;
+        y[r] = v2.x; y[r + 1] = v2.y;
+    }
 }
 
-// B pairs of the group's columns: INTRA pairs columns inside each block with
-// exact norms; otherwise x_i with y_i, norms kept and updated by the lanes
-// of pair i (rot_params' shift).
+// B pairs of the group's columns: INTRA pairs columns inside each block, with
+// scales 1 and exact norms, and applies c; otherwise x_i with y_i, norms and
+// scales kept by the lanes of pair i.
 template <bool INTRA, int B, int R>
 __device__ __forceinline__ void gstep(GTile<B, R> &t, float tol2, float ex2, int &fl, int lane) {
     constexpr int LB = Log2<B>::value;
@@ -150,7 +213,7 @@ __device__ __forceinline__ void gstep(GTile<B, R> &t, float tol2, float ex2, int
 #pragma unroll
     for (int i = 0; i < B; ++i) pc[i] = gdot(t.w[pair_p<INTRA, B>(i)], t.w[pair_q<INTRA, B>(i)]);
     group_reduce_scatter(pc, lane);
-    float app, aqq;
+    float tn, c;
     if constexpr (INTRA) {
         float pa[B], pb[B];
 #pragma unroll
@@ -161,25 +224,32 @@ __device__ __forceinline__ void gstep(GTile<B, R> &t, float tol2, float ex2, int
         }
         group_reduce_scatter(pa, lane);
         group_reduce_scatter(pb, lane);
-        app = pa[0];
-        aqq = pb[0];
-    } else {
-        app = t.nx;
-        aqq = t.ny;
-    }
-    float c, s, sh;
-    const int f = rot_params<float>(app, aqq, pc[0], tol2, 0.f, ex2, 0.f, c, s, &sh);
-    fl |= f;
-    if (!__any_sync(FULL, f != 0)) return;
-    if constexpr (!INTRA) {
-        t.nx = app - sh;
-        t.ny = aqq + sh;
-    }
+        fl |= gparams(pa[0], pb[0], pc[0], tol2, ex2, tn, c);
 #pragma unroll
-    for (int i = 0; i < B; ++i) {
-        const int src = (lane & ~(kGL - 1)) | (i << (3 - LB));
-        const float ci = __shfl_sync(FULL, c, src), si = __shfl_sync(FULL, s, src);
-        grot(t.w[pair_p<INTRA, B>(i)], t.w[pair_q<INTRA, B>(i)], ci, si);
+        for (int i = 0; i < B; ++i) {
+            const int src = (lane & ~(kGL - 1)) | (i << (3 - LB));
+            const float ti = __shfl_sync(FULL, tn, src), ci = __shfl_sync(FULL, c, src);
+            const int p = pair_p<INTRA, B>(i), q = pair_q<INTRA, B>(i);
+            grot(t.w[p], t.w[q], ti, ti);
+#pragma unroll
+            for (int r = 0; r < R; ++r) { t.w[p][r] *= ci; t.w[q][r] *= ci; }
+        }
+    } else {
+        const float apq = pc[0] * (t.dx * t.dy);
+        const int f = gparams(t.nx, t.ny, apq, tol2, ex2, tn, c);
+        fl |= f;
+        if (!__any_sync(FULL, f != 0)) return;
+        const float sh = tn * apq;
+        const float a = tn * (t.dy * rcp_ftz(t.dx)), b = tn * (t.dx * rcp_ftz(t.dy));
+        t.nx -= sh;
+        t.ny += sh;
+        t.dx *= c;
+        t.dy *= c;
+#pragma unroll
+        for (int i = 0; i < B; ++i) {
+            const int src = (lane & ~(kGL - 1)) | (i << (3 - LB));
+            grot(t.w[i], t.w[B + i], __shfl_sync(FULL, a, src), __shfl_sync(FULL, b, src));
+        }
     }
 }
 
@@ -199,7 +269,9 @@ __device__ __forceinline__ void gcircle(GTile<B, R> &t) {
 }
 template <int B, int R>
 __device__ __forceinline__ void gshift_y(GTile<B, R> &t, int lane) {
-    t.ny = __shfl_sync(FULL, t.ny, (lane & ~(kGL - 1)) | ((lane + kGL / B) & (kGL - 1)));
+    const int from = (lane & ~(kGL - 1)) | ((lane + kGL / B) & (kGL - 1));
+    t.ny = __shfl_sync(FULL, t.ny, from);
+    t.dy = __shfl_sync(FULL, t.dy, from);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const float f = t.w[B][r];
@@ -241,62 +313,67 @@ __device__ __forceinline__ void gtile_x(GTile<B, R> &t, float *xw, int X, int Y,
     }
 }
 
-// Sweeps over L (column c = G[prow[c] * ld + row], scaled by scl) until no pair
-// ratio of a sweep exceeds exit_ratio; then the normalised columns to x (n x
-// n, column-major).  G's memory becomes the exchange area.  Returns the
-// sweeps, or max_sweeps + 1.
+// Sweeps over L (x, n x n, column-major) until no pair ratio of a sweep
+// exceeds exit_ratio; then the normalised columns take L's place.  xb: the
+// exchange area.  Returns the sweeps, or max_sweeps + 1.
 template <int B, int R>
-__device__ int precondition_sweeps(double *G, int ld, const int *prow, double scl, int n, float exit_ratio,
-                                   int max_sweeps, float *x) {
+__device__ int precondition_sweeps(float *xb, int n, float exit_ratio, int max_sweeps, float *x) {
     constexpr int LB = Log2<B>::value;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (kGL - 1);
     const int group = threadIdx.x / kGL;
     const int nb = 2 * ((n + 2 * B - 1) / (2 * B));
     const bool act = group < nb / 2, wact = warp * (32 / kGL) < nb / 2;
-    const int li = gl >> (3 - LB);
-    float *xb = (float *)G, *xn = xb + nb * B * kGL * R;
+    const int li = gl >> (3 - LB), base = lane & ~(kGL - 1);
+    float2 *xn = (float2 *)(xb + nb * B * kGL * R);
     GTile<B, R> t;
     int X = act ? group : 0, Y = act ? nb - 1 - group : 0;
 #pragma unroll
     for (int c = 0; c < 2 * B; ++c) {
         const int col = c < B ? X * B + c : Y * B + (c - B);
-        const double *g = G + (size_t)(act && col < n ? prow[col] : 0) * ld;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int row = grow<R>(r, gl);
-            t.w[c][r] = act && col < n && row < n ? (float)(g[row] * scl) : 0.f;
+            t.w[c][r] = act && col < n && row < n ? x[col * n + row] : 0.f;
         }
     }
     const float tol = 10.f * Lim<float>::eps();
     const float tol2 = tol * tol, ex2 = exit_ratio * exit_ratio;
     int sweep = 1;
-    __syncthreads();
     for (; sweep <= max_sweeps; ++sweep) {
         int fl = 0;
         if (wact) {
-            if constexpr (B > 1) {
+            if (sweep > 1) {   // back to scales 1
 #pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    const float sx = __shfl_sync(FULL, t.dx, base | (i << (3 - LB)));
+                    const float sy = __shfl_sync(FULL, t.dy, base | (i << (3 - LB)));
+#pragma unroll
+                    for (int r = 0; r < R; ++r) { t.w[i][r] *= sx; t.w[B + i][r] *= sy; }
+                }
+            }
+            if constexpr (B > 1) {
+#pragma unroll 1
                 for (int j = 0; j < B - 1; ++j) {
                     gstep<true>(t, tol2, ex2, fl, lane);
                     gcircle(t);
                 }
             }
-            // exact norms: column j of the 2B on lanes j * 8 / 2B ...
-            float nrm[2 * B];
+            float nrm[2 * B];   // exact norms: column j's on lanes j * 8 / 2B ...
 #pragma unroll
             for (int c = 0; c < 2 * B; ++c) nrm[c] = gdot(t.w[c], t.w[c]);
             group_reduce_scatter(nrm, lane);
-            const int base = lane & ~(kGL - 1);
             t.nx = __shfl_sync(FULL, nrm[0], base | (li << (2 - LB)));
             t.ny = __shfl_sync(FULL, nrm[0], base | ((B + li) << (2 - LB)));
+            t.dx = t.dy = 1.f;
         }
+#pragma unroll 1
         for (int br = 0; br < nb - 1; ++br) {
             if (br > 0 || sweep > 1) {
                 if (act) {
                     gtile_x<B, R, true>(t, xb, X, Y, gl);
                     if ((gl & (kGL / B - 1)) == 0) {
-                        xn[X * B + li] = t.nx;
-                        xn[Y * B + li] = t.ny;
+                        xn[X * B + li] = make_float2(t.nx, t.dx);
+                        xn[Y * B + li] = make_float2(t.ny, t.dy);
                     }
                 }
                 __syncthreads();
@@ -304,8 +381,9 @@ __device__ int precondition_sweeps(double *G, int ld, const int *prow, double sc
                     if (X > 0) X = X == 1 ? nb - 1 : X - 1;
                     Y = Y == 1 ? nb - 1 : Y - 1;
                     gtile_x<B, R, false>(t, xb, X, Y, gl);
-                    t.nx = xn[X * B + li];
-                    t.ny = xn[Y * B + li];
+                    const float2 u = xn[X * B + li], v = xn[Y * B + li];
+                    t.nx = u.x; t.dx = u.y;
+                    t.ny = v.x; t.dy = v.y;
                 }
             }
             if (wact) {
@@ -324,7 +402,6 @@ __device__ int precondition_sweeps(double *G, int ld, const int *prow, double sc
 #pragma unroll
         for (int c = 0; c < 2 * B; ++c) nrm[c] = gdot(t.w[c], t.w[c]);
         group_reduce_scatter(nrm, lane);
-        const int base = lane & ~(kGL - 1);
 #pragma unroll
         for (int c = 0; c < 2 * B; ++c) {
             const float inv = 1.f / sqrtf(__shfl_sync(FULL, nrm[0], base | (c << (2 - LB))));
@@ -333,7 +410,7 @@ __device__ int precondition_sweeps(double *G, int ld, const int *prow, double sc
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const int row = grow<R>(r, gl);
-                    if (row < n) x[(size_t)col * n + row] = t.w[c][r] * inv;
+                    if (row < n) x[col * n + row] = t.w[c][r] * inv;
                 }
             }
         }
@@ -341,123 +418,15 @@ __device__ int precondition_sweeps(double *G, int ld, const int *prow, double sc
     return sweep;
 }
 
-// Pivoted Cholesky of G (n x n, both triangles, ld), thread i = row i: step
-// k takes the largest remaining diagonal p and leaves column k of L in row p
-// of G (rows chosen before: zero), p in prow[k].  The pivot is found on FP32
-// keys that carry the row (redux); one barrier a step.  False when a pivot is
-// <= cut.
-__device__ __forceinline__ bool pivoted_cholesky(double *G, int ld, int n, double cut, double scl, int *prow,
-                                                 double *sd, unsigned *skey) {
-    const int i = threadIdx.x, warp = i >> 5, lane = i & 31;
-    const bool mine = i < n;
-    double d = mine ? G[(size_t)i * ld + i] : 0.0;
-    bool taken = !mine;
-    if (mine) sd[i] = d;
-    for (int k = 0; k < n; ++k) {
-        const unsigned key = taken ? 0u : ((__float_as_uint(fmaxf((float)(d * scl), 0.f)) & ~63u) | (63 - i)) + 64u;
-        const unsigned kw = __reduce_max_sync(FULL, key);
-        if (lane == 0) skey[2 * (k & 1) + warp] = kw;
-        __syncthreads();
-        const unsigned kk = max(skey[2 * (k & 1)], skey[2 * (k & 1) + 1]);
-        const int p = 63 - (int)(kk & 63u);
-        const double dp = sd[p];
-        if (!(dp > cut)) return false;
-        const double rs = rsqrt(dp);
-        double *gp = G + (size_t)p * ld;
-        if (i < ld) {
-            double v[4] = {gp[i], 0.0, 0.0, 0.0};
-            int j = 0;
-            for (; j + 4 <= k; j += 4) {
-                const int4 r4 = *(const int4 *)(prow + j);
-                v[0] = fma(-G[r4.x * ld + i], G[r4.x * ld + p], v[0]);
-                v[1] = fma(-G[r4.y * ld + i], G[r4.y * ld + p], v[1]);
-                v[2] = fma(-G[r4.z * ld + i], G[r4.z * ld + p], v[2]);
-                v[3] = fma(-G[r4.w * ld + i], G[r4.w * ld + p], v[3]);
-            }
-            for (; j < k; ++j) v[0] = fma(-G[prow[j] * ld + i], G[prow[j] * ld + p], v[0]);
-            const double l = taken ? 0.0 : (i == p ? dp * rs : ((v[0] + v[1]) + (v[2] + v[3])) * rs);
-            gp[i] = l;
-            if (i == p) taken = true;
-            d = fma(-l, l, d);
-            if (mine && !taken) sd[i] = d;
-        }
-        if (i == 0) prow[k] = p;
-    }
-    __syncthreads();
-    return true;
+__host__ __device__ inline size_t pre_smem(int nt) {
+    const size_t cols = nt > 32 ? (nt + 7) / 8 * 8 : nt > 16 ? (nt + 3) / 4 * 4 : (nt + 1) / 2 * 2;
+    return cols * kGL * (nt > 48 ? 8 : nt > 32 ? 6 : nt > 16 ? 4 : 2) * 4 + cols * 8;
 }
 
-__host__ __device__ inline int pre_ld(int n8) { return n8; }
-// Shared memory: prow (64 ints), sd (64 doubles), skey (4), then G (n8 x n8
-// doubles), the staged input and the exchange area in one place.
-__host__ __device__ inline size_t pre_smem(int mt, int nt) {
-    const int m8 = round8(mt), n8 = round8(nt);
-    const size_t g = (size_t)n8 * pre_ld(n8) * 8, a = stage_floats(m8, n8) * 4;
-    const size_t x = ((size_t)64 * 64 + 64) * 4 * (nt > 32 ? 4 : nt > 16 ? 1 : 1) / 4;   // npb x 8 R floats + norms
-    size_t r = g > a ? g : a;
-    r = r > x ? r : x;
-    return 64 * 4 + 64 * 8 + 16 + r;
-}
-
-template <int JOBS>
-__device__ __forceinline__ void gram_tiles(const float *As, Stage st, int m8, int nt8, double *G, int ld) {
-    // lower tiles of G in jobs of 4 x 2 (32 rows, 16 columns) over two warps; all
-    // sums stay in registers until the staged input is no longer needed
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
-    double acc[JOBS][4][2][2];
-#pragma unroll
-    for (int j = 0; j < JOBS; ++j)
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) acc[j][a][b][0] = acc[j][a][b][1] = 0.0;
-    // jobs 0, 1: rows 0..31, columns 16 j; jobs 2..5: rows 32..63
-    auto job_row = [](int job) { return job < 2 ? 0 : 4; };
-    auto job_col = [](int job) { return job < 2 ? 2 * job : 2 * (job - 2); };
-    for (int k0 = 0; k0 < m8; k0 += 4) {
-        const float *a0 = As + (k0 + lk) * st.sr;
-#pragma unroll
-        for (int j = 0; j < JOBS; ++j) {
-            const int job = 2 * j + warp, tr = job_row(job), tc = job_col(job);
-            if (tr >= nt8 || tc >= nt8) continue;
-            double fa[4], fb[2];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) fa[a] = tr + a < nt8 ? (double)a0[((tr + a) * 8 + lr) * st.sk] : 0.0;
-#pragma unroll
-            for (int b = 0; b < 2; ++b) fb[b] = tc + b < nt8 ? (double)a0[((tc + b) * 8 + lr) * st.sk] : 0.0;
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b) dmma(acc[j][a][b], fa[a], fb[b]);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < JOBS; ++j) {
-        const int job = 2 * j + warp, tr = job_row(job), tc = job_col(job);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                if (tr + a >= nt8 || tc + b > tr + a) continue;
-                const int r = (tr + a) * 8 + lr, c = (tc + b) * 8 + 2 * lk;
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    G[(size_t)r * ld + c + e] = acc[j][a][b][e];
-                    if (tc + b < tr + a) G[(size_t)(c + e) * ld + r] = acc[j][a][b][e];
-                }
-            }
-    }
-    __syncthreads();
-}
-
-__global__ void __launch_bounds__(kPreT, 7) precondition_kernel(Params p) {
+__global__ void __launch_bounds__(kPreT, 8) precondition_kernel(Params p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_idx;
-    int *prow = (int *)smem;
-    double *sd = (double *)(smem + 64 * 4);
-    unsigned *skey = (unsigned *)(smem + 64 * 4 + 64 * 8);
-    double *G = (double *)(smem + 64 * 4 + 64 * 8 + 16);
+    float *xb = (float *)smem;
     const float exit_ratio = p.exit_ratio == 0.f ? kMixedExitRatio
                                                  : (p.exit_ratio < 0.f ? 10.f * Lim<float>::eps() : p.exit_ratio);
     for (;;) {
@@ -466,55 +435,207 @@ __global__ void __launch_bounds__(kPreT, 7) precondition_kernel(Params p) {
         if (idx >= p.count) break;
         const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
         const jb_matrix_desc d = desc_of(p, mat);
-        int st = JB_ST_OK, ns = 0;
+        if (p.status[mat] != JB_ST_OK) continue;
+        const int nt = d.m > d.n ? d.n : d.m, most = p.max_sweeps32;
+        float *x = p.x32 + d.x_off;
+        int ns;
+        if (nt > 48) ns = precondition_sweeps<4, 8>(xb, nt, exit_ratio, most, x);
+        else if (nt > 32) ns = precondition_sweeps<4, 6>(xb, nt, exit_ratio, most, x);
+        else if (nt > 16) ns = precondition_sweeps<2, 4>(xb, nt, exit_ratio, most, x);
+        else ns = precondition_sweeps<1, 2>(xb, nt, exit_ratio, most, x);
+        if (threadIdx.x == 0) {
+            p.sweeps[mat] = ns;
+            if (ns > most) {
+                p.status[mat] = kPending;
+                atomicAdd(p.n_pending, 1);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The factor L.
+// ---------------------------------------------------------------------------
+// Pivoted Cholesky of G (n x n, both triangles, ld), thread i = row i, by one
+// warp (n <= 32) or two: step k takes the largest remaining diagonal p and
+// leaves column k of L in row p of G (rows chosen before: zero), p * ld in
+// prow[k].  The pivot is found on FP32 keys that carry the row (redux); one
+// barrier a step.  scl brings the largest diagonal to about 1, rscl is its
+// square root.  False when a pivot is <= cut (scaled).
+template <int WARPS>
+__device__ __forceinline__ bool pivoted_cholesky(double *G, int ld, int n, double cut, double scl, double rscl,
+                                                 int *prow, double2 *sd, unsigned *skey) {
+    const int i = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double d = i < n ? G[i * ld + i] : 0.0;
+    bool taken = i >= n;
+    double *gi = G + min(i, ld - 1);
+    for (int k = 0; k < n; ++k) {
+        const float df = (float)(d * scl);
+        const unsigned key = taken ? 0u : ((__float_as_uint(fmaxf(df, 0.f)) & ~63u) | (63 - i)) + 64u;
+        unsigned kw = __reduce_max_sync(FULL, key);
+        // 1 / sqrt(d): FP32 estimate, one Newton step (1e-14)
+        const double r0 = (double)rsqrt_ftz(df);
+        const double rs = r0 * fma(-0.5 * (d * scl), r0 * r0, 1.5) * rscl;
+        if (!taken) sd[i] = make_double2(d, rs);
+        if (WARPS == 2) {
+            if (lane == 0) skey[2 * (k & 1) + warp] = kw;
+            asm volatile("bar.sync 1, 64;" ::: "memory");
+            const uint2 ks = *(const uint2 *)(skey + 2 * (k & 1));
+            kw = max(ks.x, ks.y);
+        } else {
+            __syncwarp();
+        }
+        const int p = 63 - (int)(kw & 63u);
+        const double2 dr = sd[p];
+        if (!(dr.x * scl > cut)) return false;
+        const double *gq = G + p;
+        double v0 = gi[p * ld], v1 = 0.0, v2 = 0.0, v3 = 0.0;
+        int j = 0;
+#pragma unroll 2
+        for (; j + 4 <= k; j += 4) {
+            const int4 r = *(const int4 *)(prow + j);
+            v0 = fma(-gi[r.x], gq[r.x], v0);
+            v1 = fma(-gi[r.y], gq[r.y], v1);
+            v2 = fma(-gi[r.z], gq[r.z], v2);
+            v3 = fma(-gi[r.w], gq[r.w], v3);
+        }
+#pragma unroll 1
+        for (; j < k; ++j) v0 = fma(-gi[prow[j]], gq[prow[j]], v0);
+        const double l = taken ? 0.0 : (i == p ? dr.x : (v0 + v1) + (v2 + v3)) * dr.y;
+        if (i < ld) gi[p * ld] = l;
+        if (i == p) taken = true;
+        d = fma(-l, l, d);
+        if (i == 0) prow[k] = p * ld;
+    }
+    return true;
+}
+
+// Shared memory: prow (64 ints), sd (64 double2), skey (8), two words, then G
+// (n8 x n8 doubles) and the staged input in one place.
+constexpr size_t kFacHead = 64 * 4 + 64 * 16 + 8 * 4 + 4 * 4;
+__host__ __device__ inline size_t fac_smem(int mt, int nt) {
+    const int m8 = round8(mt), n8 = round8(nt);
+    const size_t g = (size_t)n8 * n8 * 8, a = stage_floats(m8, n8) * 4;
+    return kFacHead + (g > a ? g : a);
+}
+
+// Lower 16 x 16 blocks of G over four warps, at most three a warp; all sums
+// stay in registers until the staged input is no longer needed.
+template <int JOBS>
+__device__ __forceinline__ void gram_tiles(const float *As, Stage st, int m8, int nt8, double *G, int ld) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    double acc[JOBS][2][2][2];
+    int tr[JOBS], tc[JOBS];
+    bool own[JOBS];
+#pragma unroll
+    for (int j = 0; j < JOBS; ++j) {
+        int g = 0, job = warp + 4 * j;   // block row g has g + 1 blocks
+        while (job > g) { job -= g + 1; ++g; }
+        tr[j] = 2 * g;
+        tc[j] = 2 * job;
+        own[j] = tr[j] < nt8;
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) acc[j][a][b][0] = acc[j][a][b][1] = 0.0;
+    }
+    const int last = nt8 - 1;
+    const float *a0 = As + lk * st.sr + lr * st.sk;
+#pragma unroll 2
+    for (int k0 = 0; k0 < m8; k0 += 4, a0 += 4 * st.sr) {
+#pragma unroll
+        for (int j = 0; j < JOBS; ++j) {
+            if (!own[j]) continue;
+            double fa[2], fb[2];
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                fa[a] = (double)a0[min(tr[j] + a, last) * 8 * st.sk];
+                fb[a] = (double)a0[min(tc[j] + a, last) * 8 * st.sk];
+            }
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) dmma(acc[j][a][b], fa[a], fb[b]);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < JOBS; ++j)
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                if (tr[j] + a >= nt8 || tc[j] + b > tr[j] + a) continue;
+                const int r = (tr[j] + a) * 8 + lr, c = (tc[j] + b) * 8 + 2 * lk;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    G[(size_t)r * ld + c + e] = acc[j][a][b][e];
+                    if (tc[j] + b < tr[j] + a) G[(size_t)(c + e) * ld + r] = acc[j][a][b][e];
+                }
+            }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kFacT, 6) factor_kernel(Params p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    int *prow = (int *)smem;
+    double2 *sd = (double2 *)(smem + 64 * 4);
+    unsigned *skey = (unsigned *)(smem + 64 * 4 + 64 * 16);
+    int *sex = (int *)(skey + 8);
+    double *G = (double *)(smem + kFacHead);
+    for (int64_t idx = blockIdx.x; idx < p.count; idx += gridDim.x) {
+        const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
+        const jb_matrix_desc d = desc_of(p, mat);
+        int st = JB_ST_OK;
         const int mt = d.m > d.n ? d.m : d.n, nt = d.m > d.n ? d.n : d.m;
         if (!rdesc_fits(d, kB32, 4, p, true)) {
             st = JB_ST_BAD_DESC;
         } else if ((d.flags & JB_FULL_MATRICES) && mt > nt) {
             st = kPending;
         } else {
-            const bool wide = d.m < d.n;
-            const int m8 = round8(mt), n8 = round8(nt), ld = pre_ld(n8);
-            const Stage sg = stage_of(wide, m8, n8);
+            const int m8 = round8(mt), n8 = round8(nt), ld = n8;
+            const Stage sg = stage_of(d.m < d.n, m8, n8);
             float *As = (float *)G;
-            const float *A = (const float *)p.A + d.a_off;
-            if (wide) stage_input<kPreT>(A, d.m, d.n, n8, m8, sg.sk, As);
-            else stage_input<kPreT>(A, d.m, d.n, m8, n8, sg.sr, As);
+            stage_tall((const float *)p.A + d.a_off, d, m8, n8, sg, As, kFacT);
+            if (threadIdx.x < 64) prow[threadIdx.x] = 0;
             __syncthreads();
             if (nt > 32) gram_tiles<3>(As, sg, m8, n8 >> 3, G, ld);
             else gram_tiles<1>(As, sg, m8, n8 >> 3, G, ld);
             // a diagonal of G is not finite exactly when the input is not
             const double gd = threadIdx.x < nt ? G[(size_t)threadIdx.x * ld + threadIdx.x] : 0.0;
-            const bool bad = __syncthreads_or(!isfinite(gd));
-            // power of two that brings the largest diagonal into [1, 2)
             const int ex = __reduce_max_sync(FULL, (__double2hiint(fabs(gd)) >> 20) & 0x7ff);
-            if ((threadIdx.x & 31) == 0) prow[threadIdx.x >> 5] = ex;
-            __syncthreads();
-            const int em = max(prow[0], prow[1]);
-            __syncthreads();
+            if ((threadIdx.x & 31) == 0) sex[threadIdx.x >> 5] = ex;
+            const bool bad = __syncthreads_or(!isfinite(gd));
+            const int em = max(sex[0], sex[1]);   // nt <= 64: the first two warps
             if (bad) {
                 st = JB_ST_NONFINITE_IN;
-            } else if (em == 0) {
-                st = kPending;   // zero matrix
+            } else if (em < 32) {
+                st = kPending;   // zero, or the squares near the bottom of FP64's range
             } else {
-                const double gscl = __hiloint2double((2046 - em) << 20, 0);
-                // sqrt of it, within a factor 2, for the columns of L
-                const double lscl = __hiloint2double((1023 - ((em - 1023) >> 1)) << 20, 0);
-                if (!pivoted_cholesky(G, ld, nt, kPivotCut / gscl, gscl, prow, sd, skey)) {
+                // even power of two that brings the largest diagonal into [1, 4)
+                const int half = (em - 1023) >> 1;
+                const double scl = __hiloint2double((1023 - 2 * half) << 20, 0);
+                const double rscl = __hiloint2double((1023 - half) << 20, 0);
+                bool ok = true;
+                if (nt > 32) {
+                    if (threadIdx.x < 64) ok = pivoted_cholesky<2>(G, ld, nt, kPivotCut, scl, rscl, prow, sd, skey);
+                } else {
+                    if (threadIdx.x < 32) ok = pivoted_cholesky<1>(G, ld, nt, kPivotCut, scl, rscl, prow, sd, skey);
+                }
+                if (__syncthreads_or(!ok)) {
                     st = kPending;
                 } else {
                     float *x = p.x32 + d.x_off;
-                    if (nt > 48) ns = precondition_sweeps<4, 8>(G, ld, prow, lscl, nt, exit_ratio, p.max_sweeps32, x);
-                    else if (nt > 32) ns = precondition_sweeps<4, 6>(G, ld, prow, lscl, nt, exit_ratio, p.max_sweeps32, x);
-                    else if (nt > 16) ns = precondition_sweeps<2, 4>(G, ld, prow, lscl, nt, exit_ratio, p.max_sweeps32, x);
-                    else ns = precondition_sweeps<1, 2>(G, ld, prow, lscl, nt, exit_ratio, p.max_sweeps32, x);
-                    if (ns > p.max_sweeps32) st = kPending;
+                    for (int c = threadIdx.x >> 5; c < nt; c += kFacT / 32)
+                        for (int i = threadIdx.x & 31; i < nt; i += 32)
+                            x[c * nt + i] = (float)(G[prow[c] + i] * rscl);
                 }
             }
         }
         if (threadIdx.x == 0) {
             p.status[mat] = st;
-            p.sweeps[mat] = ns;
+            p.sweeps[mat] = 0;
             if (st == kPending) atomicAdd(p.n_pending, 1);
         }
         __syncthreads();
@@ -524,8 +645,10 @@ __global__ void __launch_bounds__(kPreT, 7) precondition_kernel(Params p) {
 // ---------------------------------------------------------------------------
 // FP64 refinement.  Eight warps a matrix; V (n8 x ldv) and W (n8 x ldw,
 // column-major, FP64) in shared memory, the staged input and N in W's place
-// while W is not needed.  Bound by the f64 mma pipe: 3 n^3 + 6 m n^2 flop for
-// the usual one correction and its check.
+// while W is not needed: 102 KB at 128 x 64, two matrices an SM.  The floor is
+// the f64 mma pipe, 4 n^3 + 6 m n^2 flop for the usual one correction and its
+// check (0.30 ms of the uneven batch's 1.01); barriers between the products
+// and the shared-memory latency of their operands take the rest.
 // ---------------------------------------------------------------------------
 struct RefGeo {
     int m8, n8, ldv, ldw;
@@ -546,53 +669,72 @@ __host__ __device__ inline size_t ref_smem(int mt, int nt) {
     return (size_t)r.n8 * r.ldv * 8 + w + (size_t)64 * 8 * 3 + 64 * 4;
 }
 
-// W = A V: blocks of 16 x 32 over the warps, at most two a warp (m <= 128, n <= 64).
-__device__ __forceinline__ void ref_w(const float *As, Stage st, const double *V, int ldv, double *W, int ldw, int mt8,
-                                      int nt8) {
+// C (mt8 x nt8 tiles, column-major) = (ADD ? C : 0) + X Y over k8, in blocks
+// of 16 rows and NB column tiles a warp, S blocks a warp at most.  X(i, k) at
+// x[i * sr + k * sk], Y(k, j) at y[j * ldy + k].  C is written once every
+// warp is done reading: it may take X's or Y's place.  Rows and columns of a
+// block past the end repeat the last tile; their results are not stored.
+template <int NB, int S, bool ADD, typename TX>
+__device__ __forceinline__ void ref_mul(const TX *x, int sr, int sk, const double *y, int ldy, double *C, int ldc,
+                                        int k8, int mt8, int nt8) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
-    const int bm = (mt8 + 1) >> 1, bn = (nt8 + 3) >> 2;
-    double acc[2][2][4][2];
+    const int bm = (mt8 + 1) >> 1, blocks = bm * ((nt8 + NB - 1) / NB);
+    double acc[S][2][NB][2];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[s][a][b][0] = acc[s][a][b][1] = 0.0;
+    for (int s = 0; s < S; ++s) {
         const int blk = warp + 8 * s;
-        if (blk >= bm * bn) continue;
-        const int tr = 2 * (blk % bm), tc = 4 * (blk / bm);
-        for (int k0 = 0; k0 < 8 * nt8; k0 += 4) {
-            double fa[2], fb[4];
 #pragma unroll
-            for (int a = 0; a < 2; ++a)
-                fa[a] = tr + a < mt8 ? (double)As[((tr + a) * 8 + lr) * st.sr + (k0 + lk) * st.sk] : 0.0;
+        for (int b = 0; b < NB; ++b)
+            acc[s][0][b][0] = acc[s][0][b][1] = acc[s][1][b][0] = acc[s][1][b][1] = 0.0;
+        if (blk < blocks) {
+            const int tr = 2 * (blk % bm), tc = NB * (blk / bm);
+            const TX *xa = x + (tr * 8 + lr) * sr + lk * sk;
+            const TX *xb = x + (min(tr + 1, mt8 - 1) * 8 + lr) * sr + lk * sk;
+            const double *yb[NB];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) fb[b] = tc + b < nt8 ? V[((tc + b) * 8 + lr) * ldv + k0 + lk] : 0.0;
+            for (int b = 0; b < NB; ++b) yb[b] = y + (min(tc + b, nt8 - 1) * 8 + lr) * ldy + lk;
+#pragma unroll 2
+            for (int k0 = 0; k0 < k8; k0 += 4) {
+                const double fa = (double)xa[k0 * sk], fb = (double)xb[k0 * sk];
 #pragma unroll
-            for (int b = 0; b < 4; ++b)
-                if (tc + b < nt8) {
-#pragma unroll
-                    for (int a = 0; a < 2; ++a) dmma(acc[s][a][b], fa[a], fb[b]);
+                for (int b = 0; b < NB; ++b) {
+                    const double f = yb[b][k0];
+                    dmma(acc[s][0][b], fa, f);
+                    dmma(acc[s][1][b], fb, f);
                 }
+            }
         }
     }
-    __syncthreads();   // the staged input gives way to W
+    __syncthreads();
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < S; ++s) {
         const int blk = warp + 8 * s;
-        if (blk >= bm * bn) continue;
-        const int tr = 2 * (blk % bm), tc = 4 * (blk / bm);
+        if (blk < blocks) {
+            const int tr = 2 * (blk % bm), tc = NB * (blk / bm);
 #pragma unroll
-        for (int a = 0; a < 2; ++a)
+            for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b)
-                if (tr + a < mt8 && tc + b < nt8) {
-                    double *w = W + (size_t)((tc + b) * 8 + 2 * lk) * ldw + (tr + a) * 8 + lr;
-                    w[0] = acc[s][a][b][0];
-                    w[ldw] = acc[s][a][b][1];
-                }
+                for (int b = 0; b < NB; ++b)
+                    if (tr + a < mt8 && tc + b < nt8) {
+                        double *w = C + ((tc + b) * 8 + 2 * lk) * ldc + (tr + a) * 8 + lr;
+                        w[0] = acc[s][a][b][0] + (ADD ? w[0] : 0.0);
+                        w[ldc] = acc[s][a][b][1] + (ADD ? w[ldc] : 0.0);
+                    }
+        }
     }
 }
+// W = A V with A staged in W's place, and V <- V + V N, with the block width
+// (3 or 4 column tiles) that leaves the fewest idle.
+template <int NB>
+__device__ __forceinline__ void ref_w(const float *As, Stage st, const double *V, int ldv, double *W, int ldw, int mt8,
+                                      int nt8) {
+    ref_mul<NB, 2, false>(As, st.sr, st.sk, V, ldv, W, ldw, 8 * nt8, mt8, nt8);
+}
+template <int NB>
+__device__ __forceinline__ void ref_v(double *V, int ldv, const double *Nm, int nt8) {
+    ref_mul<NB, 1, true>(V, 1, ldv, Nm, ldv, V, ldv, 8 * nt8, nt8, nt8);
+}
+__device__ __forceinline__ bool ref_three(int nt8) { return nt8 == 3 || nt8 == 5 || nt8 == 6; }
 
 // Lower 16 x 8 blocks of X^T X (X column-major, ld, rows8 rows): three jobs a warp at most.
 __device__ __forceinline__ void job_place(int job, int &tr, int &tc) {
@@ -639,11 +781,16 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
         int64_t idx;
         next_ticket(p.counter2, s_idx, idx);
         if (idx >= p.count) break;
-        const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
-        const jb_matrix_desc d = desc_of(p, mat);
+        const int mat = p.order ? p.order[idx] : (int)idx;
         if (p.status[mat] != JB_ST_OK) continue;
-        const bool wide = d.m < d.n;
-        const int mt = wide ? d.n : d.m, nt = wide ? d.m : d.n;
+        int mt, nt;
+        bool wide;
+        {
+            const jb_matrix_desc d = desc_of(p, mat);
+            wide = d.m < d.n;
+            mt = wide ? d.n : d.m;
+            nt = wide ? d.m : d.n;
+        }
         const RefGeo g = ref_geo(mt, nt);
         const int ldv = g.ldv, ldw = g.ldw, nt8 = g.n8 >> 3, mt8 = g.m8 >> 3;
         double *dh = (double *)smem, *de = dh + 64, *sig = de + 64;   // diagonals of H and E; sigma
@@ -653,23 +800,24 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
         double *Nm = W;                       // n8 x ldv
         float *As = (float *)W;
         const Stage sg = stage_of(wide, g.m8, g.n8);
-        const float *A = (const float *)p.A + d.a_off;
-        const float *x = p.x32 + d.x_off;
-        for (int k = threadIdx.x; k < g.n8 * g.n8; k += kRefT) {
-            const int c = k / g.n8, i = k - c * g.n8;
-            V[c * ldv + i] = (c < nt && i < nt) ? (double)x[c * nt + i] : 0.0;
+        {
+            const float *x = p.x32 + desc_of(p, mat).x_off;
+            for (int c = warp; c < g.n8; c += kRefT / 32)
+                for (int i = lane; i < g.n8; i += 32)
+                    V[c * ldv + i] = (c < nt && i < nt) ? (double)x[c * nt + i] : 0.0;
         }
-        const double tol = p.tol > 0 ? (double)(float)p.tol : (double)(10.0f * Lim<float>::eps());
-        const double tol2 = tol * tol;
         const int nb16 = (nt8 + 1) >> 1, jobs = nb16 * (nb16 + 1);
         const int most = p.max_sweeps < kRefPasses ? p.max_sweeps : kRefPasses;
         int pass = 1;
         bool done = false;
         for (; pass <= most; ++pass) {
-            if (wide) stage_input<kRefT>(A, d.m, d.n, g.n8, g.m8, sg.sk, As);
-            else stage_input<kRefT>(A, d.m, d.n, g.m8, g.n8, sg.sr, As);
+            {
+                const jb_matrix_desc d = desc_of(p, mat);
+                stage_tall((const float *)p.A + d.a_off, d, g.m8, g.n8, sg, As, kRefT);
+            }
             __syncthreads();
-            ref_w(As, sg, V, ldv, W, ldw, mt8, nt8);
+            if (ref_three(nt8)) ref_w<3>(As, sg, V, ldv, W, ldw, mt8, nt8);
+            else ref_w<4>(As, sg, V, ldv, W, ldw, mt8, nt8);
             __syncthreads();
             double h[3][2][2], e[3][2][2];
 #pragma unroll
@@ -693,6 +841,8 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
                     }
             }
             __syncthreads();
+            const double tol = p.tol > 0 ? (double)(float)p.tol : (double)(10.0f * Lim<float>::eps());
+            const double tol2 = tol * tol;
             int need = 0;
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
@@ -757,51 +907,11 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
                     sum = fma(k, k, sum);
                 }
                 sum = warp_sum(sum);
-                if (lane == 0) dh[j] = -0.5 * sum;
+                if (lane == 0) Nm[j * ldv + j] -= 0.5 * sum;
             }
             __syncthreads();
-            // V <- V + V N: one 16 x 32 block a warp
-            {
-                const int bm = (nt8 + 1) >> 1, bn = (nt8 + 3) >> 2;
-                double acc[2][4][2];
-#pragma unroll
-                for (int a = 0; a < 2; ++a)
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-                const int tr = 2 * (warp % bm), tc = 4 * (warp / bm);
-                const bool own = warp < bm * bn;
-                if (own) {
-                    for (int k0 = 0; k0 < g.n8; k0 += 4) {
-                        double fa[2], fb[4];
-#pragma unroll
-                        for (int a = 0; a < 2; ++a)
-                            fa[a] = tr + a < nt8 ? V[(k0 + lk) * ldv + (tr + a) * 8 + lr] : 0.0;
-#pragma unroll
-                        for (int b = 0; b < 4; ++b) {
-                            const int c = (tc + b) * 8 + lr;
-                            fb[b] = tc + b < nt8 ? Nm[c * ldv + k0 + lk] + (c == k0 + lk && c < nt ? dh[c] : 0.0) : 0.0;
-                        }
-#pragma unroll
-                        for (int b = 0; b < 4; ++b)
-                            if (tc + b < nt8) {
-#pragma unroll
-                                for (int a = 0; a < 2; ++a) dmma(acc[a][b], fa[a], fb[b]);
-                            }
-                    }
-                }
-                __syncthreads();
-                if (own) {
-#pragma unroll
-                    for (int a = 0; a < 2; ++a)
-#pragma unroll
-                        for (int b = 0; b < 4; ++b)
-                            if (tr + a < nt8 && tc + b < nt8) {
-                                double *v = V + (size_t)((tc + b) * 8 + 2 * lk) * ldv + (tr + a) * 8 + lr;
-                                v[0] += acc[a][b][0];
-                                v[ldv] += acc[a][b][1];
-                            }
-                }
-            }
+            if (ref_three(nt8)) ref_v<3>(V, ldv, Nm, nt8);
+            else ref_v<4>(V, ldv, Nm, nt8);
         }
         // sigma, the stable descending order and the cut (primitives.py:356-366)
         int st = JB_ST_OK;
@@ -833,6 +943,7 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
         if (!done) {
             st = kPending;
         } else {
+            const jb_matrix_desc d = desc_of(p, mat);
             float *U = p.U ? (float *)p.U + d.u_off : nullptr;
             float *Vh = p.Vh ? (float *)p.Vh + d.v_off : nullptr;
             float *S = (float *)p.S + d.s_off;
