@@ -17,6 +17,7 @@
 #include "jb_device.cuh"
 #include "jb_regblock.cuh"
 #include "jb_gram64.cuh"
+#include "jb_group.cuh"
 
 namespace jb {
 
@@ -282,9 +283,9 @@ constexpr int kTuneFlags = JB_ROUND_ROBIN | JB_BLOCK_WIDTH_8 | JB_ONE_SIZE_CLASS
 constexpr int kB64 = 2;   // block width of the FP64 sweeps (16 warps for 64 columns)
 constexpr int kT32 = 256, kT64 = 512;  // threads of the two kernels
 constexpr int kMaxR = 4;  // rows per lane: mt <= 128
-// Size classes of the register path: matrices with nt <= kNarrowN occupy at
-// most half of the warps of a CTA (kT32 / kT64), so they run in a second
-// launch with CTAs of half the size and twice as many CTAs per SM.
+// Size classes of an uneven FP32 batch: matrices with nt <= kNarrowN occupy at
+// most half of the warps of a CTA, so they run in a second launch with CTAs of
+// half the size and twice as many CTAs per SM.
 constexpr int kNarrowN = 32;
 constexpr int kMaxRV = 2; // V rows per lane: padded width <= 64
 // Large-tile FP32 kernel (one matrix up to 256 x 128 per CTA, 16 warps).
@@ -517,7 +518,6 @@ __global__ void __launch_bounds__(THREADS, (BW == kB32 && MR <= kMaxR) ? 512 / T
         if (idx >= p.count) break;
         const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
         const jb_matrix_desc d = desc_of(p, mat);
-        if (!class_takes(d, p.cls)) continue;  // the other size class's launch solves it
         if (p.pending && p.status[mat] != kPending) continue;
         if (threadIdx.x < 4) ax.flag[threadIdx.x] = 0;
         __syncthreads();
@@ -600,14 +600,11 @@ __global__ void __launch_bounds__(THREADS, (BW == kB32 && MR <= kMaxR) ? 512 / T
 }
 
 
-// K2: FP64 sweeps.  MIXED (TI = float): start from the FP32 V of K1, made
-// orthogonal by Newton-Schulz polar steps to well below the FP32 rounding of
-// the outputs (it is orthogonal to ~1e-5 already), with W = A V recomputed
-// in FP64 from the exact input;
-// native (TI = double): start from V = I.  Runs the epilogue and writes U,
-// S, Vh in TI.
-template <typename TI, bool MIXED, int THREADS = kT64>
-__global__ void __launch_bounds__(THREADS, kT64 / THREADS) rb64_kernel(Params p) {
+// K2: FP64 sweeps of a float32 matrix from the FP32 V of K1, made orthogonal by
+// Newton-Schulz polar steps to well below the FP32 rounding of the outputs
+// (it is orthogonal to ~1e-5 already), with W = A V recomputed in FP64 from
+// the exact input.  Runs the epilogue and writes U, S, Vh.
+__global__ void __launch_bounds__(kT64, 1) rb64_kernel(Params p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_idx;
     Aux ax = carve_aux(smem, p.maxd);
@@ -615,30 +612,30 @@ __global__ void __launch_bounds__(THREADS, kT64 / THREADS) rb64_kernel(Params p)
     if (p.pending && *p.n_pending == 0) return;
     for (;;) {
         int64_t idx;
-        next_ticket(MIXED ? p.counter2 : p.counter, s_idx, idx);
+        next_ticket(p.counter2, s_idx, idx);
         if (idx >= p.count) break;
         const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
         const jb_matrix_desc d = desc_of(p, mat);
-        if (!class_takes(d, p.cls)) continue;  // the other size class's launch solves it
         if (threadIdx.x < 4) ax.flag[threadIdx.x] = 0;
         __syncthreads();
         int prev = JB_ST_OK, s1 = 0, e_k1 = 0;
         bool have_e = false;
-        if (MIXED && threadIdx.x == 0) { ax.flag[3] = p.status[mat]; ax.flag[2] = p.sweeps[mat]; }
+        if (threadIdx.x == 0) { ax.flag[3] = p.status[mat]; ax.flag[2] = p.sweeps[mat]; }
         __syncthreads();
-        if (MIXED) { prev = ax.flag[3]; have_e = unpack_handoff(ax.flag[2], s1, e_k1); }
+        prev = ax.flag[3];
+        have_e = unpack_handoff(ax.flag[2], s1, e_k1);
         __syncthreads();
         if (threadIdx.x == 0) ax.flag[2] = 0;
         __syncthreads();
         if (prev != (p.pending ? kHanded : JB_ST_OK)) continue;  // already reported
         int ns = s1, st = JB_ST_OK;
-        if (!rdesc_fits(d, kB64, 8, p, MIXED)) {
+        if (!rdesc_fits(d, kB64, 8, p, true)) {
             st = JB_ST_BAD_DESC;
         } else {
             const int mt = d.m > d.n ? d.m : d.n, nt = d.m > d.n ? d.n : d.m;
             const RGeo r = rgeo(mt, nt, kB64, d.flags);
             const Geo g = reg_geo(d, r);
-            const TI *A = (const TI *)p.A + d.a_off;
+            const float *A = (const float *)p.A + d.a_off;
             double *W = (double *)region;
             double *V = (double *)(region + align16((size_t)r.ldw * r.ncp * 8));
             bool bad = false;
@@ -648,11 +645,8 @@ __global__ void __launch_bounds__(THREADS, kT64 / THREADS) rb64_kernel(Params p)
                 st = JB_ST_NONFINITE_IN;
             } else {
                 zero_fill(V, (size_t)r.ldv * r.npb);
-                if (!MIXED) zero_fill(W, (size_t)r.ldw * r.ncp);
                 __syncthreads();
-                if (!MIXED) {
-                    load_padded(A, g, r, e, W, V);
-                } else {
+                {
                     double *X1 = (double *)(region + rregion_bytes(r, 8));
                     unsigned char *X2 = region + rregion_bytes(r, 8) + align16((size_t)r.ldv * r.npb * 8);
                     const float *x = p.x32 + d.x_off;
@@ -683,19 +677,18 @@ __global__ void __launch_bounds__(THREADS, kT64 / THREADS) rb64_kernel(Params p)
                         for (int i = threadIdx.x; i < r.ldw; i += blockDim.x) W[(size_t)j * r.ldw + i] = 0.0;
                 }
                 __syncthreads();
-                const double tol = MIXED ? (p.tol > 0 ? (double)(float)p.tol : (double)(10.0f * Lim<float>::eps()))
-                                         : (p.tol > 0 ? p.tol : 10.0 * Lim<double>::eps());
+                const double tol = p.tol > 0 ? (double)(float)p.tol : (double)(10.0f * Lim<float>::eps());
                 bool conv;
-                // MIXED: norm updates carried through ax.sig (rb_sweeps UPD 2); the
+                // norm updates carried through ax.sig (rb_sweeps UPD 2); the
                 // confirming Gram pass that ends the solve measures exact norms.
-                ns += rb_dispatch<double, kB64, kMaxR, kMaxRV, MIXED ? 2 : 0>(r, W, V, tol, p.max_sweeps, true, ax.red,
+                ns += rb_dispatch<double, kB64, kMaxR, kMaxRV, 2>(r, W, V, tol, p.max_sweeps, true, ax.red,
                                                                           conv, 0.0, ax.sig);
                 if (!conv) {
                     st = JB_ST_NOT_CONVERGED;
                 } else {
-                    TI *U = p.U ? (TI *)p.U + d.u_off : nullptr;
-                    TI *Vh = p.Vh ? (TI *)p.Vh + d.v_off : nullptr;
-                    st = epilogue<double, TI>(W, V, g, e, U, (TI *)p.S + d.s_off, Vh, ax);
+                    float *U = p.U ? (float *)p.U + d.u_off : nullptr;
+                    float *Vh = p.Vh ? (float *)p.Vh + d.v_off : nullptr;
+                    st = epilogue<double, float>(W, V, g, e, U, (float *)p.S + d.s_off, Vh, ax);
                 }
             }
         }
@@ -707,6 +700,110 @@ __global__ void __launch_bounds__(THREADS, kT64 / THREADS) rb64_kernel(Params p)
     }
 }
 
+
+// Native solve by group_sweeps (jb_group.cuh).
+template <typename R, int GL, int B, int RW, int RV>
+struct GroupKernel {
+    using C = GroupCfg<R, 1, GL, B, RW, RV>;
+    __host__ __device__ static Dims dims(int mt, int nt, int flags) {
+        Dims d;
+        d.mt = mt; d.nt = nt;
+        d.np = 2 * B * ((nt + 2 * B - 1) / (2 * B));
+        d.ncp = (flags & JB_FULL_MATRICES) ? d.np + (mt - nt) : d.np;
+        d.ldw = d.ldv = C::LD;
+        return d;
+    }
+    __host__ __device__ static size_t smem(int mt, int nt, int flags) {
+        const Dims d = dims(mt, nt, flags);
+        return aux_bytes(d) + align16((size_t)d.np * 8) + (size_t)d.ncp * C::LD * sizeof(R);
+    }
+};
+
+// One matrix by the whole CTA; every thread returns its status.
+template <typename R, int GL, int B, int RW, int RV, int THREADS>
+__device__ int group_solve(const Params &p, const jb_matrix_desc &d, unsigned char *smem, int &ns) {
+    using K = GroupKernel<R, GL, B, RW, RV>;
+    constexpr int LD = K::C::LD;
+    const int mt = d.m > d.n ? d.m : d.n, nt = d.m > d.n ? d.n : d.m;
+    const Dims dd = K::dims(mt, nt, d.flags);
+    Aux ax = carve_aux(smem, dd);
+    double *scales = (double *)(smem + aux_bytes(dd));
+    R *W = (R *)(smem + aux_bytes(dd) + align16((size_t)dd.np * 8));
+    R *V = W + K::C::VOFF;
+    Geo g = make_geo(d.m, d.n, d.rank, d.flags);
+    g.np = dd.np;
+    g.ncp = dd.ncp;
+    g.ldw = g.ldv = LD;
+    if (threadIdx.x < 4) ax.flag[threadIdx.x] = 0;
+    const R *A = (const R *)p.A + d.a_off;
+    bool bad, conv;
+    const int e = scan_input(A, g.m * g.n, ax, bad);
+    ns = 0;
+    if (bad) return JB_ST_NONFINITE_IN;
+    zero_fill(W, (size_t)dd.ncp * LD);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < g.m * g.n; idx += THREADS) {
+        const int row = idx / g.n, col = idx - row * g.n;
+        W[(g.wide ? row : col) * LD + (g.wide ? col : row)] = dscale(A[idx], -e);
+    }
+    for (int j = threadIdx.x; j < dd.np; j += THREADS) V[j * LD + j] = R(1);
+    __syncthreads();
+    const R tol = p.tol > 0 ? (R)p.tol : R(10) * Lim<R>::eps();
+    ns = group_sweeps<R, 1, GL, B, RW, RV, THREADS>(W, nt, tol, p.max_sweeps, scales, ax.red, conv);
+    if (!conv) return JB_ST_NOT_CONVERGED;
+    R *U = p.U ? (R *)p.U + d.u_off : nullptr;
+    R *Vh = p.Vh ? (R *)p.Vh + d.v_off : nullptr;
+    return epilogue<R, R>(W, V, g, e, U, (R *)p.S + d.s_off, Vh, ax);
+}
+
+// A batch of equal shapes: one CTA a matrix.
+template <typename R, int GL, int B, int RW, int RV, int THREADS>
+__global__ void __launch_bounds__(THREADS) group_kernel(Params p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    for (int64_t mat = blockIdx.x; mat < p.count; mat += gridDim.x) {
+        int ns;
+        const int st = group_solve<R, GL, B, RW, RV, THREADS>(p, desc_of(p, mat), smem, ns);
+        if (threadIdx.x == 0) {
+            if (p.status) p.status[mat] = st;
+            if (p.sweeps) p.sweeps[mat] = ns;
+        }
+        __syncthreads();
+    }
+}
+
+// An uneven FP32 batch, one size class a launch (Params::cls): persistent CTAs,
+// matrices by ticket.  The lanes a block pair follow from the shape alone, so
+// a matrix is solved with the same sums as in a batch of its own shape.
+template <int THREADS, int RV>
+__global__ void __launch_bounds__(THREADS) group_uneven_kernel(Params p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_idx;
+    for (;;) {
+        int64_t idx;
+        next_ticket(p.counter, s_idx, idx);
+        if (idx >= p.count) break;
+        const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
+        const jb_matrix_desc d = desc_of(p, mat);
+        if (!class_takes(d, p.cls)) continue;   // the other size class's launch solves it
+        const int mt = d.m > d.n ? d.m : d.n, nt = d.m > d.n ? d.n : d.m;
+        int ns = 0, st = JB_ST_BAD_DESC;
+        if (d.m >= 1 && d.n >= 1 && d.rank >= 1 && d.rank <= nt && mt <= 128 && nt <= 8 * RV &&
+            !((d.flags & JB_FULL_MATRICES) && d.rank != nt)) {
+            if (mt <= 64) {
+                if (GroupKernel<float, 8, 2, 8, RV>::smem(mt, nt, d.flags) <= p.region_cap)
+                    st = group_solve<float, 8, 2, 8, RV, THREADS>(p, d, smem, ns);
+            } else {
+                if (GroupKernel<float, 16, 2, 8, 4>::smem(mt, nt, d.flags) <= p.region_cap)
+                    st = group_solve<float, 16, 2, 8, 4, THREADS>(p, d, smem, ns);
+            }
+        }
+        if (threadIdx.x == 0) {
+            if (p.status) p.status[mat] = st;
+            if (p.sweeps) p.sweeps[mat] = ns;
+        }
+        __syncthreads();
+    }
+}
 
 // K2 of the mixed solve for large tiles (after rb32_kernel_t<true, kT32L>):
 // the FP64 phase on the Gram of W (jb_gram64.cuh).  Work arrays in the
@@ -953,12 +1050,10 @@ struct Plan {
     // register path: one sizing per kernel
     Dims d32, d64;
     size_t smem32, smem64, reg32, reg64;
-    // size-class split (kNarrowN): a second launch per phase for narrow matrices
+    // size-class split (kNarrowN) of an uneven FP32 batch: a second launch for narrow matrices
     bool split;
-    Dims d64n, d32n;
-    size_t smem64n, reg64n, smem32n, reg32n;
-    // FP32 tile exchange areas: offsets in the work area and size
-    size_t xoff32, xoff32n, xbytes32;
+    // FP32 tile exchange area: offset in the work area and size
+    size_t xoff32, xbytes32;
 };
 
 static Plan make_plan(int max_mt, int max_nt, int elem, int precision, int flags) {
@@ -989,18 +1084,6 @@ static Plan make_plan(int max_mt, int max_nt, int elem, int precision, int flags
         pl.smem64 = aux_bytes(pl.d64) + pl.reg64;
         if (pl.smem64 > kSmemLimit || pl.smem32 > kSmemLimit) pl.reg = false;
         pl.split = pl.reg && pl.bw == kB32 && max_nt > kNarrowN && !(flags & JB_ONE_SIZE_CLASS);
-        if (pl.split) {
-            const RGeo r32n = rgeo(max_mt, kNarrowN, kB32, flags);
-            pl.d32n = raux_dims(r32n);
-            pl.reg32n = rregion_bytes(r32n, 4);
-            pl.xoff32n = pl.reg32n;
-            pl.smem32n = aux_bytes(pl.d32n) + pl.reg32n + xchg_bytes(r32n.npb, kMaxR, kMaxRV);
-            const RGeo r64n = rgeo(max_mt, kNarrowN, kB64, flags);
-            pl.d64n = raux_dims(r64n);
-            pl.reg64n = (elem == 4 && precision == JB_PREC_MIXED) ? rregion_mixed64(r64n, kNarrowN)
-                                                                   : rregion_bytes(r64n, 8);
-            pl.smem64n = aux_bytes(pl.d64n) + pl.reg64n;
-        }
     }
     const RGeo r32l = rgeo(max_mt, max_nt, kB32L, flags);
     if (!pl.reg && elem == 4 && !(flags & JB_ROUND_ROBIN) && r32l.R <= kMaxRL && r32l.RV <= kMaxRVL &&
@@ -1080,12 +1163,67 @@ static int launch_rr(Params &p, const Plan &pl, unsigned char *ws, size_t ws_byt
 
 static int launch_gram(Params &p, const Plan &pl, unsigned char *ws, size_t ws_bytes, cudaStream_t st);
 
+template <typename R, int GL, int B, int RW, int RV, int THREADS>
+static int launch_group_as(Params &p, int mt, int nt, cudaStream_t st) {
+    auto kern = group_kernel<R, GL, B, RW, RV, THREADS>;
+    const size_t smem = GroupKernel<R, GL, B, RW, RV>::smem(mt, nt, p.uflags);
+    int64_t grid;
+    const int rc = occupancy_grid(kern, THREADS, smem, p.count, grid);
+    if (rc) return rc;
+    kern<<<(unsigned)(p.count < kMaxGrid ? p.count : kMaxGrid), THREADS, smem, st>>>(p);
+    return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
+}
+
+// Equal shapes in the input's precision, up to 128 x 64: lanes a block pair and
+// rows a lane from the shape (the registers hold 2B columns of W and V a
+// group, at most 96 of them).  Full bases fit too: at most 131 columns, 203 KB.
+// B200, ms a batch, this / one warp a block pair (jb_regblock.cuh): 1024 x
+// 64 x 32 FP64 0.72 / 2.00, 2048 x 45 x 61 FP32 1.29 / 2.15.
+static int launch_group(Params &p, int elem, cudaStream_t st) {
+    const int mt = p.um > p.un ? p.um : p.un, nt = p.um > p.un ? p.un : p.um;
+    if (elem == 8) {
+        if (nt <= 16 && mt <= 32) return launch_group_as<double, 8, 2, 4, 2, 32>(p, mt, nt, st);
+        if (nt <= 16) return launch_group_as<double, 16, 2, 8, 2, 64>(p, mt, nt, st);
+        if (nt <= 32 && mt <= 64) return launch_group_as<double, 8, 2, 8, 4, 64>(p, mt, nt, st);
+        if (nt <= 32) return launch_group_as<double, 16, 2, 8, 2, 128>(p, mt, nt, st);
+        if (mt <= 64) return launch_group_as<double, 16, 2, 4, 4, 256>(p, mt, nt, st);
+        return launch_group_as<double, 16, 2, 8, 4, 256>(p, mt, nt, st);
+    }
+    if (nt <= 16 && mt <= 32) return launch_group_as<float, 8, 2, 4, 4, 32>(p, mt, nt, st);
+    if (nt <= 32 && mt <= 64) return launch_group_as<float, 8, 2, 8, 4, 64>(p, mt, nt, st);
+    if (nt <= 32) return launch_group_as<float, 16, 2, 8, 4, 128>(p, mt, nt, st);
+    if (mt <= 64) return launch_group_as<float, 8, 2, 8, 8, 128>(p, mt, nt, st);
+    return launch_group_as<float, 16, 2, 8, 4, 256>(p, mt, nt, st);
+}
+
+// Uneven FP32 batch: widths above and up to 32 columns in a launch each (half
+// the threads for the narrow ones), or one launch.
+template <int THREADS, int RV>
+static int launch_group_uneven(Params &p, int mt, int nt, int cls, cudaStream_t st) {
+    auto kern = group_uneven_kernel<THREADS, RV>;
+    const int n8 = (nt + 7) & ~7;
+    const size_t a = GroupKernel<float, 8, 2, 8, RV>::smem(mt < 64 ? mt : 64, n8, 0);
+    const size_t b = GroupKernel<float, 16, 2, 8, 4>::smem(mt, n8, 0);
+    const size_t smem = a > b ? a : b;
+    int64_t grid;
+    const int rc = occupancy_grid(kern, THREADS, smem, p.count, grid);
+    if (rc) return rc;
+    p.cls = cls;
+    p.region_cap = smem;
+    kern<<<(unsigned)grid, THREADS, smem, st>>>(p);
+    return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
+}
+
 // elem: 4 (f32 input) or 8 (f64 input).
 static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsigned char *ws, size_t ws_bytes,
                       cudaStream_t st) {
     p.counter = (int *)ws;
     p.counter2 = (int *)ws + 1;
     const bool mixed = elem == 4 && precision == JB_PREC_MIXED;
+    // the input's own precision; the warm start and 8-column blocks are choices of
+    // the register kernels below
+    const bool group = elem == 8 || (!mixed && !p.vstart && pl.bw == kB32);
+    if (group && !p.descs) return launch_group(p, elem, st);
     if (mixed) {
         const size_t base = base_bytes(pl, p.count);
         if (ws_bytes < base) return JB_EWORKSPACE;
@@ -1094,10 +1232,16 @@ static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsign
     }
     // Shapes are known on the host only for a uniform batch, whose matrices
     // share one class: the split applies to descriptor (uneven) batches.
-    bool split = pl.split && p.descs != nullptr;
+    const bool split = pl.split && p.descs != nullptr;
     if (cudaMemsetAsync(ws, 0, 8 * sizeof(int), st) != cudaSuccess) return JB_ECUDA;
     int64_t grid;
     int rc;
+    if (group) {
+        if (pl.d.nt <= kNarrowN) return launch_group_uneven<128, 4>(p, pl.d.mt, pl.d.nt, 0, st);
+        if ((rc = launch_group_uneven<256, 8>(p, pl.d.mt, pl.d.nt, split ? 1 : 0, st)) || !split) return rc;
+        p.counter = (int *)ws + 2;
+        return launch_group_uneven<128, 4>(p, pl.d.mt, kNarrowN, 2, st);
+    }
     // Mixed solve: factor, precondition and refine; the register kernels below then
     // take what these left (usually nothing: they read one word and return).
     // Not with a warm start or another block width, which are choices of the
@@ -1122,65 +1266,27 @@ static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsign
         p.pending = 1;
         p.counter = (int *)ws + 5;
         p.counter2 = (int *)ws + 6;
-        split = false;
     }
-    if (elem == 4) {
-        // block width 4: 8 warps of 256 threads for 64 columns; 8: 4 warps of 128
-        auto k1 = pl.bw == 8 ? (mixed ? rb32_kernel_t<true, 128, 8, kMaxR, kMaxRV>
-                                      : rb32_kernel_t<false, 128, 8, kMaxR, kMaxRV>)
-                             : (mixed ? rb32_kernel_t<true, kT32, kB32, kMaxR, kMaxRV>
-                                      : rb32_kernel_t<false, kT32, kB32, kMaxR, kMaxRV>);
-        const int t1 = pl.bw == 8 ? 128 : kT32;
-        if ((rc = occupancy_grid(k1, t1, pl.smem32, p.count, grid))) return rc;
-        p.maxd = pl.d32;
-        p.region_cap = pl.reg32;
-        p.cls = split ? 1 : 0;
-        p.xchg = 1;
-        p.xchg_off = pl.xoff32;
-        k1<<<(unsigned)grid, t1, pl.smem32, st>>>(p);
-        if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
-        if (split) {
-            // narrow matrices: 4 warps (nt <= 32 is at most 8 blocks of 4 columns)
-            auto k1n = mixed ? rb32_kernel_t<true, kT32 / 2, kB32, kMaxR, kMaxRV>
-                             : rb32_kernel_t<false, kT32 / 2, kB32, kMaxR, kMaxRV>;
-            if ((rc = occupancy_grid(k1n, kT32 / 2, pl.smem32n, p.count, grid))) return rc;
-            p.counter = (int *)ws + 2;
-            p.cls = 2;
-            p.maxd = pl.d32n;
-            p.region_cap = pl.reg32n;
-            p.xchg_off = pl.xoff32n;
-            k1n<<<(unsigned)grid, kT32 / 2, pl.smem32n, st>>>(p);
-            if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
-            p.counter = (int *)ws;
-        }
-        p.xchg = 0;
-        if (!mixed) return JB_OK;
-        auto k2 = rb64_kernel<float, true>;
-        if ((rc = occupancy_grid(k2, kT64, pl.smem64, p.count, grid))) return rc;
-        p.maxd = pl.d64;
-        p.region_cap = pl.reg64;
-        p.cls = split ? 1 : 0;
-        k2<<<(unsigned)grid, kT64, pl.smem64, st>>>(p);
-        if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
-        if (split) {
-            // narrow matrices: 8 warps (nt <= 32 is at most 16 blocks of 2 columns),
-            // work area sized for nt <= kNarrowN
-            auto k2n = rb64_kernel<float, true, kT64 / 2>;
-            if ((rc = occupancy_grid(k2n, kT64 / 2, pl.smem64n, p.count, grid))) return rc;
-            p.maxd = pl.d64n;
-            p.region_cap = pl.reg64n;
-            p.counter2 = (int *)ws + 3;
-            p.cls = 2;
-            k2n<<<(unsigned)grid, kT64 / 2, pl.smem64n, st>>>(p);
-            if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
-        }
-        return JB_OK;
-    }
-    auto k2 = rb64_kernel<double, false>;
+    // block width 4: 8 warps of 256 threads for 64 columns; 8: 4 warps of 128
+    auto k1 = pl.bw == 8 ? (mixed ? rb32_kernel_t<true, 128, 8, kMaxR, kMaxRV>
+                                  : rb32_kernel_t<false, 128, 8, kMaxR, kMaxRV>)
+                         : (mixed ? rb32_kernel_t<true, kT32, kB32, kMaxR, kMaxRV>
+                                  : rb32_kernel_t<false, kT32, kB32, kMaxR, kMaxRV>);
+    const int t1 = pl.bw == 8 ? 128 : kT32;
+    if ((rc = occupancy_grid(k1, t1, pl.smem32, p.count, grid))) return rc;
+    p.maxd = pl.d32;
+    p.region_cap = pl.reg32;
+    p.cls = 0;
+    p.xchg = 1;
+    p.xchg_off = pl.xoff32;
+    k1<<<(unsigned)grid, t1, pl.smem32, st>>>(p);
+    if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
+    p.xchg = 0;
+    if (!mixed) return JB_OK;
+    auto k2 = rb64_kernel;
     if ((rc = occupancy_grid(k2, kT64, pl.smem64, p.count, grid))) return rc;
     p.maxd = pl.d64;
     p.region_cap = pl.reg64;
-    p.cls = 0;
     k2<<<(unsigned)grid, kT64, pl.smem64, st>>>(p);
     return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
 }

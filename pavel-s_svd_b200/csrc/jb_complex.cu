@@ -18,16 +18,19 @@
 // completion of cut columns, full bases and truncation are the host's, as
 // in the reference's svd() (solvers.py:300-304).
 //
-// One CTA per matrix (grid-stride).  W (m x np) and V (np x np), complex,
-// column-major, in shared memory when they fit, else in a per-CTA slot of
-// the workspace.  A round: one warp per pair computes its three products
-// (lanes over rows, warp reduction), a barrier, then each warp takes the
-// round's floor (a max over the pairs' norms in shared memory), rotates its
-// pair of W and V columns and records the largest active ratio.
+// One CTA per matrix.  Up to 128 x 64, W and V in registers, 8 to 16 lanes a
+// pair (cgroup_kernel, the sweeps of jb_group.cuh with blocks of one column:
+// the reference's own pair order).  Larger: W (m x np) and V (np x np),
+// column-major, in shared memory when they fit, else in a per-CTA slot of the
+// workspace (cjacobi_kernel): per round one warp per pair computes its three
+// products (lanes over rows, warp reduction), a barrier, then each warp takes
+// the round's floor (a max over the pairs' norms in shared memory), rotates
+// its pair of W and V columns and records the largest active ratio.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
 #include "jacobi_b200.h"
+#include "jb_group.cuh"
 
 namespace jb {
 namespace cx {
@@ -81,6 +84,48 @@ __host__ __device__ inline size_t smem_bytes(int m, int np, bool in_smem) {
                al16((size_t)np * 4);
     if (in_smem) b += ((size_t)m * np + (size_t)np * np) * sizeof(C<R>);
     return b;
+}
+
+// Singular values in descending order (ties by column), the cut, U = W / sigma
+// and Vh, from the rotated W (m x n, ld ldw) and V (ld ldv).
+template <typename R>
+__device__ void finish(const C<R> *W, int ldw, const C<R> *V, int ldv, int m, int n, int np, R *sig, int *perm, C<R> *u,
+                       R *so, C<R> *vh) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    // sigma, order (descending; ties by column), cut, outputs
+    for (int c = warp; c < n; c += nw) {
+        const C<R> *w = W + (size_t)c * ldw;
+        R ssq = 0;
+        for (int i = lane; i < m; i += 32) ssq += w[i].re * w[i].re + w[i].im * w[i].im;
+        ssq = wsum(ssq);
+        if (lane == 0) sig[c] = sqrt(ssq);
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        const R sj = sig[j];
+        int rk = 0;
+        for (int i = 0; i < n; ++i) rk += (sig[i] > sj) || (sig[i] == sj && i < j);
+        perm[rk] = j;
+    }
+    __syncthreads();
+    const R s1 = sig[perm[0]];
+    const R cut = eps<R>() * (R)(m > np ? m : np) * s1;
+    for (size_t idx = threadIdx.x; idx < (size_t)m * n; idx += blockDim.x) {
+        const int i = (int)(idx / n), k = (int)(idx - (size_t)i * n);
+        const int c = perm[k];
+        const R sc = sig[c];
+        const C<R> w = W[(size_t)c * ldw + i];
+        u[idx] = sc > cut ? C<R>{w.re / sc, w.im / sc} : C<R>{R(0), R(0)};
+    }
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const R sc = sig[perm[k]];
+        so[k] = sc > cut ? sc : R(0);
+    }
+    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
+        const int k = idx / n, j = idx - k * n;            // Vh[k][j] = conj(V[j][perm k])
+        const C<R> v = V[(size_t)perm[k] * ldv + j];
+        vh[idx] = C<R>{v.re, -v.im};
+    }
 }
 
 template <typename R>
@@ -181,47 +226,62 @@ __global__ void __launch_bounds__(kThreads) cjacobi_kernel(const C<R> *A, C<R> *
             __syncthreads();
             if ((R)bo <= tol) { converged = true; break; }
         }
-        // sigma, order (descending; ties by column), cut, outputs
-        for (int c = warp; c < n; c += nw) {
-            const C<R> *w = W + (size_t)c * m;
-            R ssq = 0;
-            for (int i = lane; i < m; i += 32) ssq += w[i].re * w[i].re + w[i].im * w[i].im;
-            ssq = wsum(ssq);
-            if (lane == 0) sig[c] = sqrt(ssq);
-        }
-        __syncthreads();
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            const R sj = sig[j];
-            int rk = 0;
-            for (int i = 0; i < n; ++i) rk += (sig[i] > sj) || (sig[i] == sj && i < j);
-            perm[rk] = j;
-        }
-        __syncthreads();
-        const R s1 = sig[perm[0]];
-        const R cut = eps<R>() * (R)(m > np ? m : np) * s1;
-        C<R> *u = U + z * (int64_t)m * n;
-        for (size_t idx = threadIdx.x; idx < (size_t)m * n; idx += blockDim.x) {
-            const int i = (int)(idx / n), k = (int)(idx - (size_t)i * n);
-            const int c = perm[k];
-            const R sc = sig[c];
-            const C<R> w = W[(size_t)c * m + i];
-            u[idx] = sc > cut ? C<R>{w.re / sc, w.im / sc} : C<R>{R(0), R(0)};
-        }
-        R *so = S + z * (int64_t)n;
-        for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            const R sc = sig[perm[k]];
-            so[k] = sc > cut ? sc : R(0);
-        }
-        C<R> *vh = Vh + z * (int64_t)n * n;
-        for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-            const int k = idx / n, j = idx - k * n;            // Vh[k][j] = conj(V[j][perm k])
-            const C<R> v = V[(size_t)perm[k] * np + j];
-            vh[idx] = C<R>{v.re, -v.im};
-        }
+        finish<R>(W, m, V, np, m, n, np, sig, perm, U + z * (int64_t)m * n, S + z * (int64_t)n,
+                  Vh + z * (int64_t)n * n);
         if (threadIdx.x == 0) {
             if (sweeps_out) sweeps_out[z] = sweep > max_sweeps ? max_sweeps : sweep;
             if (status) status[z] = converged ? JB_ST_OK : JB_ST_NOT_CONVERGED;
         }
+    }
+}
+
+// The same solve with W and V in registers, GL lanes a block pair
+// (jb_group.cuh).  Blocks of one column: every step is a round of the circle
+// method and the whole matrix moves through shared memory, which bounds it
+// (with the packed FP32 products); blocks of two took 9 sweeps instead of the
+// reference's 6 on a rank-4 40 x 25 matrix.  1024 x 48 x 32 complex64: 1.26 ms a
+// call, 3.96 with one warp a pair and W in shared memory.
+template <typename R, int GL, int RW, int RV, int THREADS>
+struct CGroup {
+    using G = GroupCfg<R, 2, GL, 1, RW, RV>;
+    __host__ __device__ static size_t head(int npb) {
+        return 32 * 8 + al16((size_t)npb * 8) + al16((size_t)npb * sizeof(R)) + al16((size_t)npb * 4);
+    }
+    __host__ __device__ static size_t smem(int npb) { return head(npb) + (size_t)npb * G::LD * sizeof(R); }
+};
+template <typename R, int GL, int RW, int RV, int THREADS>
+__global__ void __launch_bounds__(THREADS) cgroup_kernel(const C<R> *A, C<R> *U, R *S, C<R> *Vh, int32_t *sweeps_out,
+                                                         int32_t *status, int64_t batch, int m, int n, R tol,
+                                                         int max_sweeps) {
+    using K = CGroup<R, GL, RW, RV, THREADS>;
+    constexpr int LD = K::G::LD;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int npb = (n + 1) & ~1;
+    double *red = (double *)smem;
+    double *scales = (double *)(smem + 32 * 8);
+    R *sig = (R *)(smem + 32 * 8 + al16((size_t)npb * 8));
+    int *perm = (int *)((unsigned char *)sig + al16((size_t)npb * sizeof(R)));
+    R *area = (R *)(smem + K::head(npb));
+    const int np = n + (n & 1);
+    for (int64_t z = blockIdx.x; z < batch; z += gridDim.x) {
+        const C<R> *a = A + z * (int64_t)m * n;
+        for (int idx = threadIdx.x; idx < npb * LD; idx += THREADS) area[idx] = R(0);
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < m * n; idx += THREADS) {
+            const int i = idx / n, c = idx - i * n;
+            *(C<R> *)(area + c * LD + 2 * i) = a[idx];
+        }
+        for (int c = threadIdx.x; c < n; c += THREADS) area[c * LD + K::G::VOFF + 2 * c] = R(1);
+        __syncthreads();
+        bool conv;
+        const int ns = group_sweeps<R, 2, GL, 1, RW, RV, THREADS>(area, n, tol, max_sweeps, scales, red, conv);
+        finish<R>((const C<R> *)area, LD / 2, (const C<R> *)(area + K::G::VOFF), LD / 2, m, n, np, sig, perm,
+                  U + z * (int64_t)m * n, S + z * (int64_t)n, Vh + z * (int64_t)n * n);
+        if (threadIdx.x == 0) {
+            if (sweeps_out) sweeps_out[z] = ns;
+            if (status) status[z] = conv ? JB_ST_OK : JB_ST_NOT_CONVERGED;
+        }
+        __syncthreads();
     }
 }
 
@@ -242,12 +302,45 @@ static size_t workspace_bytes(int m, int n, int64_t batch) {
     return (size_t)grid * ((size_t)m * np + (size_t)np * np) * sizeof(C<R>);
 }
 
+template <typename R, int GL, int RW, int RV, int THREADS>
+static int launch_cgroup(const void *A, void *U, R *S, void *Vh, int32_t *sweeps, int32_t *status, int64_t batch, int m,
+                         int n, R tol, int max_sweeps, cudaStream_t st) {
+    auto kern = cgroup_kernel<R, GL, RW, RV, THREADS>;
+    const size_t smem = CGroup<R, GL, RW, RV, THREADS>::smem((n + 1) & ~1);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return JB_ECUDA;
+    const int64_t grid = batch < (1 << 20) ? batch : (1 << 20);
+    kern<<<(unsigned)grid, THREADS, smem, st>>>((const C<R> *)A, (C<R> *)U, S, (C<R> *)Vh, sweeps, status, batch, m, n,
+                                                tol, max_sweeps);
+    return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
+}
+
 template <typename R>
 static int entry(const void *A, void *U, R *S, void *Vh, int32_t *sweeps, int32_t *status, int64_t batch, int32_t m,
                  int32_t n, double tol, int32_t max_sweeps, void *workspace, size_t ws_bytes, void *stream) {
     if (!A || !U || !S || !Vh || batch < 0 || n < 1 || m < n || max_sweeps < 1) return JB_EINVAL;
     if ((int64_t)m * (n + 1) > ((int64_t)1 << 30)) return JB_ETOOBIG;
     if (batch == 0) return JB_OK;
+    const R t = tol > 0 ? (R)tol : R(10) * (sizeof(R) == 4 ? (R)1.1920928955078125e-07 : (R)2.220446049250313e-16);
+    // up to 128 x 64: in registers, lanes a pair and rows a lane from the shape
+    // (at most 48 (FP32) or 96 (FP64) registers of W and V)
+    if (m <= 128 && n <= 64) {
+#define JB_CGROUP(GL, RW, RV, TH) \
+        return launch_cgroup<R, GL, RW, RV, TH>(A, U, S, Vh, sweeps, status, batch, m, n, t, max_sweeps, \
+                                                (cudaStream_t)stream)
+        if constexpr (sizeof(R) == 4) {
+            if (n <= 16 && m <= 32) JB_CGROUP(8, 4, 2, 64);
+            if (n <= 32 && m <= 48) JB_CGROUP(8, 6, 4, 128);
+            if (n <= 32) JB_CGROUP(16, 8, 2, 256);
+            JB_CGROUP(16, 8, 4, 512);
+        } else {
+            if (n <= 16 && m <= 32) JB_CGROUP(8, 4, 2, 64);
+            if (n <= 32 && m <= 64) JB_CGROUP(8, 8, 4, 128);
+            if (n <= 32) JB_CGROUP(16, 8, 2, 256);
+            JB_CGROUP(16, 8, 4, 512);
+        }
+#undef JB_CGROUP
+    }
     const int np = n + (n & 1);
     const bool in_smem = smem_bytes<R>(m, np, true) <= kSmemLimit;
     const size_t smem = smem_bytes<R>(m, np, in_smem);
@@ -269,7 +362,6 @@ static int entry(const void *A, void *U, R *S, void *Vh, int32_t *sweeps, int32_
         if (grid > fit) grid = fit;
         gws = (C<R> *)workspace;
     }
-    const R t = tol > 0 ? (R)tol : R(10) * (sizeof(R) == 4 ? (R)1.1920928955078125e-07 : (R)2.220446049250313e-16);
     kern<<<(unsigned)grid, kThreads, smem, (cudaStream_t)stream>>>((const C<R> *)A, (C<R> *)U, S, (C<R> *)Vh, sweeps,
                                                                    status, batch, m, n, t, max_sweeps, in_smem ? 1 : 0,
                                                                    gws);

@@ -262,7 +262,7 @@ __device__ int sweeps(T *W, T *V, const Geo &g, T tol, int max_sweeps, Aux &ax, 
 // signed so that Q ~ input when the input is nearly orthogonal.  Follows
 // householder_vec/qr of primitives.py:41-89 (xLARFG: beta = -sign(alpha)
 // ||x||, backward accumulation).  `tmp` holds np x np doubles.
-__device__ void householder_orthonormalize(double *Q, int np, int ldq, double *tmp, int ldt, Aux &ax) {
+__device__ inline void householder_orthonormalize(double *Q, int np, int ldq, double *tmp, int ldt, Aux &ax) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nwarps();
     double *beta_sign = ax.sig;  // reuse: sign(R_jj)
     for (int j = 0; j < np; ++j) {
