@@ -3,20 +3,27 @@
 // (svdbench/standalone/primitives.py:370-427, the syevj structure), used by
 // its gram_jacobi and polar_* families (solvers.py:109, 170).
 //
-// One CTA per matrix: G (n x n, padded to even n with a zero row and column,
-// FP64) and V accumulated in FP64, in shared memory when they fit (n <= 118
-// both, n <= 166 G alone), else in a per-CTA global area.  Per round of the
-// round-robin tournament (primitives.py:309-313) the reference's plane
-// rotation of every active
-// pair, then G <- J^T G J and V <- V J.  A pair is active when
-// |g_pq| > tol * max|G| (the reference's absolute criterion, with max|G|
-// taken at the start of each sweep rather than each round), and the solve
-// has converged after a sweep whose largest |g_pq| / max|G| is <= tol.
+// A pair is active when |g_pq| > tol * max|G| (the reference's absolute
+// criterion, with max|G| taken at the start of each sweep rather than each
+// round), and the solve has converged after a sweep that finds none.
+//
+// n <= 64 (eigh_group_kernel): H V and V rotated together in registers, 8 or 16
+// lanes a column pair or block pair (jb_group.cuh, EIG).  Bound by the FP64 pipe
+// and the reductions of its dot products: 1024 x 32 x 32 FP64 0.31 ms, against
+// 1.27 ms for G and V in shared memory (two barriers and 3 n^2 shared-memory
+// accesses a round), and half that one's error.
+// Larger n (eigh_kernel, zeigh_kernel), one CTA per matrix: G (n x n, padded to
+// even n with a zero row and column, FP64) and V accumulated in FP64, in shared
+// memory when they fit (n <= 118 both, n <= 166 G alone), else in a per-CTA
+// global area.  Per round of the round-robin tournament (primitives.py:309-313)
+// the reference's plane rotation of every active pair, then G <- J^T G J and
+// V <- V J.
 // Eigenvalues come out ascending with V's columns in the same order.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
 #include "jacobi_b200.h"
+#include "jb_group.cuh"
 
 namespace jb {
 namespace eigh {
@@ -298,9 +305,107 @@ __global__ void __launch_bounds__(kThreads) zeigh_kernel(const R *H, R *W, R *Vo
 
 constexpr size_t kSmemLimit = 227 * 1024;
 
+// The solve with W = H V and V in registers, GL lanes a block pair
+// (jb_group.cuh EIG), one CTA a matrix, for n <= GL * RW; blocks of two columns
+// (real) or one (complex).  T: the input's real type; the arithmetic is FP64.
+template <typename T, int NC, int GL, int RW, int THREADS>
+struct EigGroup {
+    static constexpr int B = NC == 1 ? 2 : 1;
+    using G = GroupCfg<double, NC, GL, B, RW, RW>;
+    __host__ __device__ static int npb(int n) { return 2 * B * ((n + 2 * B - 1) / (2 * B)); }
+    static size_t smem(int n) { return 32 * 8 + (size_t)npb(n) * (8 + 8 + 8 + (size_t)G::LD * 8); }
+};
+template <typename T, int NC, int GL, int RW, int THREADS>
+__global__ void __launch_bounds__(THREADS) eigh_group_kernel(const T *H, T *Wo, T *Vo, int32_t *sweeps_out,
+                                                             int32_t *status, int64_t batch, int n, double tol,
+                                                             int max_sweeps) {
+    using K = EigGroup<T, NC, GL, RW, THREADS>;
+    constexpr int LD = K::G::LD, VO = K::G::VOFF;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int np = K::npb(n);
+    double *red = (double *)smem, *scales = red + 32, *lam = scales + np;
+    int *perm = (int *)(lam + np);
+    double *area = lam + 2 * np;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int64_t z = blockIdx.x; z < batch; z += gridDim.x) {
+        const T *h = H + z * (int64_t)n * n * NC;
+        for (int i = threadIdx.x; i < np * LD; i += THREADS) area[i] = 0.0;
+        __syncthreads();
+        double mx = 0.0;
+        // (H + H^H) / 2, column c at area + c LD; rows of the input are walked
+        for (int i = threadIdx.x; i < n * n; i += THREADS) {
+            const int r = i / n, c = i - r * n;
+            if constexpr (NC == 1) {
+                const double g = 0.5 * ((double)h[i] + (double)h[c * n + r]);
+                area[c * LD + r] = g;
+                mx = fmax(mx, fabs(g));
+            } else {
+                const double re = 0.5 * ((double)h[2 * i] + (double)h[2 * (c * n + r)]);
+                const double im = 0.5 * ((double)h[2 * i + 1] - (double)h[2 * (c * n + r) + 1]);
+                area[c * LD + 2 * r] = re;
+                area[c * LD + 2 * r + 1] = im;
+                mx = fmax(mx, hypot(re, im));
+            }
+        }
+        for (int c = threadIdx.x; c < n; c += THREADS) area[c * LD + VO + NC * c] = 1.0;
+        mx = warp_max(mx);
+        if (lane == 0) red[warp] = mx;
+        __syncthreads();
+        double scale0 = 0.0;
+        for (int w = 0; w < THREADS / 32; ++w) scale0 = fmax(scale0, red[w]);
+        __syncthreads();
+        bool conv;
+        const int ns = group_sweeps<double, NC, GL, K::B, RW, RW, THREADS, true>(area, n, tol, max_sweeps, scales, red,
+                                                                                 conv, scale0);
+        // eigenvalues v^H w, ascending, ties by column
+        for (int c = warp; c < n; c += THREADS / 32) {
+            const double *w = area + c * LD, *v = w + VO;
+            double sum = 0.0;
+            for (int i = lane; i < NC * n; i += 32) sum = fma(v[i], w[i], sum);
+            sum = warp_sum(sum);
+            if (lane == 0) lam[c] = sum;
+        }
+        __syncthreads();
+        for (int j = threadIdx.x; j < n; j += THREADS) {
+            const double dj = lam[j];
+            int rk = 0;
+            for (int i = 0; i < n; ++i) rk += (lam[i] < dj) || (lam[i] == dj && i < j);
+            perm[rk] = j;
+        }
+        __syncthreads();
+        T *wo = Wo + z * (int64_t)n, *vo = Vo + z * (int64_t)n * n * NC;
+        for (int k = threadIdx.x; k < n; k += THREADS) wo[k] = (T)lam[perm[k]];
+        for (int k = threadIdx.x; k < n * n; k += THREADS) {
+            const int i = k / n, j = k - i * n;                   // row-major output, column j = eigenvector j
+            const double *v = area + perm[j] * LD + VO + NC * i;
+            vo[NC * k] = (T)v[0];
+            if constexpr (NC == 2) vo[2 * k + 1] = (T)v[1];
+        }
+        if (threadIdx.x == 0) {
+            if (sweeps_out) sweeps_out[z] = ns;
+            if (status) status[z] = conv ? JB_ST_OK : JB_ST_NOT_CONVERGED;
+        }
+        __syncthreads();
+    }
+}
+template <typename T, int NC, int GL, int RW, int THREADS>
+static int launch_group(const T *H, T *W, T *V, int32_t *sweeps, int32_t *status, int64_t batch, int n, double tol,
+                        int max_sweeps, cudaStream_t st) {
+    auto kern = eigh_group_kernel<T, NC, GL, RW, THREADS>;
+    const size_t smem = EigGroup<T, NC, GL, RW, THREADS>::smem(n);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return JB_ECUDA;
+    const int64_t grid = batch < (1 << 20) ? batch : (1 << 20);
+    kern<<<(unsigned)grid, THREADS, smem, st>>>(H, W, V, sweeps, status, batch, n, tol, max_sweeps);
+    return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
+}
+
 template <typename R>
 static int zlaunch(const R *H, R *W, R *V, int32_t *sweeps, int32_t *status, int64_t batch, int n, double tol,
                    int max_sweeps, void *workspace, size_t ws_bytes, cudaStream_t st) {
+    if (n <= 16) return launch_group<R, 2, 8, 2, 64>(H, W, V, sweeps, status, batch, n, tol, max_sweeps, st);
+    if (n <= 32) return launch_group<R, 2, 8, 4, 128>(H, W, V, sweeps, status, batch, n, tol, max_sweeps, st);
+    if (n <= 64) return launch_group<R, 2, 16, 4, 512>(H, W, V, sweeps, status, batch, n, tol, max_sweeps, st);
     const int np = n + (n & 1);
     const int mode = zsmem_bytes(np, 2) <= kSmemLimit ? 2 : (zsmem_bytes(np, 1) <= kSmemLimit ? 1 : 0);
     const size_t smem = zsmem_bytes(np, mode);
@@ -325,6 +430,9 @@ static int zlaunch(const R *H, R *W, R *V, int32_t *sweeps, int32_t *status, int
 template <typename T>
 static int launch(const T *H, T *W, T *V, int32_t *sweeps, int32_t *status, int64_t batch, int n, double tol,
                   int max_sweeps, void *workspace, size_t ws_bytes, cudaStream_t st) {
+    if (n <= 16) return launch_group<T, 1, 8, 2, 32>(H, W, V, sweeps, status, batch, n, tol, max_sweeps, st);
+    if (n <= 32) return launch_group<T, 1, 8, 4, 64>(H, W, V, sweeps, status, batch, n, tol, max_sweeps, st);
+    if (n <= 64) return launch_group<T, 1, 16, 4, 256>(H, W, V, sweeps, status, batch, n, tol, max_sweeps, st);
     const int np = n + (n & 1);
     const int mode = smem_bytes(np, 2) <= kSmemLimit ? 2 : (smem_bytes(np, 1) <= kSmemLimit ? 1 : 0);
     const size_t smem = smem_bytes(np, mode);

@@ -21,6 +21,13 @@
 // exact sums each time, the active test and the angle are the reference's
 // (primitives.py:334-347); the null-column floor eps^2 max ||w_j||^2 takes the
 // norms at the start of the sweep (the reference's: of the round).
+//
+// EIG: the two-sided Jacobi of a Hermitian H (primitives.py:370-427) in the same
+// form: W = H V and V are rotated together, and the entries of G = V^H H V that a
+// rotation needs are the dot products v_p^H w_p, v_q^H w_q, v_p^H w_q -- no row
+// rotations, and G itself is never formed.  A pair is active when |g_pq| > tol
+// max|G| (the reference's absolute criterion; max|G| is that of H in the first
+// sweep, then the largest |g_pp| at the start of the sweep).
 #pragma once
 #include "jb_device.cuh"
 #include "jb_regblock.cuh"
@@ -79,10 +86,9 @@ __device__ __forceinline__ bool jacobi_tan(float app, float aqq, float a, float 
     t = copysignf(__fdividef(2.f * a, fabsf(d) + h * rsqrtf(h)), d);
     return true;
 }
-__device__ __forceinline__ bool jacobi_tan(double app, double aqq, double a, double tol2, double floor_, double &t) {
-    const double prod = app * aqq;
+__device__ __forceinline__ bool eigen_tan(double app, double aqq, double a, double threshold, double &t) {
     t = 0.0;
-    if (!(a * a > tol2 * prod && fmin(app, aqq) > floor_)) return false;
+    if (!(a > threshold)) return false;
     const double d = aqq - app, a2 = 2.0 * a;
     const int ex = (__double2hiint(fmax(fabs(d), a2)) >> 20) & 0x7ff;
     const double scl = __hiloint2double((2046 - ex) << 20, 0);
@@ -95,6 +101,10 @@ __device__ __forceinline__ bool jacobi_tan(double app, double aqq, double a, dou
     for (int k = 0; k < 2; ++k) t -= fma(aa * t, t, fma(2.0 * dd, t, -aa)) * r;
     if (d < 0.0) t = -t;
     return true;
+}
+__device__ __forceinline__ bool jacobi_tan(double app, double aqq, double a, double tol2, double floor_, double &t) {
+    const bool active = a * a > tol2 * (app * aqq) && fmin(app, aqq) > floor_;
+    return eigen_tan(app, aqq, active ? a : 0.0, 0.0, t);
 }
 // c = 1 / sqrt(1 + t2): FP32 from 1 - c with its own relative precision, FP64
 // the FP32 estimate and two Newton steps.
@@ -131,7 +141,7 @@ __device__ __forceinline__ double rsqrt_of(double x) {
     return r * __hiloint2double((1023 - (ex >> 1)) << 20, 0);
 }
 
-template <typename R, int NC, int GL, int B, int RW, int RV>
+template <typename R, int NC, int GL, int B, int RW, int RV, bool EIG = false>
 struct GroupTile {
     using C = GroupCfg<R, NC, GL, B, RW, RV>;
     static_assert(B <= 2, "blocks of one or two columns");
@@ -183,36 +193,39 @@ struct GroupTile {
 #pragma unroll
         for (int e = 0; e < C::ET; ++e) w[p][e] *= s;
     }
+    // ||w_p||^2, or v_p^H w_p
     __device__ __forceinline__ R norm2(int p) const {
+        constexpr int O = EIG ? C::EW : 0;
         R a = 0, b = 0;
 #pragma unroll
         for (int e = 0; e < C::EW; e += 2) {
             if constexpr (sizeof(R) == 4) {
-                fma2(a, b, w[p][e], w[p][e + 1], w[p][e], w[p][e + 1]);
+                fma2(a, b, w[p][O + e], w[p][O + e + 1], w[p][e], w[p][e + 1]);
             } else {
-                a = dfma(w[p][e], w[p][e], a);
-                b = dfma(w[p][e + 1], w[p][e + 1], b);
+                a = dfma(w[p][O + e], w[p][e], a);
+                b = dfma(w[p][O + e + 1], w[p][e + 1], b);
             }
         }
         return a + b;
     }
-    // re and im of x^H y
+    // re and im of w_p^H w_q, or v_p^H w_q
     __device__ __forceinline__ void dot(int p, int q, R &re, R &im) const {
+        constexpr int O = EIG ? C::EW : 0;
         R a = 0, b = 0, c = 0, d = 0;
 #pragma unroll
         for (int e = 0; e < C::EW; e += 2) {
             if constexpr (sizeof(R) == 4) {
-                fma2(a, b, w[p][e], w[p][e + 1], w[q][e], w[q][e + 1]);
+                fma2(a, b, w[p][O + e], w[p][O + e + 1], w[q][e], w[q][e + 1]);
             } else {
-                a = dfma(w[p][e], w[q][e], a);
-                b = dfma(w[p][e + 1], w[q][e + 1], b);
+                a = dfma(w[p][O + e], w[q][e], a);
+                b = dfma(w[p][O + e + 1], w[q][e + 1], b);
             }
             if constexpr (NC == 2) {
                 if constexpr (sizeof(R) == 4) {
-                    fma2(c, d, w[p][e], w[p][e + 1], w[q][e + 1], w[q][e]);
+                    fma2(c, d, w[p][O + e], w[p][O + e + 1], w[q][e + 1], w[q][e]);
                 } else {
-                    c = dfma(w[p][e], w[q][e + 1], c);
-                    d = dfma(w[p][e + 1], w[q][e], d);
+                    c = dfma(w[p][O + e], w[q][e + 1], c);
+                    d = dfma(w[p][O + e + 1], w[q][e], d);
                 }
             }
         }
@@ -221,7 +234,8 @@ struct GroupTile {
     }
 
     // One step: B disjoint pairs of each group.  INTRA pairs the two columns of
-    // each block (scales 1 before), otherwise x_i with y_i.
+    // each block (scales 1 before), otherwise x_i with y_i.  EIG: floor_ is the
+    // threshold of |g_pq|.
     template <bool INTRA>
     __device__ __forceinline__ void step(R tol2, R floor_, int &fl, int lane) {
         constexpr int LB = Log2<B>::value, LG = Log2<GL>::value;
@@ -251,11 +265,13 @@ struct GroupTile {
         if constexpr (NC == 2) {
             // t e^(i phi), phi the phase of apq
             const R g2 = dfma(re, re, im * im), ig = rsqrt_of(fmax(g2, Lim<R>::tiny()));
-            active = jacobi_tan(app, aqq, g2 * ig, tol2, floor_ * S * S, t);
+            if constexpr (EIG) active = eigen_tan(app, aqq, g2 * ig, floor_, t);
+            else active = jacobi_tan(app, aqq, g2 * ig, tol2, floor_ * S * S, t);
             tr = active ? t * ig * re : R(0);
             ti = active ? t * ig * im : R(0);
         } else {
-            active = jacobi_tan(app, aqq, dabs(re), tol2, floor_, t);
+            if constexpr (EIG) active = eigen_tan(app, aqq, dabs(re), floor_, t);
+            else active = jacobi_tan(app, aqq, dabs(re), tol2, floor_, t);
             tr = re < R(0) ? -t : t;
         }
         if (active) fl = 1;
@@ -330,14 +346,16 @@ __device__ __forceinline__ void team_sync() {
 // to the block grid zero) until one finds no active pair; the rotated columns
 // are left there, at scale 1.  scales: npb doubles of shared memory; red: 32
 // doubles.  All threads of the CTA call it.  Returns the sweeps taken.
-template <typename R, int NC, int GL, int B, int RW, int RV, int THREADS>
-__device__ int group_sweeps(R *area, int n, R tol, int max_sweeps, double *scales, double *red, bool &converged) {
+// EIG: max|H| is given as scale0.
+template <typename R, int NC, int GL, int B, int RW, int RV, int THREADS, bool EIG = false>
+__device__ int group_sweeps(R *area, int n, R tol, int max_sweeps, double *scales, double *red, bool &converged,
+                            R scale0 = R(0)) {
     constexpr int LB = Log2<B>::value, LG = Log2<GL>::value;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (GL - 1);
     const int group = threadIdx.x / GL, li = gl >> (LG - LB), base = lane & ~(GL - 1);
     const int nb = 2 * ((n + 2 * B - 1) / (2 * B));
     const bool act = group < nb / 2, wact = warp * (32 / GL) < nb / 2;
-    GroupTile<R, NC, GL, B, RW, RV> t;
+    GroupTile<R, NC, GL, B, RW, RV, EIG> t;
     int X = act ? group : 0, Y = act ? nb - 1 - group : 0;
     if (act) {
         t.template exchange<false>(area, X, Y, gl);
@@ -359,7 +377,7 @@ __device__ int group_sweeps(R *area, int n, R tol, int max_sweeps, double *scale
             for (int c = 0; c < 2 * B; ++c) {
                 R s[1] = {t.norm2(c)};
                 lanes_reduce_scatter<GL>(s, lane);
-                mx = fmax(mx, s[0]);
+                mx = fmax(mx, EIG ? dabs(s[0]) : s[0]);
             }
         }
         mx = warp_max(mx);
@@ -371,7 +389,7 @@ __device__ int group_sweeps(R *area, int n, R tol, int max_sweeps, double *scale
             for (int w = 0; w < THREADS / 32; ++w) gm = fmax(gm, red[w]);
             mx = (R)gm;
         }
-        const R floor_ = Lim<R>::eps() * Lim<R>::eps() * mx;
+        const R floor_ = EIG ? tol * (sweep == 1 ? scale0 : mx) : Lim<R>::eps() * Lim<R>::eps() * mx;
         int fl = 0;
         if (wact) {
             if constexpr (B == 2) t.template step<true>(tol2, floor_, fl, lane);

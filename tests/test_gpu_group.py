@@ -99,3 +99,28 @@ def test_uneven_equals_equal_shapes(pkg):
         u, s, vh = pkg.svd(torch.from_numpy(a).to(DEV), precision="fp32")
         for x, y in zip(plan.result(i), (u, s, vh)):
             assert torch.equal(x, y), i
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64, np.complex64, np.complex128])
+@pytest.mark.parametrize("n", [1, 2, 3, 15, 16, 17, 31, 32, 33, 63, 64, 65])
+def test_eigen_sizes(n, dt):
+    """The two-sided solve on the same sweeps, both sides of its sizes (16, 32,
+    64; 65 is the shared-memory kernel): indefinite, zero-diagonal (max|H| off
+    the diagonal) and zero matrices in one batch.  Eigenvalues to 10 n eps
+    max|w|, V and the residual to 100 n eps (n rotations a sweep, 10 sweeps)."""
+    E = importlib.import_module("pavel-s_svd_b200.eigh")
+    x = matrices((3, n, n), dt, n)
+    h = x + np.conj(np.swapaxes(x, 1, 2))
+    h[1] = 0
+    h[1][np.arange(n - 1), np.arange(1, n)] = 1
+    h[1][np.arange(1, n), np.arange(n - 1)] = 1
+    h[2] = 0
+    w, v, sweeps = E.jacobi_eigh(torch.from_numpy(h).to(DEV))
+    w, v = w.cpu().numpy().astype(np.float64), v.resolve_conj().cpu().numpy().astype(np.complex128)
+    eps = float(np.finfo(dt).eps)
+    truth = np.linalg.eigvalsh(h.astype(np.complex128))
+    scale = np.maximum(np.abs(truth).max(-1), 1e-300)
+    assert sweeps >= 1 and float((np.abs(w - truth).max(-1) / scale).max()) <= 10 * n * eps
+    assert float(np.abs(np.conj(np.swapaxes(v, 1, 2)) @ v - np.eye(n)).max()) <= 100 * n * eps
+    res = np.abs(h.astype(np.complex128) @ v - v * w[:, None, :]).max((-2, -1)) / scale
+    assert float(res.max()) <= 100 * n * eps
