@@ -828,6 +828,7 @@ __global__ void __launch_bounds__(kTG, 1) gram64_kernel(Params p) {
     unsigned char *pq = (unsigned char *)(cs + npmax);
     unsigned char *sched = pq + npmax;
     unsigned char *area = p.gws + (size_t)blockIdx.x * p.gws_stride;
+    if (p.pending && *p.n_pending == 0) return;
     for (;;) {
         int64_t idx;
         next_ticket(p.counter, s_idx, idx);
@@ -842,7 +843,7 @@ __global__ void __launch_bounds__(kTG, 1) gram64_kernel(Params p) {
         __syncthreads();
         if (threadIdx.x == 0) ax.flag[2] = 0;
         __syncthreads();
-        if (prev != JB_ST_OK) continue;  // K1 already reported this matrix
+        if (prev != (p.pending ? kHanded : JB_ST_OK)) continue;  // already reported
         int ns = s1, st = JB_ST_OK;
         if (!desc_fits(d, p.maxd) || d.x_off < 0) {
             st = JB_ST_BAD_DESC;
@@ -1252,13 +1253,13 @@ static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsign
         p.n_pending = (int *)ws + 4;
         p.maxd = pl.d32;
         p.region_cap = pl.reg32;
-        const size_t s0 = fac_smem(pl.d.mt, pl.d.nt), s1 = pre_smem(pl.d.nt), s2 = ref_smem(pl.d.mt, pl.d.nt);
+        const size_t s0 = fac_smem<64>(pl.d.mt, pl.d.nt), s1 = pre_smem(pl.d.nt), s2 = ref_smem(pl.d.mt, pl.d.nt);
         // one CTA a matrix, largest first: no state is kept from one to the next
-        if ((rc = occupancy_grid(factor_kernel, kFacT, s0, p.count, grid))) return rc;
-        factor_kernel<<<(unsigned)(p.count < kMaxGrid ? p.count : kMaxGrid), kFacT, s0, st>>>(p);
+        if ((rc = occupancy_grid(factor_kernel<kFacT>, kFacT, s0, p.count, grid))) return rc;
+        factor_kernel<kFacT><<<(unsigned)(p.count < kMaxGrid ? p.count : kMaxGrid), kFacT, s0, st>>>(p);
         if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
-        if ((rc = occupancy_grid(precondition_kernel, kPreT, s1, p.count, grid))) return rc;
-        precondition_kernel<<<(unsigned)grid, kPreT, s1, st>>>(p);
+        if ((rc = occupancy_grid(precondition_kernel<kPreT>, kPreT, s1, p.count, grid))) return rc;
+        precondition_kernel<kPreT><<<(unsigned)grid, kPreT, s1, st>>>(p);
         if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
         if ((rc = occupancy_grid(refine_kernel, kRefT, s2, p.count, grid))) return rc;
         refine_kernel<<<(unsigned)grid, kRefT, s2, st>>>(p);
@@ -1291,6 +1292,53 @@ static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsign
     return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
 }
 
+// The mixed solve above 128 x 64 (jb_mixed.cuh); the parts of H take the per-CTA
+// areas of the Gram kernel, which runs after.
+static int launch_mixed_large(Params p, const Plan &pl, unsigned char *ws, size_t ws_bytes, cudaStream_t st) {
+    const int mt = pl.d.mt, nt = pl.d.nt;
+    int64_t grid;
+    int rc;
+    p.counter = (int *)ws;
+    p.n_pending = (int *)ws + 4;
+    p.maxd = pl.d32;
+    p.region_cap = pl.reg32;
+    const size_t s0 = fac_smem<128>(mt, nt), s1 = pre_smem(nt);
+    if ((rc = occupancy_grid(factor_kernel<256>, 256, s0, p.count, grid))) return rc;
+    factor_kernel<256><<<(unsigned)(p.count < kMaxGrid ? p.count : kMaxGrid), 256, s0, st>>>(p);
+    if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
+    if ((rc = occupancy_grid(precondition_kernel<256>, 256, s1, p.count, grid))) return rc;
+    precondition_kernel<256><<<(unsigned)grid, 256, s1, st>>>(p);
+    if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
+    const int cs = mt > 4 * kLgRows ? 8 : 4;
+    const size_t s2 = lg_smem(nt, cs);
+    auto kern = cs == 8 ? refine_large_kernel<8> : refine_large_kernel<4>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2) != cudaSuccess) return JB_ECUDA;
+    // one cluster a slot of the workspace, at most about one CTA an SM
+    const int sms = sm_count();
+    if (sms <= 0) return JB_ECUDA;
+    const size_t stride = pl.gram_stride;
+    int64_t slots = sms / cs;
+    if (slots > p.count) slots = p.count;
+    const int64_t fit = (int64_t)((ws_bytes - kCounterBytes) / stride);
+    if (slots > fit) slots = fit;
+    if (slots < 1) return JB_EWORKSPACE;
+    p.gws = ws + kCounterBytes;
+    p.gws_stride = stride;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(slots * cs));
+    cfg.blockDim = dim3(kRefT);
+    cfg.dynamicSmemBytes = s2;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, p) != cudaSuccess) return JB_ECUDA;
+    return JB_OK;
+}
+
 // Large tiles (FP32 input): the 512-thread register kernel for the FP32
 // sweeps; with mixed precision the round-robin kernel then runs the FP64
 // phase from the FP32 V it left in x32.
@@ -1304,7 +1352,16 @@ static int launch_big(Params &p, const Plan &pl, int precision, unsigned char *w
         p.x32 = (float *)(ws + base);
         p.x_cap = (int64_t)((ws_bytes - base) / 4);
     }
-    if (cudaMemsetAsync(ws, 0, sizeof(int), st) != cudaSuccess) return JB_ECUDA;
+    if (cudaMemsetAsync(ws, 0, 8 * sizeof(int), st) != cudaSuccess) return JB_ECUDA;
+    // factor, precondition and refine (a cluster a matrix); the kernels below then
+    // take what these left
+    if (mixed && pl.gram_stride >= lg_part_bytes(pl.d.mt, pl.d.nt) && pl.gram_stride && (p.descs || !(p.uflags & JB_FULL_MATRICES) || p.um == p.un)) {
+        const int rc = launch_mixed_large(p, pl, ws, ws_bytes, st);
+        if (rc) return rc;
+        p.n_pending = (int *)ws + 4;
+        p.pending = 1;
+        p.counter = (int *)ws + 5;
+    }
     auto k1 = mixed ? rb32_kernel_t<true, kT32L, kB32L, kMaxRL, kMaxRVL>
                     : rb32_kernel_t<false, kT32L, kB32L, kMaxRL, kMaxRVL>;
     int64_t grid;
@@ -1337,7 +1394,7 @@ static int launch_gram(Params &p, const Plan &pl, unsigned char *ws, size_t ws_b
     p.maxd = pl.d;
     p.gws = ws + kCounterBytes;
     p.gws_stride = pl.gram_stride;
-    if (cudaMemsetAsync(p.counter, 0, sizeof(int), st) != cudaSuccess) return JB_ECUDA;
+    p.counter = (int *)ws + 6;
     gram64_kernel<<<(unsigned)g2, kTG, pl.gram_smem, st>>>(p);
     return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
 }

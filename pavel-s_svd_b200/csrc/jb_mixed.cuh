@@ -1,4 +1,4 @@
-// jb_mixed.cuh - the mixed-precision solve of float32 matrices up to 128 x 64
+// jb_mixed.cuh - the mixed-precision solve of float32 matrices up to 256 x 128
 // (tall view): a preconditioned FP32 Jacobi, then an FP64 refinement made of
 // matrix products.
 //
@@ -13,7 +13,8 @@
 //     a sweep moves n instead of m + n rows a column and fewer sweeps are
 //     needed (128 x 64 with singular values over three decades: 7 instead of
 //     13).
-//   refine_kernel (256 threads a matrix)
+//   refine_kernel (256 threads a matrix; refine_large_kernel above 128 x 64, a
+//   cluster of CTAs)
 //     repeat: E = V^T V - I, W = A V from the exact input, H = W^T W (FP64);
 //     done when every pair ratio |h_pq| / sqrt(h_pp h_qq) is <= tol -- the
 //     reference's convergence test on the current W (primitives.py:334-339,
@@ -114,7 +115,7 @@ __device__ __forceinline__ void stage_tall(const float *A, const jb_matrix_desc 
 }
 
 // ---------------------------------------------------------------------------
-// FP32 Jacobi with 8 lanes a block pair: lane gl of a group owns R rows of
+// FP32 Jacobi with GL = 8 lanes a block pair (16 above 64 columns): lane gl of a group owns R rows of
 // the 2B columns of its two blocks.  Compared with a whole warp a pair
 // (jb_regblock.cuh) a step's fixed cost -- the reductions, the rotation
 // parameters, the broadcasts -- is shared by four pairs of blocks a warp:
@@ -124,35 +125,14 @@ __device__ __forceinline__ void stage_tall(const float *A, const jb_matrix_desc 
 // scaled rotations, unrolled intra steps and the factor in the same kernel (12
 // warps an SM) took 1.62 ms for factor and sweeps on the uneven batch, 1.22 now.
 // ---------------------------------------------------------------------------
-constexpr int kGL = 8;
-
-template <int NV>
-__device__ __forceinline__ void group_reduce_scatter(float (&x)[NV], int lane) {
-    constexpr int L = Log2<NV>::value;
-#pragma unroll
-    for (int s = 0; s < L; ++s) {
-        const int h = NV >> (s + 1);
-        const int o = (kGL / 2) >> s;
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int k = 0; k < h; ++k) {
-            const float send = up ? x[k] : x[k + h];
-            const float keep = up ? x[k + h] : x[k];
-            x[k] = keep + __shfl_xor_sync(FULL, send, o);
-        }
-    }
-#pragma unroll
-    for (int o = (kGL / 2) >> L; o >= 1; o >>= 1) x[0] += __shfl_xor_sync(FULL, x[0], o);
-}
-
 // The columns are kept scaled, w = scale * (the tile's column): a rotation is
 // then x - a y, y + b x with both columns' scales multiplied by c (Gentleman's
 // square-root-free rotation), half the arithmetic of the plain form.  Scales
 // start at 1 each sweep and shrink by at most sqrt(2) a rotation.
-template <int B, int R>
+template <int GL, int B, int R>
 struct GTile {
     float w[2 * B][R];
-    // of the lane's pair (x_i, y_i), i = the lane's position in the group / (8 / B):
+    // of the lane's pair (x_i, y_i), i = the lane's position in the group / (GL / B):
     float nx, ny;   // squared norms
     float dx, dy;   // scales
 };
@@ -206,13 +186,13 @@ __device__ __forceinline__ void grot(float (&x)[R], float (&y)[R], float a, floa
 // B pairs of the group's columns: INTRA pairs columns inside each block, with
 // scales 1 and exact norms, and applies c; otherwise x_i with y_i, norms and
 // scales kept by the lanes of pair i.
-template <bool INTRA, int B, int R>
-__device__ __forceinline__ void gstep(GTile<B, R> &t, float tol2, float ex2, int &fl, int lane) {
-    constexpr int LB = Log2<B>::value;
+template <bool INTRA, int GL, int B, int R>
+__device__ __forceinline__ void gstep(GTile<GL, B, R> &t, float tol2, float ex2, int &fl, int lane) {
+    constexpr int LB = Log2<B>::value, LG = Log2<GL>::value;
     float pc[B];
 #pragma unroll
     for (int i = 0; i < B; ++i) pc[i] = gdot(t.w[pair_p<INTRA, B>(i)], t.w[pair_q<INTRA, B>(i)]);
-    group_reduce_scatter(pc, lane);
+    lanes_reduce_scatter<GL>(pc, lane);
     float tn, c;
     if constexpr (INTRA) {
         float pa[B], pb[B];
@@ -222,12 +202,12 @@ __device__ __forceinline__ void gstep(GTile<B, R> &t, float tol2, float ex2, int
             pa[i] = gdot(t.w[p], t.w[p]);
             pb[i] = gdot(t.w[q], t.w[q]);
         }
-        group_reduce_scatter(pa, lane);
-        group_reduce_scatter(pb, lane);
+        lanes_reduce_scatter<GL>(pa, lane);
+        lanes_reduce_scatter<GL>(pb, lane);
         fl |= gparams(pa[0], pb[0], pc[0], tol2, ex2, tn, c);
 #pragma unroll
         for (int i = 0; i < B; ++i) {
-            const int src = (lane & ~(kGL - 1)) | (i << (3 - LB));
+            const int src = (lane & ~(GL - 1)) | (i << (LG - LB));
             const float ti = __shfl_sync(FULL, tn, src), ci = __shfl_sync(FULL, c, src);
             const int p = pair_p<INTRA, B>(i), q = pair_q<INTRA, B>(i);
             grot(t.w[p], t.w[q], ti, ti);
@@ -247,14 +227,14 @@ __device__ __forceinline__ void gstep(GTile<B, R> &t, float tol2, float ex2, int
         t.dy *= c;
 #pragma unroll
         for (int i = 0; i < B; ++i) {
-            const int src = (lane & ~(kGL - 1)) | (i << (3 - LB));
+            const int src = (lane & ~(GL - 1)) | (i << (LG - LB));
             grot(t.w[i], t.w[B + i], __shfl_sync(FULL, a, src), __shfl_sync(FULL, b, src));
         }
     }
 }
 
-template <int B, int R>
-__device__ __forceinline__ void gcircle(GTile<B, R> &t) {
+template <int GL, int B, int R>
+__device__ __forceinline__ void gcircle(GTile<GL, B, R> &t) {
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int o = half * B;
@@ -267,9 +247,9 @@ __device__ __forceinline__ void gcircle(GTile<B, R> &t) {
         }
     }
 }
-template <int B, int R>
-__device__ __forceinline__ void gshift_y(GTile<B, R> &t, int lane) {
-    const int from = (lane & ~(kGL - 1)) | ((lane + kGL / B) & (kGL - 1));
+template <int GL, int B, int R>
+__device__ __forceinline__ void gshift_y(GTile<GL, B, R> &t, int lane) {
+    const int from = (lane & ~(GL - 1)) | ((lane + GL / B) & (GL - 1));
     t.ny = __shfl_sync(FULL, t.ny, from);
     t.dy = __shfl_sync(FULL, t.dy, from);
 #pragma unroll
@@ -284,18 +264,18 @@ __device__ __forceinline__ void gshift_y(GTile<B, R> &t, int lane) {
 // Row of register r of lane gl: chunks of 4 (then 2) consecutive rows, chunk
 // by chunk over the lanes, so that a group's vector access to a column in the
 // exchange area is one run of 128 (64) bytes.
-template <int R>
+template <int GL, int R>
 __device__ __forceinline__ int grow(int r, int gl) {
-    return r < (R & ~3) ? (r >> 2) * 4 * kGL + gl * 4 + (r & 3) : (R & ~3) * kGL + gl * (R & 3) + (r - (R & ~3));
+    return r < (R & ~3) ? (r >> 2) * 4 * GL + gl * 4 + (r & 3) : (R & ~3) * GL + gl * (R & 3) + (r - (R & ~3));
 }
-template <int B, int R, bool STORE>
-__device__ __forceinline__ void gtile_x(GTile<B, R> &t, float *xw, int X, int Y, int gl) {
+template <int GL, int B, int R, bool STORE>
+__device__ __forceinline__ void gtile_x(GTile<GL, B, R> &t, float *xw, int X, int Y, int gl) {
 #pragma unroll
     for (int c = 0; c < 2 * B; ++c) {
-        float *col = xw + (c < B ? X * B + c : Y * B + (c - B)) * (kGL * R);
+        float *col = xw + (c < B ? X * B + c : Y * B + (c - B)) * (GL * R);
 #pragma unroll
         for (int k = 0; k < R / 4; ++k) {
-            float4 *p = (float4 *)(col + k * 4 * kGL) + gl;
+            float4 *p = (float4 *)(col + k * 4 * GL) + gl;
             if (STORE) *p = make_float4(t.w[c][4 * k], t.w[c][4 * k + 1], t.w[c][4 * k + 2], t.w[c][4 * k + 3]);
             else {
                 const float4 v = *p;
@@ -303,7 +283,7 @@ __device__ __forceinline__ void gtile_x(GTile<B, R> &t, float *xw, int X, int Y,
             }
         }
         if (R & 2) {
-            float2 *p = (float2 *)(col + (R & ~3) * kGL) + gl;
+            float2 *p = (float2 *)(col + (R & ~3) * GL) + gl;
             if (STORE) *p = make_float2(t.w[c][R - 2], t.w[c][R - 1]);
             else {
                 const float2 v = *p;
@@ -316,23 +296,23 @@ __device__ __forceinline__ void gtile_x(GTile<B, R> &t, float *xw, int X, int Y,
 // Sweeps over L (x, n x n, column-major) until no pair ratio of a sweep
 // exceeds exit_ratio; then the normalised columns take L's place.  xb: the
 // exchange area.  Returns the sweeps, or max_sweeps + 1.
-template <int B, int R>
+template <int GL, int B, int R>
 __device__ int precondition_sweeps(float *xb, int n, float exit_ratio, int max_sweeps, float *x) {
-    constexpr int LB = Log2<B>::value;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (kGL - 1);
-    const int group = threadIdx.x / kGL;
+    constexpr int LB = Log2<B>::value, LG = Log2<GL>::value;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = lane & (GL - 1);
+    const int group = threadIdx.x / GL;
     const int nb = 2 * ((n + 2 * B - 1) / (2 * B));
-    const bool act = group < nb / 2, wact = warp * (32 / kGL) < nb / 2;
-    const int li = gl >> (3 - LB), base = lane & ~(kGL - 1);
-    float2 *xn = (float2 *)(xb + nb * B * kGL * R);
-    GTile<B, R> t;
+    const bool act = group < nb / 2, wact = warp * (32 / GL) < nb / 2;
+    const int li = gl >> (LG - LB), base = lane & ~(GL - 1);
+    float2 *xn = (float2 *)(xb + nb * B * GL * R);
+    GTile<GL, B, R> t;
     int X = act ? group : 0, Y = act ? nb - 1 - group : 0;
 #pragma unroll
     for (int c = 0; c < 2 * B; ++c) {
         const int col = c < B ? X * B + c : Y * B + (c - B);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int row = grow<R>(r, gl);
+            const int row = grow<GL, R>(r, gl);
             t.w[c][r] = act && col < n && row < n ? x[col * n + row] : 0.f;
         }
     }
@@ -345,8 +325,8 @@ __device__ int precondition_sweeps(float *xb, int n, float exit_ratio, int max_s
             if (sweep > 1) {   // back to scales 1
 #pragma unroll
                 for (int i = 0; i < B; ++i) {
-                    const float sx = __shfl_sync(FULL, t.dx, base | (i << (3 - LB)));
-                    const float sy = __shfl_sync(FULL, t.dy, base | (i << (3 - LB)));
+                    const float sx = __shfl_sync(FULL, t.dx, base | (i << (LG - LB)));
+                    const float sy = __shfl_sync(FULL, t.dy, base | (i << (LG - LB)));
 #pragma unroll
                     for (int r = 0; r < R; ++r) { t.w[i][r] *= sx; t.w[B + i][r] *= sy; }
                 }
@@ -358,20 +338,20 @@ __device__ int precondition_sweeps(float *xb, int n, float exit_ratio, int max_s
                     gcircle(t);
                 }
             }
-            float nrm[2 * B];   // exact norms: column j's on lanes j * 8 / 2B ...
+            float nrm[2 * B];   // exact norms: column j's on lanes j * GL / 2B ...
 #pragma unroll
             for (int c = 0; c < 2 * B; ++c) nrm[c] = gdot(t.w[c], t.w[c]);
-            group_reduce_scatter(nrm, lane);
-            t.nx = __shfl_sync(FULL, nrm[0], base | (li << (2 - LB)));
-            t.ny = __shfl_sync(FULL, nrm[0], base | ((B + li) << (2 - LB)));
+            lanes_reduce_scatter<GL>(nrm, lane);
+            t.nx = __shfl_sync(FULL, nrm[0], base | (li << (LG - 1 - LB)));
+            t.ny = __shfl_sync(FULL, nrm[0], base | ((B + li) << (LG - 1 - LB)));
             t.dx = t.dy = 1.f;
         }
 #pragma unroll 1
         for (int br = 0; br < nb - 1; ++br) {
             if (br > 0 || sweep > 1) {
                 if (act) {
-                    gtile_x<B, R, true>(t, xb, X, Y, gl);
-                    if ((gl & (kGL / B - 1)) == 0) {
+                    gtile_x<GL, B, R, true>(t, xb, X, Y, gl);
+                    if ((gl & (GL / B - 1)) == 0) {
                         xn[X * B + li] = make_float2(t.nx, t.dx);
                         xn[Y * B + li] = make_float2(t.ny, t.dy);
                     }
@@ -380,7 +360,7 @@ __device__ int precondition_sweeps(float *xb, int n, float exit_ratio, int max_s
                 if (act) {
                     if (X > 0) X = X == 1 ? nb - 1 : X - 1;
                     Y = Y == 1 ? nb - 1 : Y - 1;
-                    gtile_x<B, R, false>(t, xb, X, Y, gl);
+                    gtile_x<GL, B, R, false>(t, xb, X, Y, gl);
                     const float2 u = xn[X * B + li], v = xn[Y * B + li];
                     t.nx = u.x; t.dx = u.y;
                     t.ny = v.x; t.dy = v.y;
@@ -401,15 +381,15 @@ __device__ int precondition_sweeps(float *xb, int n, float exit_ratio, int max_s
         float nrm[2 * B];
 #pragma unroll
         for (int c = 0; c < 2 * B; ++c) nrm[c] = gdot(t.w[c], t.w[c]);
-        group_reduce_scatter(nrm, lane);
+        lanes_reduce_scatter<GL>(nrm, lane);
 #pragma unroll
         for (int c = 0; c < 2 * B; ++c) {
-            const float inv = 1.f / sqrtf(__shfl_sync(FULL, nrm[0], base | (c << (2 - LB))));
+            const float inv = 1.f / sqrtf(__shfl_sync(FULL, nrm[0], base | (c << (LG - 1 - LB))));
             const int col = c < B ? X * B + c : Y * B + (c - B);
             if (act && col < n) {
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
-                    const int row = grow<R>(r, gl);
+                    const int row = grow<GL, R>(r, gl);
                     if (row < n) x[col * n + row] = t.w[c][r] * inv;
                 }
             }
@@ -420,10 +400,14 @@ __device__ int precondition_sweeps(float *xb, int n, float exit_ratio, int max_s
 
 __host__ __device__ inline size_t pre_smem(int nt) {
     const size_t cols = nt > 32 ? (nt + 7) / 8 * 8 : nt > 16 ? (nt + 3) / 4 * 4 : (nt + 1) / 2 * 2;
-    return cols * kGL * (nt > 48 ? 8 : nt > 32 ? 6 : nt > 16 ? 4 : 2) * 4 + cols * 8;
+    const size_t rows = nt > 96 ? 128 : nt > 64 ? 96 : nt > 48 ? 64 : nt > 32 ? 48 : nt > 16 ? 32 : 16;
+    return cols * rows * 4 + cols * 8;
 }
 
-__global__ void __launch_bounds__(kPreT, 8) precondition_kernel(Params p) {
+// THREADS 64 up to 64 columns, 256 up to 128 (which also takes the narrower
+// matrices of such a batch).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == kPreT ? 8 : 2) precondition_kernel(Params p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_idx;
     float *xb = (float *)smem;
@@ -438,11 +422,16 @@ __global__ void __launch_bounds__(kPreT, 8) precondition_kernel(Params p) {
         if (p.status[mat] != JB_ST_OK) continue;
         const int nt = d.m > d.n ? d.n : d.m, most = p.max_sweeps32;
         float *x = p.x32 + d.x_off;
-        int ns;
-        if (nt > 48) ns = precondition_sweeps<4, 8>(xb, nt, exit_ratio, most, x);
-        else if (nt > 32) ns = precondition_sweeps<4, 6>(xb, nt, exit_ratio, most, x);
-        else if (nt > 16) ns = precondition_sweeps<2, 4>(xb, nt, exit_ratio, most, x);
-        else ns = precondition_sweeps<1, 2>(xb, nt, exit_ratio, most, x);
+        int ns = 0;
+        if (THREADS > kPreT && nt > 64) {
+            if constexpr (THREADS > kPreT) {
+                if (nt > 96) ns = precondition_sweeps<16, 4, 8>(xb, nt, exit_ratio, most, x);
+                else ns = precondition_sweeps<16, 4, 6>(xb, nt, exit_ratio, most, x);
+            }
+        } else if (nt > 48) ns = precondition_sweeps<8, 4, 8>(xb, nt, exit_ratio, most, x);
+        else if (nt > 32) ns = precondition_sweeps<8, 4, 6>(xb, nt, exit_ratio, most, x);
+        else if (nt > 16) ns = precondition_sweeps<8, 2, 4>(xb, nt, exit_ratio, most, x);
+        else ns = precondition_sweeps<8, 1, 2>(xb, nt, exit_ratio, most, x);
         if (threadIdx.x == 0) {
             p.sweeps[mat] = ns;
             if (ns > most) {
@@ -458,7 +447,7 @@ __global__ void __launch_bounds__(kPreT, 8) precondition_kernel(Params p) {
 // The factor L.
 // ---------------------------------------------------------------------------
 // Pivoted Cholesky of G (n x n, both triangles, ld), thread i = row i, by one
-// warp (n <= 32) or two: step k takes the largest remaining diagonal p and
+// warp (n <= 32), two or four: step k takes the largest remaining diagonal p and
 // leaves column k of L in row p of G (rows chosen before: zero), p * ld in
 // prow[k].  The pivot is found on FP32 keys that carry the row (redux); one
 // barrier a step.  scl brings the largest diagonal to about 1, rscl is its
@@ -467,26 +456,28 @@ template <int WARPS>
 __device__ __forceinline__ bool pivoted_cholesky(double *G, int ld, int n, double cut, double scl, double rscl,
                                                  int *prow, double2 *sd, unsigned *skey) {
     const int i = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr unsigned M = WARPS == 4 ? 127u : 63u;   // the key's bits for the row
     double d = i < n ? G[i * ld + i] : 0.0;
     bool taken = i >= n;
     double *gi = G + min(i, ld - 1);
     for (int k = 0; k < n; ++k) {
         const float df = (float)(d * scl);
-        const unsigned key = taken ? 0u : ((__float_as_uint(fmaxf(df, 0.f)) & ~63u) | (63 - i)) + 64u;
+        const unsigned key = taken ? 0u : ((__float_as_uint(fmaxf(df, 0.f)) & ~M) | (M - i)) + (M + 1u);
         unsigned kw = __reduce_max_sync(FULL, key);
         // 1 / sqrt(d): FP32 estimate, one Newton step (1e-14)
         const double r0 = (double)rsqrt_ftz(df);
         const double rs = r0 * fma(-0.5 * (d * scl), r0 * r0, 1.5) * rscl;
         if (!taken) sd[i] = make_double2(d, rs);
-        if (WARPS == 2) {
-            if (lane == 0) skey[2 * (k & 1) + warp] = kw;
-            asm volatile("bar.sync 1, 64;" ::: "memory");
-            const uint2 ks = *(const uint2 *)(skey + 2 * (k & 1));
-            kw = max(ks.x, ks.y);
+        if (WARPS > 1) {
+            if (lane == 0) skey[WARPS * (k & 1) + warp] = kw;
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * WARPS) : "memory");
+            const unsigned *ks = skey + WARPS * (k & 1);
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) kw = max(kw, ks[w]);
         } else {
             __syncwarp();
         }
-        const int p = 63 - (int)(kw & 63u);
+        const int p = (int)(M - (kw & M));
         const double2 dr = sd[p];
         if (!(dr.x * scl > cut)) return false;
         const double *gq = G + p;
@@ -511,18 +502,19 @@ __device__ __forceinline__ bool pivoted_cholesky(double *G, int ld, int n, doubl
     return true;
 }
 
-// Shared memory: prow (64 ints), sd (64 double2), skey (8), two words, then G
-// (n8 x n8 doubles) and the staged input in one place.
-constexpr size_t kFacHead = 64 * 4 + 64 * 16 + 8 * 4 + 4 * 4;
+// Shared memory: prow (N ints), sd (N double2), skey (8), sex (8), then G (n8 x
+// n8 doubles) and the staged input in one place; N = 64 or 128 columns.
+template <int N> struct FacHead { static constexpr size_t bytes = N * 4 + N * 16 + 8 * 4 + 8 * 4; };
+template <int N>
 __host__ __device__ inline size_t fac_smem(int mt, int nt) {
     const int m8 = round8(mt), n8 = round8(nt);
     const size_t g = (size_t)n8 * n8 * 8, a = stage_floats(m8, n8) * 4;
-    return kFacHead + (g > a ? g : a);
+    return FacHead<N>::bytes + (g > a ? g : a);
 }
 
-// Lower 16 x 16 blocks of G over four warps, at most three a warp; all sums
-// stay in registers until the staged input is no longer needed.
-template <int JOBS>
+// Lower 16 x 16 blocks of G over WARPS warps, at most JOBS a warp; all sums stay
+// in registers until the staged input is no longer needed.
+template <int JOBS, int WARPS>
 __device__ __forceinline__ void gram_tiles(const float *As, Stage st, int m8, int nt8, double *G, int ld) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
     double acc[JOBS][2][2][2];
@@ -530,7 +522,7 @@ __device__ __forceinline__ void gram_tiles(const float *As, Stage st, int m8, in
     bool own[JOBS];
 #pragma unroll
     for (int j = 0; j < JOBS; ++j) {
-        int g = 0, job = warp + 4 * j;   // block row g has g + 1 blocks
+        int g = 0, job = warp + WARPS * j;   // block row g has g + 1 blocks
         while (job > g) { job -= g + 1; ++g; }
         tr[j] = 2 * g;
         tc[j] = 2 * job;
@@ -577,19 +569,23 @@ __device__ __forceinline__ void gram_tiles(const float *As, Stage st, int m8, in
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kFacT, 6) factor_kernel(Params p) {
+// THREADS 128 up to 128 x 64, 256 up to 256 x 128.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == kFacT ? 6 : 1) factor_kernel(Params p) {
+    constexpr bool BIG = THREADS != kFacT;
+    constexpr int N = BIG ? 128 : 64;
     extern __shared__ __align__(16) unsigned char smem[];
     int *prow = (int *)smem;
-    double2 *sd = (double2 *)(smem + 64 * 4);
-    unsigned *skey = (unsigned *)(smem + 64 * 4 + 64 * 16);
+    double2 *sd = (double2 *)(smem + N * 4);
+    unsigned *skey = (unsigned *)(smem + N * 4 + N * 16);
     int *sex = (int *)(skey + 8);
-    double *G = (double *)(smem + kFacHead);
+    double *G = (double *)(smem + FacHead<N>::bytes);
     for (int64_t idx = blockIdx.x; idx < p.count; idx += gridDim.x) {
         const int64_t mat = p.order ? (int64_t)p.order[idx] : idx;
         const jb_matrix_desc d = desc_of(p, mat);
         int st = JB_ST_OK;
         const int mt = d.m > d.n ? d.m : d.n, nt = d.m > d.n ? d.n : d.m;
-        if (!rdesc_fits(d, kB32, 4, p, true)) {
+        if (!rdesc_fits(d, kB32, 4, p, true, BIG ? kMaxRL : kMaxR, BIG ? kMaxRVL : kMaxRV)) {
             st = JB_ST_BAD_DESC;
         } else if ((d.flags & JB_FULL_MATRICES) && mt > nt) {
             st = kPending;
@@ -597,17 +593,20 @@ __global__ void __launch_bounds__(kFacT, 6) factor_kernel(Params p) {
             const int m8 = round8(mt), n8 = round8(nt), ld = n8;
             const Stage sg = stage_of(d.m < d.n, m8, n8);
             float *As = (float *)G;
-            stage_tall((const float *)p.A + d.a_off, d, m8, n8, sg, As, kFacT);
-            if (threadIdx.x < 64) prow[threadIdx.x] = 0;
+            stage_tall((const float *)p.A + d.a_off, d, m8, n8, sg, As, THREADS);
+            if (threadIdx.x < N) prow[threadIdx.x] = 0;
             __syncthreads();
-            if (nt > 32) gram_tiles<3>(As, sg, m8, n8 >> 3, G, ld);
-            else gram_tiles<1>(As, sg, m8, n8 >> 3, G, ld);
+            if (BIG) gram_tiles<5, THREADS / 32>(As, sg, m8, n8 >> 3, G, ld);
+            else if (nt > 32) gram_tiles<3, THREADS / 32>(As, sg, m8, n8 >> 3, G, ld);
+            else gram_tiles<1, THREADS / 32>(As, sg, m8, n8 >> 3, G, ld);
             // a diagonal of G is not finite exactly when the input is not
             const double gd = threadIdx.x < nt ? G[(size_t)threadIdx.x * ld + threadIdx.x] : 0.0;
             const int ex = __reduce_max_sync(FULL, (__double2hiint(fabs(gd)) >> 20) & 0x7ff);
             if ((threadIdx.x & 31) == 0) sex[threadIdx.x >> 5] = ex;
             const bool bad = __syncthreads_or(!isfinite(gd));
-            const int em = max(sex[0], sex[1]);   // nt <= 64: the first two warps
+            int em = sex[0];   // the warps that hold rows
+#pragma unroll
+            for (int w = 1; w < N / 32; ++w) em = max(em, sex[w]);
             if (bad) {
                 st = JB_ST_NONFINITE_IN;
             } else if (em < 32) {
@@ -618,7 +617,9 @@ __global__ void __launch_bounds__(kFacT, 6) factor_kernel(Params p) {
                 const double scl = __hiloint2double((1023 - 2 * half) << 20, 0);
                 const double rscl = __hiloint2double((1023 - half) << 20, 0);
                 bool ok = true;
-                if (nt > 32) {
+                if (BIG && nt > 64) {
+                    if (threadIdx.x < 128) ok = pivoted_cholesky<4>(G, ld, nt, kPivotCut, scl, rscl, prow, sd, skey);
+                } else if (nt > 32) {
                     if (threadIdx.x < 64) ok = pivoted_cholesky<2>(G, ld, nt, kPivotCut, scl, rscl, prow, sd, skey);
                 } else {
                     if (threadIdx.x < 32) ok = pivoted_cholesky<1>(G, ld, nt, kPivotCut, scl, rscl, prow, sd, skey);
@@ -627,7 +628,7 @@ __global__ void __launch_bounds__(kFacT, 6) factor_kernel(Params p) {
                     st = kPending;
                 } else {
                     float *x = p.x32 + d.x_off;
-                    for (int c = threadIdx.x >> 5; c < nt; c += kFacT / 32)
+                    for (int c = threadIdx.x >> 5; c < nt; c += THREADS / 32)
                         for (int i = threadIdx.x & 31; i < nt; i += 32)
                             x[c * nt + i] = (float)(G[prow[c] + i] * rscl);
                 }
@@ -989,6 +990,338 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
             else p.sweeps[mat] += pass;
         }
         __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 refinement above 128 x 64 (up to 256 x 128): the same passes by a cluster
+// of CTAs a matrix, as W (266 KB) does not fit one SM.  Every CTA keeps all of
+// V and 32 rows of W in shared memory.  Per pass: W rows = A rows V; the CTA's
+// part of H = W^T W to the workspace (16 x 16 blocks in mma layout); each CTA
+// then sums its share of the blocks over the parts, forms E and N there, and
+// writes N into the shared memory of the CTAs that own its columns; these
+// update their columns of V and write them into every CTA's copy.  Four
+// cluster barriers a pass.  One matrix uses 8 SMs instead of one: 256 x 128 in
+// 0.09 ms, against 2.31 ms for gram64_kernel.
+// ---------------------------------------------------------------------------
+constexpr int kLgRows = 32, kLgN = 128;
+
+struct LgGeo {
+    int n8, ldv, nb16, gpc;   // padded width, its ld, 16-column groups, groups a CTA
+};
+__host__ __device__ inline LgGeo lg_geo(int nt, int cs) {
+    LgGeo g;
+    g.n8 = round8(nt);
+    g.ldv = ld4odd(g.n8);
+    g.nb16 = (g.n8 + 15) >> 4;
+    g.gpc = (g.nb16 + cs - 1) / cs;
+    return g;
+}
+__host__ __device__ inline size_t lg_panel(const LgGeo &g) {   // N panel or the staged rows of A
+    const size_t n = (size_t)16 * g.gpc * g.ldv * 8, a = stage_floats(kLgRows, g.n8) * 4;
+    return n > a ? n : a;
+}
+__host__ __device__ inline size_t lg_smem(int nt, int cs) {
+    const LgGeo g = lg_geo(nt, cs);
+    return (size_t)kLgN * 8 * 3 + kLgN * 4 + 16 * 4 + (size_t)g.n8 * g.ldv * 8 + (size_t)g.n8 * ld4odd(kLgRows) * 8 +
+           lg_panel(g);
+}
+// Workspace of one matrix: a part of H for every CTA with rows.
+__host__ __device__ inline size_t lg_part_bytes(int mt, int nt) {
+    const int nb = (round8(nt) + 15) >> 4;
+    return (size_t)((mt + kLgRows - 1) / kLgRows) * (nb * (nb + 1) / 2) * 256 * 8;
+}
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// This CTA's shared address as seen in CTA `rank` of the cluster.
+__device__ __forceinline__ unsigned remote_smem(const void *ptr, unsigned rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(ptr)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void remote_store(unsigned addr, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ void remote_store(unsigned addr, int v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+// Block index -> block row and column (rows of the lower triangle).
+__device__ __forceinline__ void lower_block(int b, int &bi, int &bj) {
+    bi = 0;
+    while (b > bi) { b -= bi + 1; ++bi; }
+    bj = b;
+}
+
+template <int CS>
+__global__ void __launch_bounds__(kRefT, 1) refine_large_kernel(Params p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    const unsigned rank = cluster_rank();
+    const int slot = blockIdx.x / CS, slots = gridDim.x / CS;
+    double *part = (double *)(p.gws + (size_t)slot * p.gws_stride);
+    double *dh = (double *)smem, *de = dh + kLgN, *sig = de + kLgN;
+    int *perm = (int *)(sig + kLgN);
+    int *flags = perm + kLgN;            // one word of every CTA
+    double *V = (double *)(flags + 16);
+    for (int64_t idx = slot; idx < p.count; idx += slots) {
+        const int mat = p.order ? p.order[idx] : (int)idx;
+        if (p.status[mat] != JB_ST_OK) continue;      // the same for the whole cluster
+        const jb_matrix_desc d = desc_of(p, mat);
+        const bool wide = d.m < d.n;
+        const int mt = wide ? d.n : d.m, nt = wide ? d.m : d.n;
+        const LgGeo g = lg_geo(nt, CS);
+        const int ldv = g.ldv, nt8 = g.n8 >> 3, nblk = g.nb16 * (g.nb16 + 1) / 2;
+        constexpr int ldw = 36;                        // ld4odd(kLgRows)
+        const int row0 = rank * kLgRows, rows = min(max(mt - row0, 0), kLgRows);
+        const int parts = (mt + kLgRows - 1) / kLgRows;
+        double *W = V + (size_t)g.n8 * ldv;
+        double *Np = W + (size_t)g.n8 * ldw;           // columns 16 gpc rank ..., ld ldv
+        float *As = (float *)Np;
+        const Stage sg = stage_of(wide, kLgRows, g.n8);
+        {
+            const float *x = p.x32 + d.x_off;
+            for (int c = warp; c < g.n8; c += kRefT / 32)
+                for (int i = lane; i < g.n8; i += 32)
+                    V[c * ldv + i] = (c < nt && i < nt) ? (double)x[c * nt + i] : 0.0;
+        }
+        const double tol = p.tol > 0 ? (double)(float)p.tol : (double)(10.0f * Lim<float>::eps());
+        const double tol2 = tol * tol;
+        const int most = p.max_sweeps < kRefPasses ? p.max_sweeps : kRefPasses;
+        int pass = 1;
+        bool done = false;
+        for (; pass <= most; ++pass) {
+            // rows row0 .. of A, zero past the end
+            const float *A = (const float *)p.A + d.a_off;
+            for (int k = threadIdx.x; k < kLgRows * g.n8; k += kRefT) {
+                const int i = wide ? k % kLgRows : k / g.n8, c = wide ? k / kLgRows : k % g.n8;
+                const bool in = i < rows && c < nt;
+                const float *src = wide ? A + (size_t)c * mt + row0 + i : A + (size_t)(row0 + i) * nt + c;
+                cp_async4(As + i * sg.sr + c * sg.sk, in ? src : A, in);
+            }
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            ref_mul<4, 1, false>(As, sg.sr, sg.sk, V, ldv, W, ldw, g.n8, kLgRows / 8, nt8);
+            __syncthreads();
+            if (rows > 0) {
+                double *mine = part + (size_t)rank * nblk * 256;
+                for (int b = warp; b < nblk; b += kRefT / 32) {
+                    int bi, bj;
+                    lower_block(b, bi, bj);
+                    double h0[2][2], h1[2][2];
+                    ref_gram(W, ldw, kLgRows, 2 * bi, min(2 * bj, nt8 - 1), nt8, h0);
+                    ref_gram(W, ldw, kLgRows, 2 * bi, min(2 * bj + 1, nt8 - 1), nt8, h1);
+                    double2 *o = (double2 *)(mine + b * 256 + lane * 8);   // tiles (0,0) (0,1) (1,0) (1,1)
+                    o[0] = make_double2(h0[0][0], h0[0][1]);
+                    o[1] = make_double2(h1[0][0], h1[0][1]);
+                    o[2] = make_double2(h0[1][0], h0[1][1]);
+                    o[3] = make_double2(h1[1][0], h1[1][1]);
+                }
+            }
+            cluster_sync();
+            // diagonals of H (over the parts) and of E, in every CTA
+            for (int c = threadIdx.x; c < nt; c += kRefT) {
+                const int b16 = c >> 4, b = b16 * (b16 + 1) / 2 + b16, e = c & 15, f = e & 7;
+                const int at = b * 256 + (f * 4 + (f >> 1)) * 8 + (e >> 3) * 6 + (f & 1);
+                double sum = 0.0;
+                for (int q = 0; q < parts; ++q) sum += part[(size_t)q * nblk * 256 + at];
+                dh[c] = sum;
+            }
+            for (int c = warp; c < nt; c += kRefT / 32) {
+                double sum = 0.0;
+                for (int i = lane; i < nt; i += 32) sum = fma(V[c * ldv + i], V[c * ldv + i], sum);
+                sum = warp_sum(sum);
+                if (lane == 0) de[c] = sum - 1.0;
+            }
+            __syncthreads();
+            // this CTA's blocks: the test, and N to the owners of its columns
+            int need = 0, wild = 0;
+            for (int b = rank + CS * warp; b < nblk; b += CS * (kRefT / 32)) {
+                int bi, bj;
+                lower_block(b, bi, bj);
+                double h[2][2][2] = {}, e0[2][2], e1[2][2];
+                for (int q = 0; q < parts; ++q) {
+                    const double2 *o = (const double2 *)(part + ((size_t)q * nblk + b) * 256 + lane * 8);
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        const double2 v = o[t];
+                        h[t >> 1][t & 1][0] += v.x;
+                        h[t >> 1][t & 1][1] += v.y;
+                    }
+                }
+                ref_gram(V, ldv, g.n8, 2 * bi, min(2 * bj, nt8 - 1), nt8, e0);
+                ref_gram(V, ldv, g.n8, 2 * bi, min(2 * bj + 1, nt8 - 1), nt8, e1);
+                const unsigned to_c = remote_smem(Np, bj / g.gpc), to_r = remote_smem(Np, bi / g.gpc);
+                const int c0 = (bj % g.gpc) * 16, r0 = (bi % g.gpc) * 16;
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int rl = a * 8 + lr, cl = t * 8 + 2 * lk + u;
+                            const int r = bi * 16 + rl, c = bj * 16 + cl;
+                            if (r >= g.n8 || c > r) continue;
+                            double nrc = 0.0, ncr = 0.0;
+                            if (r < nt) {
+                                const double hh = h[a][t][u], ee = c == r ? de[r] : (t ? e1 : e0)[a][u];
+                                if (!(fabs(ee) <= kRefOrth)) need = 1;
+                                if (c == r) {
+                                    nrc = -0.5 * ee;
+                                } else {
+                                    if (!(hh * hh <= tol2 * dh[r] * dh[c])) need = 1;
+                                    const double off = hh - 0.5 * ee * (dh[r] + dh[c]);
+                                    const double k = ref_angle(dh[r] * (1.0 - de[r]) - dh[c] * (1.0 - de[c]), off);
+                                    if (!(fabs(k) <= 0.25 && fabs(ee) <= 0.1)) wild = 1;
+                                    ncr = k - 0.5 * ee;     // N(c, r)
+                                    nrc = -k - 0.5 * ee;    // N(r, c)
+                                }
+                            }
+                            remote_store(to_c + ((c0 + cl) * ldv + r) * 8, nrc);
+                            if (c < r) remote_store(to_r + ((r0 + rl) * ldv + c) * 8, ncr);
+                        }
+            }
+            const int word = (__syncthreads_or(need) ? 1 : 0) | (__syncthreads_or(wild) ? 2 : 0);
+            if (threadIdx.x < CS) remote_store(remote_smem(flags + rank, threadIdx.x), word);
+            cluster_sync();
+            int all = 0;
+#pragma unroll
+            for (int q = 0; q < CS; ++q) all |= flags[q];
+            if (!(all & 1)) { done = true; break; }
+            if ((all & 2) || pass == most) break;
+            // second-order term on the diagonal of the owned columns: -sum_i N_ij^2 / 2
+            const int own0 = rank * g.gpc * 16, cols = min(max(nt - own0, 0), 16 * g.gpc);
+            for (int c = warp; c < cols; c += kRefT / 32) {
+                double sum = 0.0;
+                for (int i = lane; i < nt; i += 32)
+                    if (i != own0 + c) sum = fma(Np[c * ldv + i], Np[c * ldv + i], sum);
+                sum = warp_sum(sum);
+                if (lane == 0) Np[c * ldv + own0 + c] -= 0.5 * sum;
+            }
+            __syncthreads();
+            // the owned columns of V + V N: 16 x 16 blocks, one a warp and group
+            double acc[2][2][2][2];
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const int tc = 2 * (rank * g.gpc + s);     // first column tile
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) acc[s][a][t][0] = acc[s][a][t][1] = 0.0;
+                if (s < g.gpc && tc < nt8 && 2 * warp < nt8) {
+                    const double *x0 = V + lk * ldv + 16 * warp + lr;
+                    const double *x1 = V + lk * ldv + (2 * warp + 1 < nt8 ? 16 * warp + 8 : 16 * warp) + lr;
+                    const double *y0 = Np + (16 * s + lr) * ldv + lk;
+                    const double *y1 = tc + 1 < nt8 ? y0 + 8 * ldv : y0;
+#pragma unroll 2
+                    for (int k0 = 0; k0 < g.n8; k0 += 4) {
+                        const double fa = x0[k0 * ldv], fb = x1[k0 * ldv], f0 = y0[k0], f1 = y1[k0];
+                        dmma(acc[s][0][0], fa, f0);
+                        dmma(acc[s][1][0], fb, f0);
+                        dmma(acc[s][0][1], fa, f1);
+                        dmma(acc[s][1][1], fb, f1);
+                    }
+#pragma unroll
+                    for (int a = 0; a < 2; ++a)
+#pragma unroll
+                        for (int t = 0; t < 2; ++t)
+                            if (2 * warp + a < nt8 && tc + t < nt8) {
+                                const double *v = V + ((tc + t) * 8 + 2 * lk) * ldv + (2 * warp + a) * 8 + lr;
+                                acc[s][a][t][0] += v[0];
+                                acc[s][a][t][1] += v[ldv];
+                            }
+                }
+            }
+            cluster_sync();    // every CTA is done with the old V
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const int tc = 2 * (rank * g.gpc + s);
+                if (s < g.gpc && tc < nt8 && 2 * warp < nt8) {
+#pragma unroll
+                    for (int a = 0; a < 2; ++a)
+#pragma unroll
+                        for (int t = 0; t < 2; ++t)
+                            if (2 * warp + a < nt8 && tc + t < nt8) {
+                                const double *v = V + ((tc + t) * 8 + 2 * lk) * ldv + (2 * warp + a) * 8 + lr;
+#pragma unroll
+                                for (int q = 0; q < CS; ++q) {
+                                    const unsigned to = remote_smem(v, q);
+                                    remote_store(to, acc[s][a][t][0]);
+                                    remote_store(to + ldv * 8, acc[s][a][t][1]);
+                                }
+                            }
+                }
+            }
+            cluster_sync();
+        }
+        // sigma, the stable descending order and the cut (primitives.py:356-366), in every CTA
+        int st = JB_ST_OK;
+        if (done) {
+            for (int j = threadIdx.x; j < nt; j += kRefT) sig[j] = sqrt(dh[j]);
+            __syncthreads();
+            int below = 0;
+            for (int j = threadIdx.x; j < nt; j += kRefT) {
+                const double sj = sig[j];
+                int rnk = 0;
+                double smax = 0.0;
+                for (int i = 0; i < nt; ++i) {
+                    const double si = sig[i];
+                    rnk += (si > sj) || (si == sj && i < j);
+                    smax = fmax(smax, si);
+                }
+                const int npref = nt + (nt & 1);
+                if (!(sj > Lim<double>::eps() * (mt > npref ? mt : npref) * smax)) below = 1;
+                perm[rnk] = j;
+                dh[j] = 1.0 / sj;
+            }
+            if (__syncthreads_or(below)) done = false;   // columns to complete: not here
+        }
+        int bad = 0;
+        if (!done) {
+            st = kPending;
+        } else {
+            if (rank == 0 && threadIdx.x < d.rank) {
+                const float o = (float)sig[perm[threadIdx.x]];
+                if (!isfinite(o)) bad = 1;
+                ((float *)p.S + d.s_off)[threadIdx.x] = o;
+            }
+            if (!(d.flags & JB_VALUES_ONLY)) {
+                float *U = (float *)p.U + d.u_off, *Vh = (float *)p.Vh + d.v_off;
+                // W's rows of this CTA: rows of U, or columns of Vh of a wide matrix
+                for (int k = threadIdx.x; k < rows * d.rank; k += kRefT) {
+                    const int i = wide ? k % rows : k / d.rank, r = wide ? k / rows : k % d.rank, c = perm[r];
+                    const float o = (float)(W[c * ldw + i] * dh[c]);
+                    if (!isfinite(o)) bad = 1;
+                    if (wide) Vh[(size_t)r * mt + row0 + i] = o;
+                    else U[(size_t)(row0 + i) * d.rank + r] = o;
+                }
+                // V's part: nt x rank entries shared out over the cluster
+                for (int k = rank * kRefT + threadIdx.x; k < nt * d.rank; k += CS * kRefT) {
+                    const int i = wide ? k / d.rank : k % nt, r = wide ? k % d.rank : k / nt;
+                    const float o = (float)V[perm[r] * ldv + i];
+                    if (!isfinite(o)) bad = 1;
+                    if (wide) U[(size_t)i * d.rank + r] = o;
+                    else Vh[(size_t)r * nt + i] = o;
+                }
+            }
+        }
+        const int word = __syncthreads_or(bad);
+        if (threadIdx.x == 0) remote_store(remote_smem(flags + 8 + rank, 0), word);
+        cluster_sync();   // also: no CTA starts on the next matrix while another reads this one's
+        if (rank == 0 && threadIdx.x == 0) {
+            for (int q = 0; q < CS; ++q)
+                if (flags[8 + q]) st = JB_ST_NONFINITE_OUT;
+            p.status[mat] = st;
+            if (st == kPending) atomicAdd(p.n_pending, 1);
+            else p.sweeps[mat] += pass;
+        }
     }
 }
 
