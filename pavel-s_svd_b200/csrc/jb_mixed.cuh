@@ -24,9 +24,10 @@
 //     refinement of Ogita and Aishima).  Usually one correction.
 //
 // Measured (B200, 8192 matrices n ~ U[8,64], m ~ U[n,2n]; ms a batch): factor
-// 0.37, precondition 0.86, refine 1.01, against 4.55 + 3.03 of the register
+// 0.33, precondition 0.86, refine 1.01, against 4.55 + 3.03 of the register
 // kernels' FP32 and FP64 phases from V = I; 4096 x 128 x 64 over three decades
-// 0.44 + 1.00 + 1.03 against 12.9.  U is also closer to LAPACK's (1.4e-7 against
+// 0.38 + 1.00 + 1.04 against 12.9; one 256 x 128 over four decades 0.14 + 0.41 +
+// 0.15 against 4.1 + 2.3.  U is also closer to LAPACK's (1.4e-7 against
 // 1.4e-6: all pairs are corrected, not only those above tol).
 //
 // A matrix that this does not suit -- numerically rank-deficient, full bases
@@ -123,7 +124,7 @@ __device__ __forceinline__ void stage_tall(const float *A, const jb_matrix_desc 
 // groups hold all columns, so a matrix needs two warps.  Issue-bound (62 % of
 // the issue slots at 16 warps an SM, registers the limit); plain instead of
 // scaled rotations, unrolled intra steps and the factor in the same kernel (12
-// warps an SM) took 1.62 ms for factor and sweeps on the uneven batch, 1.22 now.
+// warps an SM) took 1.62 ms for factor and sweeps on the uneven batch, 1.19 now.
 // ---------------------------------------------------------------------------
 // The columns are kept scaled, w = scale * (the tile's column): a rotation is
 // then x - a y, y + b x with both columns' scales multiplied by c (Gentleman's
@@ -407,7 +408,7 @@ __host__ __device__ inline size_t pre_smem(int nt) {
 // THREADS 64 up to 64 columns, 256 up to 128 (which also takes the narrower
 // matrices of such a batch).
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == kPreT ? 8 : 2) precondition_kernel(Params p) {
+__global__ void __launch_bounds__(THREADS, THREADS == kPreT ? 8 : 1) precondition_kernel(Params p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_idx;
     float *xb = (float *)smem;
@@ -447,19 +448,24 @@ __global__ void __launch_bounds__(THREADS, THREADS == kPreT ? 8 : 2) preconditio
 // The factor L.
 // ---------------------------------------------------------------------------
 // Pivoted Cholesky of G (n x n, both triangles, ld), thread i = row i, by one
-// warp (n <= 32), two or four: step k takes the largest remaining diagonal p and
-// leaves column k of L in row p of G (rows chosen before: zero), p * ld in
-// prow[k].  The pivot is found on FP32 keys that carry the row (redux); one
+// warp (n <= 32), two or four.  Step k takes the largest remaining diagonal, row
+// p at column position q; every thread swaps columns k and q of its own row,
+// so that columns 0 .. k - 1 of a row hold L's and both factors of a dot
+// product are runs of shared memory (ld = 2 mod 4: conflict-free 16-byte reads,
+// row p a broadcast).  At the end G(i, k) is column k of L (0 in rows chosen
+// before).  The pivot is found on FP32 keys that carry the row (redux); one
 // barrier a step.  scl brings the largest diagonal to about 1, rscl is its
 // square root.  False when a pivot is <= cut (scaled).
 template <int WARPS>
 __device__ __forceinline__ bool pivoted_cholesky(double *G, int ld, int n, double cut, double scl, double rscl,
-                                                 int *prow, double2 *sd, unsigned *skey) {
-    const int i = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+                                                 double2 *sd, int *spos, unsigned *skey) {
     constexpr unsigned M = WARPS == 4 ? 127u : 63u;   // the key's bits for the row
-    double d = i < n ? G[i * ld + i] : 0.0;
-    bool taken = i >= n;
-    double *gi = G + min(i, ld - 1);
+    const int i = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool row = i < n;
+    double *gi = G + min(i, n - 1) * ld;
+    double d = row ? gi[i] : 0.0;
+    bool taken = !row;
+    int pos = i;
     for (int k = 0; k < n; ++k) {
         const float df = (float)(d * scl);
         const unsigned key = taken ? 0u : ((__float_as_uint(fmaxf(df, 0.f)) & ~M) | (M - i)) + (M + 1u);
@@ -467,7 +473,10 @@ __device__ __forceinline__ bool pivoted_cholesky(double *G, int ld, int n, doubl
         // 1 / sqrt(d): FP32 estimate, one Newton step (1e-14)
         const double r0 = (double)rsqrt_ftz(df);
         const double rs = r0 * fma(-0.5 * (d * scl), r0 * r0, 1.5) * rscl;
-        if (!taken) sd[i] = make_double2(d, rs);
+        if (!taken) {
+            sd[i] = make_double2(d, rs);
+            spos[i] = pos;
+        }
         if (WARPS > 1) {
             if (lane == 0) skey[WARPS * (k & 1) + warp] = kw;
             asm volatile("bar.sync 1, %0;" ::"n"(32 * WARPS) : "memory");
@@ -479,36 +488,50 @@ __device__ __forceinline__ bool pivoted_cholesky(double *G, int ld, int n, doubl
         }
         const int p = (int)(M - (kw & M));
         const double2 dr = sd[p];
+        const int q = spos[p];
         if (!(dr.x * scl > cut)) return false;
-        const double *gq = G + p;
-        double v0 = gi[p * ld], v1 = 0.0, v2 = 0.0, v3 = 0.0;
+        const double *gp = G + p * ld;
+        const double g = gi[q], gk = gi[k];
+        double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
         int j = 0;
 #pragma unroll 2
-        for (; j + 4 <= k; j += 4) {
-            const int4 r = *(const int4 *)(prow + j);
-            v0 = fma(-gi[r.x], gq[r.x], v0);
-            v1 = fma(-gi[r.y], gq[r.y], v1);
-            v2 = fma(-gi[r.z], gq[r.z], v2);
-            v3 = fma(-gi[r.w], gq[r.w], v3);
+        for (; j + 8 <= k; j += 8) {
+#pragma unroll
+            for (int t = 0; t < 8; t += 4) {
+                const double2 a = *(const double2 *)(gi + j + t), b = *(const double2 *)(gp + j + t);
+                const double2 e = *(const double2 *)(gi + j + t + 2), f = *(const double2 *)(gp + j + t + 2);
+                v0 = fma(a.x, b.x, v0);
+                v1 = fma(a.y, b.y, v1);
+                v2 = fma(e.x, f.x, v2);
+                v3 = fma(e.y, f.y, v3);
+            }
         }
 #pragma unroll 1
-        for (; j < k; ++j) v0 = fma(-gi[prow[j]], gq[prow[j]], v0);
-        const double l = taken ? 0.0 : (i == p ? dr.x : (v0 + v1) + (v2 + v3)) * dr.y;
-        if (i < ld) gi[p * ld] = l;
+        for (; j + 2 <= k; j += 2) {
+            const double2 a = *(const double2 *)(gi + j), b = *(const double2 *)(gp + j);
+            v0 = fma(a.x, b.x, v0);
+            v1 = fma(a.y, b.y, v1);
+        }
+        if (j < k) v2 = fma(gi[j], gp[j], v2);
+        const double l = taken ? 0.0 : (i == p ? dr.x : g - ((v0 + v1) + (v2 + v3))) * dr.y;
+        if (row) {
+            gi[q] = gk;
+            gi[k] = l;
+        }
         if (i == p) taken = true;
+        else if (pos == k) pos = q;
         d = fma(-l, l, d);
-        if (i == 0) prow[k] = p * ld;
     }
     return true;
 }
 
-// Shared memory: prow (N ints), sd (N double2), skey (8), sex (8), then G (n8 x
-// n8 doubles) and the staged input in one place; N = 64 or 128 columns.
+// Shared memory: spos (N ints), sd (N double2), skey (8), sex (8), then G (n8
+// rows of n8 + 2 doubles) and the staged input in one place; N = 64 or 128 columns.
 template <int N> struct FacHead { static constexpr size_t bytes = N * 4 + N * 16 + 8 * 4 + 8 * 4; };
 template <int N>
 __host__ __device__ inline size_t fac_smem(int mt, int nt) {
     const int m8 = round8(mt), n8 = round8(nt);
-    const size_t g = (size_t)n8 * n8 * 8, a = stage_floats(m8, n8) * 4;
+    const size_t g = (size_t)n8 * (n8 + 2) * 8, a = stage_floats(m8, n8) * 4;
     return FacHead<N>::bytes + (g > a ? g : a);
 }
 
@@ -575,7 +598,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == kFacT ? 6 : 1) factor_kern
     constexpr bool BIG = THREADS != kFacT;
     constexpr int N = BIG ? 128 : 64;
     extern __shared__ __align__(16) unsigned char smem[];
-    int *prow = (int *)smem;
+    int *spos = (int *)smem;
     double2 *sd = (double2 *)(smem + N * 4);
     unsigned *skey = (unsigned *)(smem + N * 4 + N * 16);
     int *sex = (int *)(skey + 8);
@@ -590,11 +613,10 @@ __global__ void __launch_bounds__(THREADS, THREADS == kFacT ? 6 : 1) factor_kern
         } else if ((d.flags & JB_FULL_MATRICES) && mt > nt) {
             st = kPending;
         } else {
-            const int m8 = round8(mt), n8 = round8(nt), ld = n8;
+            const int m8 = round8(mt), n8 = round8(nt), ld = n8 + 2;
             const Stage sg = stage_of(d.m < d.n, m8, n8);
             float *As = (float *)G;
             stage_tall((const float *)p.A + d.a_off, d, m8, n8, sg, As, THREADS);
-            if (threadIdx.x < N) prow[threadIdx.x] = 0;
             __syncthreads();
             if (BIG) gram_tiles<5, THREADS / 32>(As, sg, m8, n8 >> 3, G, ld);
             else if (nt > 32) gram_tiles<3, THREADS / 32>(As, sg, m8, n8 >> 3, G, ld);
@@ -618,11 +640,11 @@ __global__ void __launch_bounds__(THREADS, THREADS == kFacT ? 6 : 1) factor_kern
                 const double rscl = __hiloint2double((1023 - half) << 20, 0);
                 bool ok = true;
                 if (BIG && nt > 64) {
-                    if (threadIdx.x < 128) ok = pivoted_cholesky<4>(G, ld, nt, kPivotCut, scl, rscl, prow, sd, skey);
+                    if (threadIdx.x < 128) ok = pivoted_cholesky<4>(G, ld, nt, kPivotCut, scl, rscl, sd, spos, skey);
                 } else if (nt > 32) {
-                    if (threadIdx.x < 64) ok = pivoted_cholesky<2>(G, ld, nt, kPivotCut, scl, rscl, prow, sd, skey);
+                    if (threadIdx.x < 64) ok = pivoted_cholesky<2>(G, ld, nt, kPivotCut, scl, rscl, sd, spos, skey);
                 } else {
-                    if (threadIdx.x < 32) ok = pivoted_cholesky<1>(G, ld, nt, kPivotCut, scl, rscl, prow, sd, skey);
+                    if (threadIdx.x < 32) ok = pivoted_cholesky<1>(G, ld, nt, kPivotCut, scl, rscl, sd, spos, skey);
                 }
                 if (__syncthreads_or(!ok)) {
                     st = kPending;
@@ -630,7 +652,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == kFacT ? 6 : 1) factor_kern
                     float *x = p.x32 + d.x_off;
                     for (int c = threadIdx.x >> 5; c < nt; c += THREADS / 32)
                         for (int i = threadIdx.x & 31; i < nt; i += 32)
-                            x[c * nt + i] = (float)(G[prow[c] + i] * rscl);
+                            x[c * nt + i] = (float)(G[i * ld + c] * rscl);
                 }
             }
         }
@@ -1002,7 +1024,7 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
 // writes N into the shared memory of the CTAs that own its columns; these
 // update their columns of V and write them into every CTA's copy.  Four
 // cluster barriers a pass.  One matrix uses 8 SMs instead of one: 256 x 128 in
-// 0.09 ms, against 2.31 ms for gram64_kernel.
+// 0.145 ms, against 2.31 ms for gram64_kernel.
 // ---------------------------------------------------------------------------
 constexpr int kLgRows = 32, kLgN = 128;
 
