@@ -235,8 +235,9 @@ def svd(a, algorithm='jacobi', *, full_matrices=False, values_only=False, return
 # (complex, 48 x 32 to 128 x 64) no longer hold the matrix.
 QR_FIRST_ROWS = {torch.float32: 256, torch.float64: 128, torch.complex64: 128, torch.complex128: 128}
 # ... and its QR runs as TSQR for a batch of fewer matrices than SMs from this
-# m n^2 up (measured on B200, float64: 4096 x 128 77.7 -> 16.9 ms, 16 x
-# 1024 x 64 4.1 -> 3.4 ms; 2048 x 32 stays faster as one QR, 2.4 vs 3.6 ms).
+# m n^2 up when a matrix does not fit the QR's on-chip panels (up to 16 SMs,
+# about 3.5 MB: 4096 x 64 float64 fits; measured on B200, 4096 x 128 float64
+# 77.7 -> 16.9 ms).
 TSQR_WORK = 1 << 22
 
 
@@ -294,9 +295,11 @@ def _tall_svd(a, full_matrices, values_only, return_info, rank, precision, opts)
         b = xw.shape[0]
         sms = torch.cuda.get_device_properties(a.device).multi_processor_count
         leaves = min(sms // b, mt // (2 * nt))
-        if leaves >= 2 and mt * nt * nt >= TSQR_WORK:
-            # few large matrices: their QR by row tiles in parallel (TSQR), about
-            # one leaf per SM, instead of one CTA per matrix
+        if (leaves >= 2 and mt * nt * nt >= TSQR_WORK
+                and N.lib().jb_qr_workspace_bytes(mt, nt, b, xw.element_size()) > 0):
+            # few large matrices beyond the on-chip panels of a cluster of CTAs:
+            # their QR by row tiles in parallel (TSQR), about one leaf per SM,
+            # instead of one CTA per matrix
             q, r = Q.tsqr(xw, -(-mt // leaves), {})
         else:
             q, r = Q.qr(xw)
