@@ -446,6 +446,19 @@ JB_API size_t jb_complete_null_workspace_bytes(int32_t dtype, int64_t batch, int
 JB_API int jb_complete_null(void *U, const uint8_t *keep, int32_t dtype, int64_t batch, int64_t m, int64_t n,
                             int32_t *status, void *workspace, size_t workspace_bytes, void *stream);
 
+/* A batch before a solver composed on the host (svd() of
+ * svdbench/standalone/solvers.py:291-295, 224-227): x (batch, rows, cols),
+ * row-major, dtype 0 float32, 1 float64, 2 complex64, 3 complex128, scaled by
+ * 2^-e per matrix (exact; max |x| = f 2^e, f in [0.5, 1)) into out, as it is or
+ * as its conjugate transpose (transpose), float32 as float64 when widen.
+ * scale[z] = 2^e; status[z] = JB_ST_OK, or JB_ST_NONFINITE_IN (out is then not
+ * to be used); keys: batch ints of scratch.  Two launches, no host round
+ * trip.  jb_check_finite sets *flag = 1 when an element of x is NaN or infinite
+ * (:305-306), and leaves it alone otherwise. */
+JB_API int jb_prepare(const void *x, int32_t dtype, void *out, int32_t widen, int32_t transpose, double *scale,
+                      int32_t *keys, int32_t *status, int64_t batch, int32_t rows, int32_t cols, void *stream);
+JB_API int jb_check_finite(const void *x, int32_t dtype, int64_t count, int32_t *flag, void *stream);
+
 /* Measurement kernel for the rooflines of the FP32/FP64 Jacobi kernels (no
  * counterpart in the reference): `blocks` CTAs of 256 threads, each thread
  * 16 independent fused multiply-add chains of `iters` steps; mode 0 FP32

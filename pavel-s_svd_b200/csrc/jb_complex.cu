@@ -152,10 +152,17 @@ __global__ void __launch_bounds__(kThreads) cjacobi_kernel(const C<R> *A, C<R> *
     for (int64_t z = blockIdx.x; z < batch; z += gridDim.x) {
         const C<R> *a = A + z * (int64_t)m * n;
         __syncthreads();
+        bool bad = false;
         for (size_t idx = threadIdx.x; idx < wsz; idx += blockDim.x) {
             const int c = (int)(idx / m), i = (int)(idx - (size_t)c * m);
-            W[idx] = c < n ? a[(size_t)i * n + c] : C<R>{R(0), R(0)};
+            const C<R> v = c < n ? a[(size_t)i * n + c] : C<R>{R(0), R(0)};
+            bad |= !(isfinite(v.re) && isfinite(v.im));
+            W[idx] = v;
         }
+        // NaN or infinity: reported, and a zero matrix solved in its place
+        bad = __syncthreads_or(bad);
+        if (bad)
+            for (size_t idx = threadIdx.x; idx < wsz; idx += blockDim.x) W[idx] = C<R>{R(0), R(0)};
         for (size_t idx = threadIdx.x; idx < vsz; idx += blockDim.x) {
             const int c = (int)(idx / np), i = (int)(idx - (size_t)c * np);
             V[idx] = C<R>{i == c ? R(1) : R(0), R(0)};
@@ -230,7 +237,7 @@ __global__ void __launch_bounds__(kThreads) cjacobi_kernel(const C<R> *A, C<R> *
                   Vh + z * (int64_t)n * n);
         if (threadIdx.x == 0) {
             if (sweeps_out) sweeps_out[z] = sweep > max_sweeps ? max_sweeps : sweep;
-            if (status) status[z] = converged ? JB_ST_OK : JB_ST_NOT_CONVERGED;
+            if (status) status[z] = bad ? JB_ST_NONFINITE_IN : converged ? JB_ST_OK : JB_ST_NOT_CONVERGED;
         }
     }
 }
@@ -267,10 +274,18 @@ __global__ void __launch_bounds__(THREADS) cgroup_kernel(const C<R> *A, C<R> *U,
         const C<R> *a = A + z * (int64_t)m * n;
         for (int idx = threadIdx.x; idx < npb * LD; idx += THREADS) area[idx] = R(0);
         __syncthreads();
+        bool bad = false;
         for (int idx = threadIdx.x; idx < m * n; idx += THREADS) {
             const int i = idx / n, c = idx - i * n;
-            *(C<R> *)(area + c * LD + 2 * i) = a[idx];
+            const C<R> v = a[idx];
+            bad |= !(isfinite(v.re) && isfinite(v.im));
+            *(C<R> *)(area + c * LD + 2 * i) = v;
         }
+        // NaN or infinity: reported, and a zero matrix solved in its place
+        bad = __syncthreads_or(bad);
+        if (bad)
+            for (int idx = threadIdx.x; idx < npb * LD; idx += THREADS) area[idx] = R(0);
+        __syncthreads();
         for (int c = threadIdx.x; c < n; c += THREADS) area[c * LD + K::G::VOFF + 2 * c] = R(1);
         __syncthreads();
         bool conv;
@@ -279,7 +294,7 @@ __global__ void __launch_bounds__(THREADS) cgroup_kernel(const C<R> *A, C<R> *U,
                   U + z * (int64_t)m * n, S + z * (int64_t)n, Vh + z * (int64_t)n * n);
         if (threadIdx.x == 0) {
             if (sweeps_out) sweeps_out[z] = ns;
-            if (status) status[z] = conv ? JB_ST_OK : JB_ST_NOT_CONVERGED;
+            if (status) status[z] = bad ? JB_ST_NONFINITE_IN : conv ? JB_ST_OK : JB_ST_NOT_CONVERGED;
         }
         __syncthreads();
     }

@@ -37,6 +37,9 @@ __device__ __forceinline__ int circ(int pos, int r, int n) {
 
 constexpr int kThreads = 512;
 
+// NaN (from a non-finite input) sorts last, so that the ranks are a permutation.
+__device__ __forceinline__ double order_key(double x) { return x == x ? x : INFINITY; }
+
 // mode 2: G and V in shared memory; 1: G only; 0: neither
 __host__ __device__ inline size_t smem_bytes(int np, int mode) {
     return (size_t)np * np * 8 * mode + (size_t)np * 8 + (size_t)np + 32 * 8 + (size_t)np * 4 + 64;
@@ -135,10 +138,10 @@ __global__ void __launch_bounds__(kThreads) eigh_kernel(const T *H, T *W, T *Vou
         __syncthreads();
         // ascending, stable; the padding column (index n) is left out
         for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            const double dj = G[(size_t)j * np + j];
+            const double dj = order_key(G[(size_t)j * np + j]);
             int rk = 0;
             for (int i = 0; i < n; ++i) {
-                const double di = G[(size_t)i * np + i];
+                const double di = order_key(G[(size_t)i * np + i]);
                 rk += (di < dj) || (di == dj && i < j);
             }
             perm[rk] = j;
@@ -278,10 +281,10 @@ __global__ void __launch_bounds__(kThreads) zeigh_kernel(const R *H, R *W, R *Vo
         }
         __syncthreads();
         for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            const double dj = G[(size_t)j * np + j].re;
+            const double dj = order_key(G[(size_t)j * np + j].re);
             int rk = 0;
             for (int i = 0; i < n; ++i) {
-                const double di = G[(size_t)i * np + i].re;
+                const double di = order_key(G[(size_t)i * np + i].re);
                 rk += (di < dj) || (di == dj && i < j);
             }
             perm[rk] = j;
@@ -363,7 +366,7 @@ __global__ void __launch_bounds__(THREADS) eigh_group_kernel(const T *H, T *Wo, 
             double sum = 0.0;
             for (int i = lane; i < NC * n; i += 32) sum = fma(v[i], w[i], sum);
             sum = warp_sum(sum);
-            if (lane == 0) lam[c] = sum;
+            if (lane == 0) lam[c] = order_key(sum);
         }
         __syncthreads();
         for (int j = threadIdx.x; j < n; j += THREADS) {

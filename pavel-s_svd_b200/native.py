@@ -33,7 +33,7 @@ SYMBOLS = ("jb_version", "jb_device_sm_count", "jb_workspace_bytes", "jb_svd_bat
            "jb_eigh_f64", "jb_eigh_complex_workspace_bytes", "jb_eigh_c64", "jb_eigh_c128",
            "jb_qr_workspace_bytes", "jb_qr_f32", "jb_qr_f64", "jb_qr_c64", "jb_qr_c128",
            "jb_svd_complex_workspace_bytes", "jb_svd_batched_c64", "jb_svd_batched_c128", "jb_jacobi_rounds",
-           "jb_complete_null_workspace_bytes", "jb_complete_null", "jb_fma_loop_flops", "jb_fma_loop",
+           "jb_complete_null_workspace_bytes", "jb_complete_null", "jb_prepare", "jb_check_finite", "jb_fma_loop_flops", "jb_fma_loop",
            "jb_svd_batched_f32_noalloc")
 GEMM_PLAIN, GEMM_SPLIT3, GEMM_SPLIT6, GEMM_B_MN, GEMM_CHAIN128, GEMM_SYRK = 0, 1, 2, 4, 8, 16
 EIG_FP32 = 128  # JB_EIG_FP32
@@ -136,6 +136,10 @@ def _declare(l):
     l.jb_complete_null_workspace_bytes.argtypes = [I32, I64, I64, I64]
     l.jb_complete_null.restype = ctypes.c_int
     l.jb_complete_null.argtypes = [P, P, I32, I64, I64, I64, P, P, SZ, P]
+    l.jb_prepare.restype = ctypes.c_int
+    l.jb_prepare.argtypes = [P, I32, P, I32, I32, P, P, P, I64, I32, I32, P]
+    l.jb_check_finite.restype = ctypes.c_int
+    l.jb_check_finite.argtypes = [P, I32, I64, P, P]
     l.jb_fma_loop_flops.restype = F64
     l.jb_fma_loop_flops.argtypes = [I32, I32]
     l.jb_fma_loop.restype = ctypes.c_int
@@ -158,12 +162,18 @@ def load(path: Path | None = None):
         return _lib
 
 
+_have_device = False
+
+
 def lib():
     """The loaded library, for compute calls: also requires a CUDA device."""
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("the B200 Jacobi solver needs a CUDA device; there is no CPU fallback")
-    return load()
+    global _have_device
+    if not _have_device:
+        import torch
+        if not torch.cuda.is_available():
+            raise RuntimeError("the B200 Jacobi solver needs a CUDA device; there is no CPU fallback")
+        _have_device = True
+    return _lib or load()
 
 
 def check(rc: int, what: str):

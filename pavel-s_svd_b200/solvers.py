@@ -97,6 +97,8 @@ def _validate(a, algorithm, full_matrices, opts):
 def raise_for_status(status, max_sweeps):
     """Map per-matrix status words to the reference's exceptions, with the
     reference's precedence (input check first, then convergence, then output)."""
+    if not bool(status.any()):
+        return
     if (status == N.ST_NONFINITE_IN).any():
         raise ValueError('input contains NaN or infinity')                        # solvers.py:291-292
     if (status == N.ST_NOT_CONVERGED).any():
@@ -229,6 +231,60 @@ def svd(a, algorithm='jacobi', *, full_matrices=False, values_only=False, return
     return (*result, stats) if return_info else result
 
 
+class _Verdicts:
+    """The words a composed solve leaves on the device and reads at once: the
+    input check of every matrix, the solver's sweeps and status, the null
+    completions' status, the output check."""
+
+    def __init__(self, batch, device):
+        self.batch = batch
+        self.words = torch.zeros(4 * batch + 1, dtype=torch.int32, device=device)
+        self.input, self.sweeps, self.status = (self.words[k * batch:(k + 1) * batch] for k in range(3))
+        self.keys = self.words[3 * batch:4 * batch]           # scratch of jb_prepare
+        self.finite = self.words[4 * batch:]
+        self.null = []
+
+    def check_finite(self, *tensors):
+        lib, stream = N.lib(), torch.cuda.current_stream(self.words.device).cuda_stream
+        for t in tensors:
+            if t.numel() == 0:
+                continue
+            t = t.conj() if t.is_conj() else t                # the memory, in any order
+            t = t.mT if t.mT.is_contiguous() else t.contiguous()
+            N.check(lib.jb_check_finite(t.data_ptr(), _NULL_DTYPES[t.dtype], t.numel(), self.finite.data_ptr(),
+                                        stream), 'jb_check_finite')
+
+    def read(self, max_sweeps=0):
+        """One copy to the host; the reference's exceptions in its order."""
+        host = (torch.cat([self.words] + self.null) if self.null else self.words).cpu()
+        b = self.batch
+        if bool(host[:b].any()):
+            raise ValueError('input contains NaN or infinity')                    # solvers.py:291-292
+        raise_for_status(host[2 * b:3 * b], max_sweeps)
+        _raise_for_null(host[4 * b + 1:])
+        if int(host[4 * b]):
+            raise RuntimeError('standalone solver produced nonfinite output')     # solvers.py:305-306
+        return int(host[b:2 * b].max()) if b else 0
+
+
+def _prepare(a, transpose, widen=False):
+    """The batch a (..., m, n) as (b, m, n), scaled by a power of two (exact),
+    conjugate-transposed when `transpose`, float32 in float64 when `widen`:
+    contiguous, with the scales (b, float64) and the verdicts to read later."""
+    m, n = a.shape[-2:]
+    x = a.detach().resolve_conj().resolve_neg().reshape(-1, m, n).contiguous()   # the kernel reads memory
+    b = x.shape[0]
+    out = torch.empty((b, n, m) if transpose else (b, m, n), dtype=torch.float64 if widen else a.dtype,
+                      device=a.device)
+    scale = torch.empty(b, dtype=torch.float64, device=a.device)
+    words = _Verdicts(b, a.device)
+    if b:
+        N.check(N.lib().jb_prepare(x.data_ptr(), _NULL_DTYPES[a.dtype], out.data_ptr(), int(widen), int(transpose),
+                                   scale.data_ptr(), words.keys.data_ptr(), words.input.data_ptr(), b, m, n,
+                                   torch.cuda.current_stream(a.device).cuda_stream), 'jb_prepare')
+    return out, scale, words
+
+
 # 'jacobi' input taller than this (tall view) and at least twice as tall as
 # wide is reduced to its R factor first (_tall_svd): beyond these rows the
 # register and large-tile kernels (real) or a shared-memory work area
@@ -279,19 +335,9 @@ def _tall_svd(a, full_matrices, values_only, return_info, rank, precision, opts)
     tol = opts.get('tol') or 10 * eps
     max_sweeps = opts.get('max_sweeps', 60)
     with torch.no_grad(), torch.cuda.device(a.device):
-        x = a.detach().reshape(-1, m, n)
-        if not bool(torch.isfinite(x).all()):
-            raise ValueError('input contains NaN or infinity')
-        amax = x.abs().amax((-2, -1), keepdim=True)
-        e = torch.where(amax > 0, torch.frexp(amax)[1], torch.zeros_like(amax, dtype=torch.int32))
-        scale = torch.ldexp(torch.ones_like(amax), e)
-        xs = x / scale
-        if wide:
-            xs = xs.mH
-        work = a.dtype
-        if a.dtype == torch.float32 and precision == 'mixed':
-            work = torch.float64
-        xw = xs.to(work).resolve_conj().contiguous()
+        widen = a.dtype == torch.float32 and precision == 'mixed'
+        xw, scale, words = _prepare(a, wide, widen)
+        work = xw.dtype
         b = xw.shape[0]
         sms = torch.cuda.get_device_properties(a.device).multi_processor_count
         leaves = min(sms // b, mt // (2 * nt))
@@ -311,9 +357,9 @@ def _tall_svd(a, full_matrices, values_only, return_info, rank, precision, opts)
         ur, sv, vhr, info = svd(r, 'jacobi', return_info=True, tol=tol, max_sweeps=max_sweeps, precision=rprec,
                                 ordering=opts.get('ordering', 'block'))
         keep = sv > eps * max(mt, nt + nt % 2) * sv[:, :1]
-        sv = (torch.where(keep, sv, torch.zeros_like(sv)) * scale[:, 0, :].to(sv.dtype)).to(real)
+        sv = (torch.where(keep, sv, torch.zeros_like(sv)) * scale[:, None]).to(real)
         v = vhr.mH.to(a.dtype)
-        u = None if values_only else _complete_null_columns((q @ ur.to(q.dtype)).to(a.dtype), keep)
+        u = None if values_only else _complete_null_columns((q @ ur.to(q.dtype)).to(a.dtype), keep, words)
         if wide:
             u, v = v, u
         if values_only:
@@ -323,8 +369,8 @@ def _tall_svd(a, full_matrices, values_only, return_info, rank, precision, opts)
         else:
             u, v = u[:, :, :rank], v[:, :, :rank]
         sv = sv[:, :rank] if not full_matrices else sv
-        if not all(bool(torch.isfinite(t).all()) for t in (sv,) + (() if values_only else (u, v))):
-            raise RuntimeError('standalone solver produced nonfinite output')
+        words.check_finite(sv, *(() if values_only else (u, v)))
+        words.read(max_sweeps)
         result = (None if values_only else u.resolve_conj().reshape(*shape, *u.shape[-2:]),
                   sv.reshape(*shape, sv.shape[-1]),
                   None if values_only else v.mH.resolve_conj().reshape(*shape, v.shape[-1], v.shape[-2]))
@@ -338,14 +384,24 @@ def _tall_svd(a, full_matrices, values_only, return_info, rank, precision, opts)
 _NULL_DTYPES = {torch.float32: 0, torch.float64: 1, torch.complex64: 2, torch.complex128: 3}
 
 
-def _complete_null_columns(u, keep):
+def _raise_for_null(status):
+    if not bool(status.any()):
+        return
+    if bool((status == N.ST_NULL_FAILED).any()):
+        raise RuntimeError("null-space completion failed: supplied live columns are not independent")
+    if bool((status == N.ST_TIMEOUT).any()):
+        raise RuntimeError("null-space completion: a device wait timed out")
+
+
+def _complete_null_columns(u, keep, words=None):
     """Replace the columns of u (b, m, n) not in keep by unit vectors
     orthogonal to the kept ones (primitives.py:430-455): per missing column,
     in column order, the coordinate vector of largest leftover leverage
     1 - sum |u|^2, projected out against the kept and completed columns,
     normalised; the same failure.  One launch of jb_complete_null on the
-    device holding u, then one read of the status words."""
-    u = u.contiguous().clone()
+    device holding u, then one read of the status words.  words (_Verdicts):
+    u is the caller's to overwrite, and the status is read with the others."""
+    u = u.resolve_conj().contiguous() if words is not None else u.contiguous().clone()
     b, m, n = u.shape
     if b == 0 or n == 0:
         return u
@@ -356,11 +412,10 @@ def _complete_null_columns(u, keep):
     status = torch.empty(b, dtype=torch.int32, device=u.device)
     N.check(lib.jb_complete_null(u.data_ptr(), keep.data_ptr(), dt, b, m, n, status.data_ptr(), ws.data_ptr(),
                                  ws.numel(), torch.cuda.current_stream(u.device).cuda_stream), "jb_complete_null")
-    st = status.cpu()
-    if bool((st == N.ST_NULL_FAILED).any()):
-        raise RuntimeError("null-space completion failed: supplied live columns are not independent")
-    if bool((st == N.ST_TIMEOUT).any()):
-        raise RuntimeError("null-space completion: a device wait timed out")
+    if words is not None:
+        words.null.append(status)
+    else:
+        _raise_for_null(status.cpu())
     return u
 
 
@@ -376,27 +431,22 @@ def _gram_svd(a, full_matrices, values_only, return_info, rank, opts):
     m, n = a.shape[-2:]
     shape = a.shape[:-2]
     with torch.no_grad(), torch.cuda.device(a.device):
-        x = a.detach().reshape(-1, m, n)
-        if not bool(torch.isfinite(x).all()):
-            raise ValueError('input contains NaN or infinity')
         wide = m < n
-        if wide:
-            x = x.mH
-        amax = x.abs().amax((-2, -1), keepdim=True)
-        e = torch.where(amax > 0, torch.frexp(amax)[1], torch.zeros_like(amax, dtype=torch.int32))
-        scale = torch.ldexp(torch.ones_like(amax), e)
-        xs = x / scale
+        xs, scale, words = _prepare(a, wide)
         g = xs.mH @ xs
         g = (g + g.mH) / 2
-        w, v, it = jacobi_eigh(g, max_sweeps=opts.get('max_sweeps', 60))
+        try:
+            w, v, it = jacobi_eigh(g, max_sweeps=opts.get('max_sweeps', 60))
+        finally:
+            words.read()     # the input check comes first, and nothing below sees a NaN
         w, v = w.flip(-1), v.flip(-1)
         nt = xs.shape[-1]
         cut = torch.finfo(w.dtype).eps * nt * w[:, :1].clamp_min(0)
         keep = w > cut
         sv = torch.where(keep, w.clamp_min(0).sqrt(), torch.zeros_like(w))
         u = (xs @ v) / torch.where(keep, sv, torch.ones_like(sv))[:, None, :]
-        u = _complete_null_columns(u, keep)
-        sv = sv * scale[:, 0, :]
+        u = _complete_null_columns(u, keep, words)
+        sv = (sv * scale[:, None]).to(sv.dtype)
         if wide:
             u, v = v, u
         if full_matrices:
@@ -408,8 +458,8 @@ def _gram_svd(a, full_matrices, values_only, return_info, rank, opts):
                                        torch.arange(n, device=v.device)[None, :].expand(v.shape[0], n) < v.shape[-1])
         else:
             u, sv, v = u[:, :, :rank], sv[:, :rank], v[:, :, :rank]
-        if not all(bool(torch.isfinite(t).all()) for t in (u, sv, v)):
-            raise RuntimeError('standalone solver produced nonfinite output')
+        words.check_finite(u, sv, v)
+        words.read()
         result = (None if values_only else u.resolve_conj().reshape(*shape, *u.shape[-2:]),
                   sv.reshape(*shape, sv.shape[-1]),
                   None if values_only else v.mH.resolve_conj().reshape(*shape, v.shape[-1], v.shape[-2]))
@@ -432,21 +482,13 @@ def _complex_svd(a, full_matrices, values_only, return_info, rank, opts):
     shape = a.shape[:-2]
     max_sweeps = opts.get('max_sweeps', 60)
     with torch.no_grad(), torch.cuda.device(a.device):
-        x = a.detach().reshape(-1, m, n)
-        if not bool(torch.isfinite(x).all()):
-            raise ValueError('input contains NaN or infinity')
-        amax = x.abs().amax((-2, -1), keepdim=True)
-        e = torch.where(amax > 0, torch.frexp(amax)[1], torch.zeros_like(amax, dtype=torch.int32))
-        scale = torch.ldexp(torch.ones_like(amax), e)
         wide = m < n
-        xs = (x / scale).mH if wide else x / scale
-        xs = xs.resolve_conj().contiguous()   # the kernel reads memory: no lazy conjugate view
+        xs, scale, words = _prepare(a, wide)
         b, mt, nt = xs.shape
         real = a.real.dtype
         u = torch.empty(b, mt, nt, dtype=a.dtype, device=a.device)
         sv = torch.empty(b, nt, dtype=real, device=a.device)
         vh = torch.empty(b, nt, nt, dtype=a.dtype, device=a.device)
-        info = torch.zeros(2, max(b, 1), dtype=torch.int32, device=a.device)
         if b:
             lib = N.lib()
             elem = xs.element_size()
@@ -454,16 +496,11 @@ def _complex_svd(a, full_matrices, values_only, return_info, rank, opts):
                 lib.jb_svd_complex_workspace_bytes(mt, nt, b, elem), a.device)
             fn = lib.jb_svd_batched_c64 if a.dtype == torch.complex64 else lib.jb_svd_batched_c128
             N.check(fn(xs.data_ptr(), u.data_ptr(), sv.data_ptr(), vh.data_ptr(), b, mt, nt,
-                       float(opts.get('tol') or 0.0), max_sweeps, info[0].data_ptr(), info[1].data_ptr(),
-                       ws.data_ptr(), ws.numel(), torch.cuda.current_stream(a.device).cuda_stream),
-                    'jb_svd_batched_complex')
-            host = info[:, :b].cpu()
-            raise_for_status(host[1], max_sweeps)
-            sweeps = int(host[0].max())
-        else:
-            sweeps = 0
-        u = _complete_null_columns(u, sv > 0)
-        sv = sv * scale[:, 0, :]
+                       float(opts.get('tol') or 0.0), max_sweeps, words.sweeps.data_ptr(),
+                       words.status.data_ptr(), ws.data_ptr(), ws.numel(),
+                       torch.cuda.current_stream(a.device).cuda_stream), 'jb_svd_batched_complex')
+        u = _complete_null_columns(u, sv > 0, words)
+        sv = (sv * scale[:, None]).to(real)
         v = vh.mH
         if wide:
             u, v = v, u
@@ -471,8 +508,8 @@ def _complex_svd(a, full_matrices, values_only, return_info, rank, opts):
             u, v = _complete_basis(u, m), _complete_basis(v, n)
         else:
             u, sv, v = u[:, :, :rank], sv[:, :rank], v[:, :, :rank]
-        if not all(bool(torch.isfinite(t).all()) for t in (u, sv, v)):
-            raise RuntimeError('standalone solver produced nonfinite output')
+        words.check_finite(u, sv, v)
+        sweeps = words.read(max_sweeps)
         result = (None if values_only else u.resolve_conj().reshape(*shape, *u.shape[-2:]),
                   sv.reshape(*shape, sv.shape[-1]),
                   None if values_only else v.mH.resolve_conj().reshape(*shape, v.shape[-1], v.shape[-2]))
@@ -566,25 +603,20 @@ def _composed_svd(a, algorithm, full_matrices, values_only, return_info, rank, o
         return u, s, vh.mH
 
     with torch.no_grad(), torch.cuda.device(a.device):
-        x = a.detach().reshape(-1, m, n)
-        if not bool(torch.isfinite(x).all()):
-            raise ValueError('input contains NaN or infinity')
-        amax = x.abs().amax((-2, -1), keepdim=True)
-        e = torch.where(amax > 0, torch.frexp(amax)[1], torch.zeros_like(amax, dtype=torch.int32))
-        scale = torch.ldexp(torch.ones_like(amax), e)
-        y = (x / scale).contiguous()
+        y, scale, words = _prepare(a, False)
         if algorithm == 'block_jacobi':
+            words.read()      # the rounds loop on the host: no NaN may enter them
             pair_v, check = _pair_solver(jopts, stats)
             u, sv, v = BR.raw(y, stats, opts, pair_v, check, _complete_null_columns)
         else:
             u, sv, v = Q.raw(y, algorithm, stats, opts, jacobi)
-        sv = sv * scale[:, 0, :]
+        sv = (sv * scale[:, None]).to(sv.dtype)
         if full_matrices:
             u, v = _complete_basis(u, m), _complete_basis(v, n)
         else:
             u, sv, v = u[:, :, :rank], sv[:, :rank], v[:, :, :rank]
-        if not all(bool(torch.isfinite(t).all()) for t in (u, sv, v)):
-            raise RuntimeError('standalone solver produced nonfinite output')
+        words.check_finite(u, sv, v)
+        words.read()
         result = (None if values_only else u.resolve_conj().reshape(*shape, *u.shape[-2:]),
                   sv.reshape(*shape, sv.shape[-1]),
                   None if values_only else v.mH.resolve_conj().reshape(*shape, v.shape[-1], v.shape[-2]))
