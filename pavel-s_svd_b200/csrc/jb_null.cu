@@ -141,44 +141,30 @@ __device__ __forceinline__ unsigned long long gtimer() {
     return t;
 }
 
-// Team-wide barrier.  G == 1: the CTA barrier.  G > 1: a two-level
-// generation barrier over the whole (co-resident, cooperative) grid: CTAs
-// arrive on the counter of their group of kGroupCTAs, the last of a group on
-// the counter of groups, and the last group releases everyone by bumping the
-// generation word, so no counter takes more than ~20 contending atomics.
-// Waits are bounded; returns false once any CTA of the team gave up.
-// bar[0] generation, bar[1] groups arrived, bar[2] error flag, bar[4 + k]
-// CTAs of group k arrived (the area is zeroed before the launch).
-constexpr int kGroupCTAs = 8;
+// Team-wide barrier.  G == 1: the CTA barrier.  G > 1: one counter of
+// arrivals over the whole (co-resident, cooperative) grid, waited on until the
+// generation's last arrival; a few ns a CTA on one L2 word, where two levels of
+// counters cost three dependent atomics (3.3 us a barrier over 128 CTAs; 1.9
+// with the one counter).  Waits are bounded; returns false once any CTA of the
+// team gave up.  bar[0] arrivals, bar[2] error flag (the area is zeroed before
+// the launch).
 __device__ __forceinline__ bool team_sync(unsigned *bar, int G) {
     __syncthreads();
     if (G == 1) return true;
     __shared__ int s_ok;
     if (threadIdx.x == 0) {
-        volatile unsigned *vgen = bar;
+        volatile unsigned *vbar = bar;
         volatile int *verr = (volatile int *)(bar + 2);
-        const unsigned gen = *vgen;
         __threadfence();
-        const int grp = blockIdx.x / kGroupCTAs, ngroups = (G + kGroupCTAs - 1) / kGroupCTAs;
-        const int gsize = min(kGroupCTAs, G - grp * kGroupCTAs);
+        const unsigned target = (atomicAdd(bar, 1u) / (unsigned)G + 1u) * (unsigned)G;
         int ok = 1;
-        if (atomicAdd(bar + 4 + grp, 1u) == (unsigned)gsize - 1) {
-            atomicExch(bar + 4 + grp, 0u);
-            __threadfence();
-            if (atomicAdd(bar + 1, 1u) == (unsigned)ngroups - 1) {
-                atomicExch(bar + 1, 0u);
-                __threadfence();
-                atomicAdd(bar, 1u);
-            }
-        }
         const unsigned long long t0 = gtimer();
-        while (*vgen == gen) {
+        while ((int)(*vbar - target) < 0) {
             if (gtimer() - t0 > kWaitNs) {
                 ok = 0;
                 atomicExch((int *)(bar + 2), 1);
                 break;
             }
-            __nanosleep(32);
         }
         __threadfence();
         s_ok = ok && !*verr;
@@ -266,19 +252,20 @@ __host__ __device__ inline int64_t x_stride(int64_t n, int esz) {
     return (n + v - 1) / v * v;
 }
 
-// Blocked pass of the team path (block_pass): the most candidate rows of a
-// block, columns per block at most, K chunk of its row products, and the
-// most rows a CTA may hold for it (its local sort).
-constexpr int kCandMax = 256;
+// Blocked pass of the team path (block_pass): the most rows the CTAs publish
+// for a block, the most of them it takes as candidates (their projector block
+// then fits in shared memory), columns per block at most, and the most rows a
+// CTA may hold for it (its local sort).
+constexpr int kPubMax = 256;
+constexpr int kCand = 128;
 constexpr int kBlk = 32;
-constexpr int kKC = 128;
 constexpr int kSortMax = 1024;
-static_assert(kCandMax % 64 == 0 && kBlk == 32 && kSortMax >= 64, "blocked pass sizes");
+static_assert(kCand == kThreads / 4 && kCand % 32 == 0 && kPubMax == kThreads / 2 && kBlk == 32 && kSortMax >= 64, "blocked pass sizes");
 
 // Per-team workspace layout (byte offsets from the team's base).  X, the
 // packed columns, and the blocked pass's areas exist only for multi-CTA teams:
 // cand (every CTA's best rows), bm (the candidate block of the projector,
-// kCandMax^2), bl (kBlk^2 triangular factor), bp (pivot rows), bv (pivot
+// kCand^2), bl (kBlk^2 triangular factor), bp (pivot rows), bv (pivot
 // leverages), bmeta.
 struct Layout {
     size_t x, lev, y, part, cmap, slots, bar, cand, bm, bl, bp, bv, bmeta, total;
@@ -295,8 +282,8 @@ __host__ __device__ inline Layout layout(int64_t m, int64_t n, int esz, int asz,
     L.cmap = o;  o += al256((size_t)n * 4);
     L.slots = o; o += al256((size_t)2 * G * sizeof(Slot));
     L.bar = o;   o += 256;
-    L.cand = o;  o += team ? al256((size_t)kCandMax * sizeof(Slot)) : 0;
-    L.bm = o;    o += team ? al256((size_t)kCandMax * kCandMax * 8) : 0;
+    L.cand = o;  o += team ? al256((size_t)kPubMax * sizeof(Slot)) : 0;
+    L.bm = o;    o += team ? al256((size_t)kCand * kCand * 8) : 0;
     L.bl = o;    o += team ? al256((size_t)kBlk * kBlk * 8) : 0;
     L.bp = o;    o += team ? al256((size_t)kBlk * 8) : 0;
     L.bv = o;    o += team ? al256((size_t)kBlk * 8) : 0;
@@ -305,23 +292,21 @@ __host__ __device__ inline Layout layout(int64_t m, int64_t n, int esz, int asz,
     return L;
 }
 
-// Candidates each CTA of a team of G contributes (its best rows) and the
-// candidate count padded to whole 64-row tiles: G q <= kCandMax.
+// Rows each CTA of a team of G publishes (its best): G q <= kPubMax.
 __host__ __device__ inline int cand_per_cta(int G) {
-    int q = kCandMax / G;
+    int q = kPubMax / G;
     return q > 64 ? 64 : (q < 1 ? 1 : q);
 }
-__host__ __device__ inline int cand_count(int G) { return (G * cand_per_cta(G) + 63) & ~63; }
 
 // Dynamic shared memory of the blocked pass: the candidates (row, leverage),
 // then the largest of its phases' work areas.
 __host__ __device__ constexpr size_t block_smem() {
     constexpr size_t sort = (size_t)kSortMax * 16;
-    constexpr size_t chol = (size_t)kCandMax * (kBlk + 1) * 8 + kCandMax * 8 + kBlk * 4 * 2 + 64;
-    constexpr size_t rows = (size_t)kBlk * kBlk * 8 + kBlk * 8 * 2 + (size_t)(64 + kBlk) * (kKC + 1) * 8 +
-                            (size_t)64 * (kBlk + 1) * 8 + 64 * 8 + kSortMax;
+    constexpr size_t chol = (size_t)kCand * (kBlk + 1) * 8 + (size_t)kCand * (kCand + 1) / 2 * 8;
+    constexpr size_t rows = (size_t)kBlk * kBlk * 8 + kBlk * 8 * 3 + (size_t)kSortMax * 9 +
+                            (size_t)4 * 64 * (kBlk + 1) * 8;
     constexpr size_t w = sort > chol ? (sort > rows ? sort : rows) : (chol > rows ? chol : rows);
-    return (size_t)kCandMax * 16 + w;
+    return (size_t)kCand * 16 + w;
 }
 
 // Rows are processed TPR threads per row, THREADS / TPR rows at a time, so a
@@ -395,108 +380,86 @@ __device__ __forceinline__ bool before(double va, int64_t ia, double vb, int64_t
     return va > vb || (va == vb && ia < ib);
 }
 
-// Rows rowA[0..64) (entries of INT64_MAX are zero rows) times rows
-// rowB[0..32) of X over its first `a` columns, in FP64: Yb (64 x 32, ld
-// kBlk + 1) = X_A X_B^T.  Staged through shared memory in FP64, kKC columns
-// at a time, the next chunk's loads in flight (registers) while the current
-// one is multiplied: warp w stages rows w + 16 j, lanes the columns.  Each
-// thread owns 4 x 4 outputs (rows r + 16 v, four consecutive columns) of one
-// quarter of the chunk's columns, the quarters summed at the end.  All
-// threads of the CTA call it.
+// Four consecutive columns k..k+3 of a packed row in FP64, those past column
+// a as zeros.  k is a multiple of 4 below a, so the vector loads are aligned
+// and stay inside the row (x_stride); through L2, other CTAs write X.
 template <typename S>
-__device__ void rows_dot(const S *X, int64_t ldx, int a, const int64_t *rowA, const int64_t *rowB, double *Xr,
-                         double *Xs, double *Yb) {
-    constexpr int LDK = kKC + 1, LDY = kBlk + 1, NW = kThreads / 32;
-    constexpr int KC = sizeof(S) == 8 ? kKC / 2 : kKC;     // chunk: FP64 storage keeps half in flight
-    constexpr int RA = 64 / NW, RB = kBlk / NW, KL = KC / 32;    // rows per warp, columns per lane
-    static_assert(kThreads == 512 && kKC % 32 == 0, "rows_dot layout");
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int kq = tid >> 7, t7 = tid & 127, rr = t7 & 15, cg = t7 >> 4;   // K quarter, row, column group
-    const S *pa[RA], *pb[RB];
-#pragma unroll
-    for (int j = 0; j < RA; ++j) {
-        const int64_t row = rowA[warp + NW * j];
-        pa[j] = row != INT64_MAX ? X + row * ldx : nullptr;
+__device__ __forceinline__ void load4(const S *row, int k, int a, double (&v)[4]) {
+    if constexpr (sizeof(S) == 4) {
+        const float4 x = __ldcg((const float4 *)(row + k));
+        v[0] = (double)x.x; v[1] = (double)x.y; v[2] = (double)x.z; v[3] = (double)x.w;
+    } else {
+        const double2 x = __ldcg((const double2 *)(row + k));
+        double2 y = make_double2(0.0, 0.0);
+        if (k + 2 < a) y = __ldcg((const double2 *)(row + k + 2));
+        v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
     }
+    if (k + 4 > a) {
 #pragma unroll
-    for (int j = 0; j < RB; ++j) {
-        const int64_t row = rowB[warp + NW * j];
-        pb[j] = row != INT64_MAX ? X + row * ldx : nullptr;
+        for (int e = 1; e < 4; ++e)
+            if (k + e >= a) v[e] = 0.0;
     }
-    S va[RA][KL], vb[RB][KL];                              // the next chunk, in the storage type
-    auto fetch = [&](int k0) {
+}
+
+// One warp's share of the products of 8 RT rows of X with 8 CT rows over the
+// first `a` columns, in FP64 on the matrix unit (m8n8k4): pa[r] is the row
+// 8 r + lane / 4 of the first set, pb[c] of the second, and acc[r][c] holds
+// the products of row lane / 4 of tile r with rows 2 (lane % 4) and
+// 2 (lane % 4) + 1 of tile c.  A lane's four consecutive columns (one 16-byte load
+// of FP32) feed four instructions, which permutes the columns of a 16-column
+// step alike on both sides.  Steps share, share + shares, ... are this warp's.
+// The operands go from L2 to registers: a CTA reads each row of its own set
+// once, so staging through shared memory would only add a pass.
+template <typename S, int RT, int CT>
+__device__ __forceinline__ void warp_dots(const S *const (&pa)[RT], const S *const (&pb)[CT], int a, int share,
+                                          int shares, double (&acc)[RT][CT][2]) {
+    const int k1 = 4 * (threadIdx.x & 3);
 #pragma unroll
-        for (int u = 0; u < KL; ++u) {
-            const int k = k0 + lane + 32 * u;
-            const bool in = k < a;
+    for (int r = 0; r < RT; ++r)
 #pragma unroll
-            for (int j = 0; j < RA; ++j) va[j][u] = in && pa[j] ? __ldcg(pa[j] + k) : S(0);
+        for (int c = 0; c < CT; ++c) acc[r][c][0] = acc[r][c][1] = 0.0;
+#pragma unroll 2
+    for (int k0 = 16 * share; k0 < a; k0 += 16 * shares) {
+        const int k = k0 + k1;
+        double x[RT][4], y[CT][4];
 #pragma unroll
-            for (int j = 0; j < RB; ++j) vb[j][u] = in && pb[j] ? __ldcg(pb[j] + k) : S(0);
+        for (int r = 0; r < RT; ++r)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[r][e] = 0.0;
+#pragma unroll
+        for (int c = 0; c < CT; ++c)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[c][e] = 0.0;
+        if (k < a) {
+#pragma unroll
+            for (int r = 0; r < RT; ++r) load4(pa[r], k, a, x[r]);
+#pragma unroll
+            for (int c = 0; c < CT; ++c) load4(pb[c], k, a, y[c]);
         }
-    };
-    auto stage = [&]() {
+        __syncwarp();
 #pragma unroll
-        for (int u = 0; u < KL; ++u) {
+        for (int e = 0; e < 4; ++e)
 #pragma unroll
-            for (int j = 0; j < RA; ++j) Xr[(warp + NW * j) * LDK + lane + 32 * u] = (double)va[j][u];
+            for (int r = 0; r < RT; ++r)
 #pragma unroll
-            for (int j = 0; j < RB; ++j) Xs[(warp + NW * j) * LDK + lane + 32 * u] = (double)vb[j][u];
-        }
-    };
-    double acc[4][4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[v][u] = 0.0;
-    fetch(0);
-    stage();
-    __syncthreads();
-    for (int k0 = 0; k0 < a; k0 += KC) {
-        const int kc = (a - k0) < KC ? (a - k0) : KC;
-        const bool more = k0 + KC < a;
-        if (more) fetch(k0 + KC);                          // in flight during the products
-        for (int k = kq; k < kc; k += 4) {
-            double x[4], y[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) x[v] = Xr[(rr + 16 * v) * LDK + k];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) y[u] = Xs[(4 * cg + u) * LDK + k];
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-#pragma unroll
-                for (int u = 0; u < 4; ++u) acc[v][u] = fma(x[v], y[u], acc[v][u]);
-        }
-        __syncthreads();
-        if (more) {
-            stage();
-            __syncthreads();
-        }
-    }
-    // the four quarters, summed in a fixed order
-    for (int q4 = 0; q4 < 4; ++q4) {
-        if (kq == q4)
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    double *y = Yb + (rr + 16 * v) * LDY + 4 * cg + u;
-                    *y = q4 ? *y + acc[v][u] : acc[v][u];
-                }
-        __syncthreads();
+                for (int c = 0; c < CT; ++c)
+                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                                 : "+d"(acc[r][c][0]), "+d"(acc[r][c][1])
+                                 : "d"(x[r][e]), "d"(y[c][e]));
     }
 }
 
 // This CTA's best q rows by leverage ("before" order: bitonic sort of its
-// nrow <= kSortMax rows in `work`), written to out[0..q).
-__device__ void publish_best(const double *lev, int64_t r0, int nrow, int q, Slot *out, unsigned char *work) {
+// nrow <= kSortMax rows in `work`), written to out[0..q).  own[i] is the leverage
+// of row r0 + i.
+__device__ void publish_best(const double *own, int64_t r0, int nrow, int q, Slot *out, unsigned char *work) {
     double *kv = (double *)work;
     int64_t *ki = (int64_t *)(work + (size_t)kSortMax * 8);
     const int tid = threadIdx.x;
     int np2 = 64;
     while (np2 < nrow || np2 < q) np2 <<= 1;
     for (int i = tid; i < np2; i += kThreads) {
-        kv[i] = i < nrow ? lev[r0 + i] : -1e300;
+        kv[i] = i < nrow ? own[i] : -1e300;
         ki[i] = i < nrow ? r0 + i : INT64_MAX;
     }
     __syncthreads();
@@ -523,14 +486,58 @@ __device__ void publish_best(const double *lev, int64_t r0, int nrow, int q, Slo
     __syncthreads();
 }
 
+// The same for q <= 16 of at most 256 rows, by one warp: eight rows a lane,
+// the best taken q times by 32-bit reductions over the leverage's high word,
+// low word and row (0.3 us for two of 64 rows, the sort 9 us).  `first` gets
+// the best row (row 0 with the lowest value when no leverage is a number).
+constexpr int kFewRows = 256, kFewBest = 16;
+__device__ void publish_few(const double *own, int64_t r0, int nrow, int q, Slot *out, Slot *first) {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int E = kFewRows / 32;
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    unsigned long long key[E];                             // ordered bits; 0: none
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int i = lane + 32 * e;
+        const double v = i < nrow ? own[i] : -1e300;
+        const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+        key[e] = v > -1e300 ? ((long long)b < 0 ? ~b : b | (1ull << 63)) : 0ull;
+    }
+    for (int r = 0; r < q; ++r) {
+        unsigned long long k = 0;
+        int at = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (key[e] > k) { k = key[e]; at = e; }        // first of equals: the smaller row
+        const unsigned hi = (unsigned)(k >> 32), mh = __reduce_max_sync(FULL, hi);
+        const unsigned lo = hi == mh ? (unsigned)k : 0u, ml = __reduce_max_sync(FULL, lo);
+        const unsigned row = k && hi == mh && lo == ml ? (unsigned)(lane + 32 * at) : ~0u;
+        const unsigned mr = __reduce_min_sync(FULL, row);
+        const unsigned long long best = ((unsigned long long)mh << 32) | ml;
+        const long long b = (long long)(best >> 63 ? best & ~(1ull << 63) : ~best);
+        const bool any = mr != ~0u;
+        if (lane == 0) {
+            const double v = any ? __longlong_as_double(b) : -1e300;
+            out[r] = {v, any ? r0 + (int64_t)mr : INT64_MAX};
+            if (r == 0) *first = {v, any ? r0 + (int64_t)mr : 0};
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            if (row == mr && at == e) key[e] = 0ull;
+    }
+}
+
 // Blocked pass of the team path (real types).  The missing columns are the
 // pivoted Cholesky factor of the projector P = I - X X^T onto the complement
 // of the packed columns X, pivot = the largest leverage (P's remaining
 // diagonal), exactly as the per-column loop builds them: column k =
 // P_k e_p / sqrt(lev_p).  A block of up to kBlk columns is built
-// speculatively on a candidate set C (every CTA's best rows), then checked:
+// speculatively on a candidate set C (the kCand best of every CTA's best
+// rows), then checked:
 //   P2  M = P[C, C] (diagonal: the tracked leverages; off-diagonal
-//       -X_i . X_j in FP64), shared out over the team in 64 x 32 tiles;
+//       -X_i . X_j in FP64), its lower triangle shared out over the team in
+//       16 x 16 tiles, the columns over the warps of a CTA;
 //   P3  CTA 0: the pivoted Cholesky of M, pivot = the best remaining
 //       leverage in C, until kBlk columns, the missing columns run out, or
 //       the best is below 1/2 (the per-column loop then takes that column,
@@ -541,11 +548,12 @@ __device__ void publish_best(const double *lev, int64_t r0, int nrow, int q, Slo
 //       step by step: a row whose leverage at step s ranks before the
 //       pivot's would have been step s's pivot, so the block keeps only the
 //       steps before the first such s (step 0 always stands: the best row of
-//       every CTA is in C);
-//   P5  the leverages lowered by |N_i|^2 over the kept steps, the slots and
-//       the next block's candidates published.
+//       all is in C); the slots and the next block's candidates are
+//       published as if all steps stood;
+//   P5  when they do not: the leverages lowered by |N_i|^2 over the kept
+//       steps, slots and candidates published again.
 // The kept pivots and columns are, in exact arithmetic, the per-column
-// loop's, at four team barriers per block instead of one per column.
+// loop's, at three team barriers per block instead of one per column.
 // `fresh`: the candidate lists match the current leverages (else P1
 // publishes them first).  Returns the columns completed (0: the per-column
 // loop takes the next one), or -1 when a barrier wait ran out; `slow` is set
@@ -557,10 +565,9 @@ __device__ int block_pass(const Params &p, const Layout &L, unsigned char *base,
                           Slot *s_red) {
     using T = Tr<S>;
     constexpr unsigned FULL = 0xffffffffu;
-    constexpr int LDK = kKC + 1, LDY = kBlk + 1;
     const int64_t n = p.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int q = cand_per_cta(G), nc = cand_count(G), nreal = G * q;
+    const int q = cand_per_cta(G), npub = G * q, nc = npub < kCand ? npub : kCand;
     Slot *cand = (Slot *)(base + L.cand);
     double *bm = (double *)(base + L.bm);
     double *bl = (double *)(base + L.bl);
@@ -568,127 +575,227 @@ __device__ int block_pass(const Params &p, const Layout &L, unsigned char *base,
     double *bpv = (double *)(base + L.bv);
     int *bmeta = (int *)(base + L.bmeta);
     int64_t *cidx = (int64_t *)smem;                       // candidates: row, leverage
-    double *cval = (double *)(smem + kCandMax * 8);
-    unsigned char *work = smem + kCandMax * 16;
+    double *cval = (double *)(smem + kCand * 8);
+    unsigned char *work = smem + kCand * 16;
     __shared__ int s_nmiss, s_fail;
     const int nrow = (int)(r1 - r0);
     slow = false;
 
     if (!fresh) {                                          // P1
-        publish_best(lev, r0, nrow, q, cand + (size_t)g * q, work);
+        __shared__ Slot s_first;
+        if (q <= kFewBest && nrow <= kFewRows) publish_few(lev + r0, r0, nrow, q, cand + (size_t)g * q, &s_first);
+        else publish_best(lev + r0, r0, nrow, q, cand + (size_t)g * q, work);
         if (!team_sync(bar, G)) return -1;
     }
     fresh = false;
     // P2
-    for (int i = tid; i < nc; i += kThreads) {
-        cidx[i] = i < nreal ? __ldcg(&cand[i].idx) : INT64_MAX;
-        cval[i] = i < nreal ? __ldcg(&cand[i].val) : -1e300;
+    if (tid < kCand) {
+        cidx[tid] = tid < npub ? __ldcg(&cand[tid].idx) : INT64_MAX;
+        cval[tid] = tid < npub ? __ldcg(&cand[tid].val) : -1e300;
+    }
+    if (npub > kCand) {
+        // The kCand best of the published rows, by their ranks: keys of the
+        // leverage to 2^-44 and the place in the list, two threads a row.
+        // (Any set will do that holds the best row: P4 checks the others.)
+        unsigned long long *key = (unsigned long long *)work;
+        const int t = tid >> 1, h = tid & 1;
+        Slot mine = {-1e300, INT64_MAX};
+        if (t < npub) mine = {__ldcg(&cand[t].val), __ldcg(&cand[t].idx)};
+        const bool real = mine.idx != INT64_MAX && mine.val > 0.0;
+        const unsigned long long kt =
+            (real ? (unsigned long long)__double_as_longlong(mine.val) & ~255ull : 0ull) | (unsigned)(255 - t);
+        if (h == 0) key[t] = kt;
+        __syncthreads();
+        int rank = 0;
+        const ulonglong2 *kp = (const ulonglong2 *)key + 64 * h;
+#pragma unroll 8
+        for (int u = 0; u < 64; ++u) {
+            const ulonglong2 k2 = kp[u];
+            rank += (k2.x > kt) + (k2.y > kt);
+        }
+        rank += __shfl_xor_sync(FULL, rank, 1);
+        if (h == 0 && rank < kCand) {
+            cidx[rank] = mine.idx;
+            cval[rank] = mine.val;
+        }
     }
     __syncthreads();
     {
-        double *Xr = (double *)work, *Xs = Xr + 64 * LDK, *Yb = Xs + kBlk * LDK;
-        const int tcol = nc / kBlk, tiles = (nc / 64) * tcol;
+        constexpr int LDP = 17;
+        double *part = (double *)work;                     // [warp][16][16] (ld LDP)
+        const int nt = (nc + 15) / 16, tiles = nt * (nt + 1) / 2;
         for (int tt = g; tt < tiles; tt += G) {
-            const int i0 = 64 * (tt / tcol), j0 = kBlk * (tt % tcol);
-            rows_dot<S>(X, ldx, a, cidx + i0, cidx + j0, Xr, Xs, Yb);
-            for (int e = tid; e < 64 * kBlk; e += kThreads) {
-                const int r = e / kBlk, cc = e - r * kBlk, ia = i0 + r, jb = j0 + cc;
+            int ti = (int)((sqrtf(8.f * (float)tt + 1.f) - 1.f) * 0.5f);
+            while (ti * (ti + 1) / 2 > tt) --ti;
+            while ((ti + 1) * (ti + 2) / 2 <= tt) ++ti;
+            const int i0 = 16 * ti, j0 = 16 * (tt - ti * (ti + 1) / 2);
+            // padding and absent candidates read row 0; their products are not used
+            const S *pa[2], *pb[2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int64_t ra = cidx[i0 + 8 * r + (lane >> 2)], rb = cidx[j0 + 8 * r + (lane >> 2)];
+                pa[r] = X + (ra != INT64_MAX ? ra : 0) * ldx;
+                pb[r] = X + (rb != INT64_MAX ? rb : 0) * ldx;
+            }
+            double acc[2][2][2];
+            warp_dots<S, 2, 2>(pa, pb, a, warp, kWarps, acc);
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int cc = 0; cc < 2; ++cc)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        part[(warp * 16 + 8 * r + (lane >> 2)) * LDP + 8 * cc + 2 * (lane & 3) + e] = acc[r][cc][e];
+            __syncthreads();
+            if (tid < 256) {
+                const int r = tid >> 4, cc = tid & 15, ia = i0 + r, jb = j0 + cc;
+                double y = 0.0;
+#pragma unroll
+                for (int w = 0; w < kWarps; ++w) y += part[(w * 16 + r) * LDP + cc];
                 const bool ok = cidx[ia] != INT64_MAX && cidx[jb] != INT64_MAX;
-                bm[(size_t)ia * nc + jb] = ia == jb ? (ok ? cval[ia] : 0.0) : (ok ? -Yb[r * LDY + cc] : 0.0);
+                const double v = ok ? (ia == jb ? cval[ia] : -y) : 0.0;
+                bm[ia * kCand + jb] = v;
             }
             __syncthreads();
         }
     }
     if (!team_sync(bar, G)) return -1;
 
-    // P3: CTA 0, the pivoted Cholesky of M
+    // P3: CTA 0, the pivoted Cholesky of M.  A serial chain of up to kBlk
+    // steps, so the step is kept short: four threads a candidate with its row
+    // of the factor in registers (every fourth step each), the pivot's row a
+    // broadcast from shared memory, M's lower triangle staged there (the L2
+    // latency of its row would be in every step), the best candidate by 32-bit
+    // warp reductions over the leverage's high word, low word and row, and
+    // one barrier.  One thread a candidate with the factor in shared memory
+    // and M behind L2 took 59 us a block (8192 rows, 256 candidates); this form takes 22.
+    // Two threads a candidate: 31 us, the factor's row and its select twice as
+    // long and 1 / sqrt in the chain.
     if (g == 0) {
         constexpr int LDL = kBlk + 1;                      // odd: candidates' rows in different banks
-        double *Lc = (double *)work;                       // L[t][s], nc x kBlk (ld LDL)
-        double *d = Lc + (size_t)kCandMax * LDL;           // remaining leverage of candidate t
-        int *pa = (int *)(d + kCandMax);                   // candidate of pivot s
-        int *cols = pa + kBlk;                             // U column of pivot s
+        double *Lc = (double *)work;                       // L[t][s], kCand x kBlk (ld LDL)
+        double *Mp = Lc + (size_t)kCand * LDL;             // lower triangle of M by rows
+        __shared__ int s_pa[kBlk], s_cols[kBlk];           // candidate, U column of pivot s
+        __shared__ double s_pv[kBlk];                      // leverage of pivot s
+        __shared__ uint4 s_best[2][kWarps];                // leverage high, low, row, candidate
+        constexpr int TP = 4, LE = kBlk / TP;              // threads a candidate, steps a thread
+        const int t = tid / TP, h = tid % TP;
+        const bool real = t < nc && cidx[t] != INT64_MAX;
         for (int i = tid; i < nc * LDL; i += kThreads) Lc[i] = 0.0;
-        for (int i = tid; i < nc; i += kThreads) d[i] = cidx[i] != INT64_MAX ? cval[i] : -1e300;
-        if (tid == 0) {
-            int k = 0;
-            for (int64_t cc = c; cc < n && k < kBlk; ++cc)
-                if (!keep[cc]) cols[k++] = (int)cc;
-            s_nmiss = k;
+        constexpr int RB = 4, CB = kCand / 32;             // rows of M in flight a warp, words a lane and row
+        for (int i0 = warp; i0 < nc; i0 += RB * kWarps) {
+            double v[RB][CB];
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+#pragma unroll
+                for (int k = 0; k < CB; ++k) {
+                    const int i = i0 + kWarps * r, kk = lane + 32 * k;
+                    v[r][k] = i < nc && kk <= i ? __ldcg(bm + i * kCand + kk) : 0.0;
+                }
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+#pragma unroll
+                for (int k = 0; k < CB; ++k) {
+                    const int i = i0 + kWarps * r, kk = lane + 32 * k;
+                    if (i < nc && kk <= i) Mp[i * (i + 1) / 2 + kk] = v[r][k];
+                }
         }
+        if (warp == kWarps - 1) {
+            int k = 0;
+            for (int64_t c0 = c; c0 < n && k < kBlk; c0 += 32) {
+                const bool miss = c0 + lane < n && !keep[c0 + lane];
+                const unsigned bm_ = __ballot_sync(FULL, miss);
+                const int at = k + __popc(bm_ & ((1u << lane) - 1u));
+                if (miss && at < kBlk) s_cols[at] = (int)(c0 + lane);
+                k += __popc(bm_);
+            }
+            if (lane == 0) s_nmiss = k < kBlk ? k : kBlk;
+        }
+        double d = real ? cval[t] : 0.0, l[LE];            // remaining leverage; steps TP j + h
+#pragma unroll
+        for (int j = 0; j < LE; ++j) l[j] = 0.0;
+        bool open = real;                                  // a candidate that is no pivot yet
+        const unsigned row = real ? (unsigned)cidx[t] : ~0u;
+        // the lane with the best of the warp's (leverage bits, row) keys, "before"
+        // order, or -1; one reduction unless high words tie
+        auto best_lane = [&](unsigned hi, unsigned lo, unsigned rw, bool in) -> int {
+            const unsigned mh = __reduce_max_sync(FULL, in ? hi : 0u);
+            unsigned b = __ballot_sync(FULL, in && hi == mh);
+            if (b & (b - 1u)) {
+                const bool e0 = in && hi == mh;
+                const unsigned ml = __reduce_max_sync(FULL, e0 ? lo : 0u);
+                const unsigned mr = __reduce_min_sync(FULL, e0 && lo == ml ? rw : ~0u);
+                b = __ballot_sync(FULL, e0 && lo == ml && rw == mr);
+            }
+            return __ffs(b) - 1;
+        };
+        // this warp's best open candidate (none above zero: key 0)
+        auto warp_best = [&](int buf) {
+            const int dh = __double2hiint(d);
+            const unsigned hi = dh > 0 ? (unsigned)dh : 0u, lo = dh > 0 ? (unsigned)__double2loint(d) : 0u;
+            const int w = best_lane(hi, lo, row, open && h == 0);
+            if (w < 0 ? lane == 0 : lane == w) s_best[buf][warp] = make_uint4(hi, lo, row, w < 0 ? ~0u : (unsigned)t);
+        };
+        warp_best(0);
         __syncthreads();
         const int nmax = s_nmiss;
         int ns = 0, stop_slow = 0;
-        // the best remaining candidate: each warp's best of its 32 (after the
-        // step's update), then the warps' bests in shared memory
-        __shared__ double s_wv[kWarps];
-        __shared__ int64_t s_wi[kWarps];
-        __shared__ int s_wa[kWarps];
-        auto warp_best = [&]() {
-            double bv = -1e300;
-            int64_t bi = INT64_MAX;
-            int ba = -1;
-            for (int t = tid; t < nc; t += kThreads)
-                if (d[t] > -1e299 && before(d[t], cidx[t], bv, bi)) { bv = d[t]; bi = cidx[t]; ba = t; }
-            for (int o = 16; o; o >>= 1) {
-                const double ov = __shfl_xor_sync(FULL, bv, o);
-                const int64_t oi = __shfl_xor_sync(FULL, bi, o);
-                const int oa = __shfl_xor_sync(FULL, ba, o);
-                if (before(ov, oi, bv, bi)) { bv = ov; bi = oi; ba = oa; }
-            }
-            if (lane == 0) { s_wv[warp] = bv; s_wi[warp] = bi; s_wa[warp] = ba; }
-        };
-        auto cta_best = [&](double &bv, int &ba) {
-            bv = s_wv[0];
-            int64_t bi = s_wi[0];
-            ba = s_wa[0];
-            for (int w = 1; w < kWarps; ++w)
-                if (before(s_wv[w], s_wi[w], bv, bi)) { bv = s_wv[w]; bi = s_wi[w]; ba = s_wa[w]; }
-        };
-        warp_best();
-        __syncthreads();
         for (; ns < nmax; ++ns) {
-            double bv;
-            int pb;
-            cta_best(bv, pb);
-            if (pb < 0 || bv < 0.5) {
+            const uint4 mine = s_best[ns & 1][lane & (kWarps - 1)];
+            const int w = best_lane(mine.x, mine.y, mine.z, lane < kWarps && (int)mine.w >= 0);
+            const uint4 top = s_best[ns & 1][w < 0 ? 0 : w];
+            const int pb = w < 0 ? -1 : (int)top.w;
+            if (pb < 0 || top.x < 0x3fe00000u) {           // none left, or its leverage below 1/2
                 stop_slow = pb >= 0;
                 break;
             }
-            const double lpp = sqrt(bv);
-            for (int t = tid; t < nc; t += kThreads) {
-                if (t == pb) {
-                    Lc[t * LDL + ns] = lpp;
-                    d[t] = -1e300;                         // pivoted
-                } else if (d[t] > -1e299) {
-                    const double mt = __ldcg(bm + (size_t)pb * nc + t);   // row pb of M (symmetric), in flight
-                    double acc0 = 0.0, acc1 = 0.0;
-                    int u = 0;
-                    for (; u + 1 < ns; u += 2) {
-                        acc0 = fma(Lc[t * LDL + u], Lc[pb * LDL + u], acc0);
-                        acc1 = fma(Lc[t * LDL + u + 1], Lc[pb * LDL + u + 1], acc1);
-                    }
-                    if (u < ns) acc0 = fma(Lc[t * LDL + u], Lc[pb * LDL + u], acc0);
-                    const double l = (mt - (acc0 + acc1)) / lpp;
-                    Lc[t * LDL + ns] = l;
-                    d[t] -= l * l;
+            const double bv = __hiloint2double((int)top.x, (int)top.y);
+            const double mt = open ? (t <= pb ? Mp[pb * (pb + 1) / 2 + t] : Mp[t * (t + 1) / 2 + pb]) : 0.0;
+            // 1 / sqrt(bv), bv in [1/2, 2): FP32 estimate and one third-order
+            // step (the residual e is 1e-7), beside the product's chain
+            const double r0_ = (double)rsqrtf((float)bv);
+            const double e_ = fma(-bv * r0_, r0_, 1.0);
+            const double rp = fma(r0_ * e_, fma(0.375, e_, 0.5), r0_);
+            const double *lp = Lc + pb * LDL + h;
+            double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll
+            for (int j = 0; j < LE; j += 4)
+                if (TP * j < ns) {
+                    s0 = fma(l[j], lp[TP * j], s0);
+                    s1 = fma(l[j + 1], lp[TP * (j + 1)], s1);
+                    s2 = fma(l[j + 2], lp[TP * (j + 2)], s2);
+                    s3 = fma(l[j + 3], lp[TP * (j + 3)], s3);
                 }
+            double sum = (s0 + s1) + (s2 + s3);
+            sum += __shfl_xor_sync(FULL, sum, 1);
+            sum += __shfl_xor_sync(FULL, sum, 2);
+            const double v = (mt - sum) * rp;
+            open = open && t != pb;
+            if (open) {
+                d = fma(-v, v, d);
+                if (h == 0) Lc[t * LDL + ns] = v;
             }
+#pragma unroll
+            for (int j = 0; j < LE; ++j) {
+                int at = TP * j + h;
+                asm("" : "+r"(at));                        // a select, not an indexed store to local memory
+                l[j] = ns == at ? v : l[j];
+            }
+            warp_best((ns + 1) & 1);
             if (tid == 0) {
-                pa[ns] = pb;
-                bpv[ns] = bv;
+                s_pa[ns] = pb;
+                s_pv[ns] = bv;
             }
-            __syncthreads();                               // everyone has read this step's s_w*
-            warp_best();                                   // each thread's candidates are its own: no barrier before
-            __syncthreads();
+            __syncthreads();                               // the factor's column and the warps' bests
         }
         for (int i = tid; i < ns * kBlk; i += kThreads) {
-            const int s2 = i / kBlk, t = i - s2 * kBlk;
-            bl[i] = t <= s2 ? Lc[pa[s2] * LDL + t] : 0.0;
+            const int r = i / kBlk, k = i - r * kBlk;
+            bl[i] = k < r ? Lc[s_pa[r] * LDL + k] : (k == r ? sqrt(s_pv[r]) : 0.0);
         }
         for (int i = tid; i < ns; i += kThreads) {
-            bp[i] = cidx[pa[i]];
-            cmap[a + i] = cols[i];
+            bp[i] = cidx[s_pa[i]];
+            bpv[i] = s_pv[i];
+            cmap[a + i] = s_cols[i];
         }
         if (tid == 0) {
             bmeta[0] = ns;
@@ -704,79 +811,158 @@ __device__ int block_pass(const Params &p, const Layout &L, unsigned char *base,
         return 0;
     }
 
-    // P4: this CTA's rows of the block, 64 at a time, and the check
-    double *Ls = (double *)work;                           // kBlk x kBlk
-    int64_t *Sv = (int64_t *)(Ls + kBlk * kBlk);           // pivot rows
-    double *Pv = (double *)(Sv + kBlk);                    // pivot leverages
-    double *Xr = Pv + kBlk;                                // 64 x kKC (ld LDK)
-    double *Xs = Xr + 64 * LDK;                            // kBlk x kKC (ld LDK)
-    double *Yb = Xs + kBlk * LDK;                          // 64 x kBlk (ld LDY)
-    int64_t *rowsA = (int64_t *)(Yb + 64 * LDY);           // this chunk's rows
-    unsigned char *incand = (unsigned char *)(rowsA + 64); // own rows in C
-    for (int i = tid; i < ns * kBlk; i += kThreads) Ls[i] = __ldcg(bl + i);
+    // P4: this CTA's rows of the block, 64 at a time, and the check.  Warp w
+    // forms the products of 16 rows with the pivots over a quarter of the
+    // columns; then eight threads a row run the forward substitution, four
+    // columns of the block each, the step's value a shuffle, and check the
+    // leverages afterwards.
+    constexpr int LDY = kBlk + 1;
+    double *Lt = (double *)work;                           // kBlk x kBlk, Lt[s][t] = L[t][s] below the diagonal
+    double *Li = Lt + kBlk * kBlk;                         // 1 / L[s][s]
+    double *Pv = Li + kBlk;                                // pivot leverages
+    int64_t *Sv = (int64_t *)(Pv + kBlk);                  // pivot rows
+    double *lvs = (double *)(Sv + kBlk);                   // own rows' leverages after the whole block
+    unsigned char *incand = (unsigned char *)(lvs + kSortMax);   // own rows in C
+    double *part = (double *)(incand + kSortMax);          // [quarter][64][kBlk] (ld LDY); later the sort's area
+    for (int i = tid; i < kBlk * kBlk; i += kThreads) {
+        const int r = i / kBlk, k = i - r * kBlk;
+        Lt[k * kBlk + r] = r < ns && k < r ? __ldcg(bl + i) : 0.0;
+    }
     for (int i = tid; i < kBlk; i += kThreads) {
         Sv[i] = i < ns ? __ldcg(bp + i) : INT64_MAX;
         Pv[i] = i < ns ? __ldcg(bpv + i) : 0.0;
+        Li[i] = i < ns ? 1.0 / __ldcg(bl + i * kBlk + i) : 0.0;
     }
     for (int i = tid; i < nrow; i += kThreads) incand[i] = 0;
     if (tid == 0) s_fail = ns;
     __syncthreads();
     for (int i = tid; i < nc; i += kThreads)
         if (cidx[i] >= r0 && cidx[i] < r1) incand[cidx[i] - r0] = 1;
-    __syncthreads();
     int fail = ns;
     for (int64_t rc = r0; rc < r1; rc += 64) {
         const int nr = (int)((r1 - rc) < 64 ? (r1 - rc) : 64);
-        if (tid < 64) rowsA[tid] = tid < nr ? rc + tid : INT64_MAX;
-        __syncthreads();
-        rows_dot<S>(X, ldx, a, rowsA, Sv, Xr, Xs, Yb);
-        if (tid < nr) {
-            const int64_t i = rc + tid;
-            double *yr = Yb + tid * LDY;
-            const bool check = !incand[i - r0];
-            double lv = lev[i];
-            for (int s2 = 0; s2 < ns; ++s2) {
-                if (check && s2 < fail && before(lv, i, Pv[s2], Sv[s2])) fail = s2;
-                double y0 = (i == Sv[s2] ? 1.0 : 0.0) - yr[s2], y1 = 0.0;
-                int t = 0;
-                for (; t + 1 < s2; t += 2) {
-                    y0 = fma(-yr[t], Ls[s2 * kBlk + t], y0);
-                    y1 = fma(-yr[t + 1], Ls[s2 * kBlk + t + 1], y1);
+        const int rg = warp & 3, kq = warp >> 2;
+        if (16 * rg < nr) {
+            const S *pa[2], *pb[4];                        // rows past the last, absent pivots: not used
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int i = 16 * rg + 8 * r + (lane >> 2);
+                pa[r] = X + (rc + (i < nr ? i : 0)) * ldx;
+            }
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) {
+                const int64_t i = Sv[8 * cc + (lane >> 2)];
+                pb[cc] = X + (i != INT64_MAX ? i : r0) * ldx;
+            }
+            double acc[2][4][2];
+            warp_dots<S, 2, 4>(pa, pb, a, kq, 4, acc);
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        part[(kq * 64 + 16 * rg + 8 * r + (lane >> 2)) * LDY + 8 * cc + 2 * (lane & 3) + e] =
+                            acc[r][cc][e];
+        }
+        __syncthreads();                                   // the products; incand in the first pass
+        {
+            const int rl = tid >> 3, sub = tid & 7;
+            const bool own = rl < nr;
+            const int64_t i = rc + (own ? rl : 0);
+            const int il = (int)(i - r0);
+            const bool check = own && !incand[il];
+            double y[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const double *yp = part + (own ? rl : 0) * LDY + 4 * sub + e;
+                y[e] = (i == Sv[4 * sub + e] ? 1.0 : 0.0) -
+                       ((yp[0] + yp[64 * LDY]) + (yp[128 * LDY] + yp[192 * LDY]));
+            }
+            for (int s4 = 0; s4 < ns; s4 += 4) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {              // steps past ns: Li and Lt are zero
+                    const double ys = __shfl_sync(FULL, y[e] * Li[s4 + e], s4 >> 2, 8);
+                    const double2 *lt = (const double2 *)(Lt + (s4 + e) * kBlk + 4 * sub);
+                    const double2 l0 = lt[0], l1 = lt[1];
+                    y[0] = fma(-ys, l0.x, y[0]);
+                    y[1] = fma(-ys, l0.y, y[1]);
+                    y[2] = fma(-ys, l1.x, y[2]);
+                    y[3] = fma(-ys, l1.y, y[3]);
+                    if (sub == s4 >> 2) y[e] = ys;
                 }
-                if (t < s2) y0 = fma(-yr[t], Ls[s2 * kBlk + t], y0);
-                const double y = (y0 + y1) / Ls[s2 * kBlk + s2];
-                yr[s2] = y;
-                const S ys = (S)y;                         // the stored value, as the leverage sees it
-                X[i * ldx + a + s2] = ys;
-                lv -= (double)ys * (double)ys;
+            }
+            // the leverage before each of this thread's four steps: the squares
+            // of the stored values, summed over the threads before it
+            double sq[4], pre = 0.0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const double st = 4 * sub + e < ns ? (double)(S)y[e] : 0.0;
+                sq[e] = st * st;
+                pre += sq[e];
+            }
+            double run = pre;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const double up = __shfl_up_sync(FULL, run, o, 8);
+                if (sub >= o) run += up;
+            }
+            double lv = lev[i] - (run - pre);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int s2 = 4 * sub + e;
+                if (check && s2 < fail && before(lv, i, Pv[s2], Sv[s2])) fail = s2;
+                lv -= sq[e];
+            }
+            if (own) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (4 * sub + e < ns) X[i * ldx + a + 4 * sub + e] = (S)y[e];
+                if (sub == 7) lvs[il] = lv;
             }
         }
         __syncthreads();
     }
     if (fail < ns) atomicMin(&s_fail, fail);
     __syncthreads();
+    // P5, as if every step of the block stands (the usual case): the slots
+    // and the next block's candidates from the new leverages, before the
+    // team agrees on the steps kept, so that one barrier serves both.
+    auto publish = [&](const double *own) {
+        if (q <= kFewBest && nrow <= kFewRows) {
+            publish_few(own, r0, nrow, q, cand + (size_t)g * q, slots + g);
+            return;
+        }
+        double best = -1e300;
+        int64_t bidx = 0;
+        for (int i = tid; i < nrow; i += kThreads)
+            if (own[i] > best) { best = own[i]; bidx = r0 + i; }
+        const Slot sb = cta_argmax(best, bidx, s_red);
+        if (tid == 0) slots[g] = sb;
+        publish_best(own, r0, nrow, q, cand + (size_t)g * q, (unsigned char *)part);
+    };
+    publish(lvs);
     if (tid == 0 && s_fail < ns) atomicMin(bmeta + 2, s_fail);
     if (!team_sync(bar, G)) return -1;
     const int kept = __ldcg(bmeta + 2);
-
-    // P5: leverages over the kept steps, slots, the next candidates
-    double best = -1e300;
-    int64_t bidx = 0;
-    for (int64_t i = r0 + tid; i < r1; i += kThreads) {
-        double lv = lev[i];
-        const S *xi = X + i * ldx + a;
+    if (kept == ns) {
+        for (int i = tid; i < nrow; i += kThreads) lev[r0 + i] = lvs[i];
+        __syncthreads();
+    } else {
+        for (int64_t i = r0 + tid; i < r1; i += kThreads) {
+            double lv = lev[i];
+            const S *xi = X + i * ldx + a;
 #pragma unroll 8
-        for (int s2 = 0; s2 < kept; ++s2) {
-            const double x = (double)__ldcg(xi + s2);
-            lv -= x * x;
+            for (int s2 = 0; s2 < kept; ++s2) {
+                const double x = (double)__ldcg(xi + s2);
+                lv -= x * x;
+            }
+            lev[i] = lv;
         }
-        lev[i] = lv;
-        if (lv > best) { best = lv; bidx = i; }
+        __syncthreads();
+        publish(lev + r0);
+        if (!team_sync(bar, G)) return -1;
     }
-    const Slot sb = cta_argmax(best, bidx, s_red);
-    if (tid == 0) slots[g] = sb;
-    publish_best(lev, r0, nrow, q, cand + (size_t)g * q, work);
-    if (!team_sync(bar, G)) return -1;
     fresh = true;
     slow = kept == ns && __ldcg(bmeta + 1) != 0;
     return kept;
