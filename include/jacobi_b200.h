@@ -459,6 +459,23 @@ JB_API int jb_prepare(const void *x, int32_t dtype, void *out, int32_t widen, in
                       int32_t *keys, int32_t *status, int64_t batch, int32_t rows, int32_t cols, void *stream);
 JB_API int jb_check_finite(const void *x, int32_t dtype, int64_t count, int32_t *flag, void *stream);
 
+/* One round of the block Jacobi (svdbench/standalone/solvers.py:43-53) on a
+ * batch of float64 matrices, kept transposed: Wt (batch, n, m) and Vt (batch,
+ * n, n), row j = column j.  cols (pairs, c): the columns of each pair of groups,
+ * disjoint between pairs, each in [0, n).  Every pair's columns are
+ * orthogonalised by one-sided Jacobi (tol <= 0: 10 eps; at most max_sweeps
+ * sweeps) and sorted by descending norm in place, V's rotated alike.  status,
+ * sweeps: batch * pairs words, JB_ST_OK, JB_ST_NOT_CONVERGED or
+ * JB_ST_NONFINITE_IN (the pair is then left as it was).  m >= n, m <= 128, c <=
+ * 32.  jb_worst_correlation_f64: *worst = the largest |w_p . w_q| / (||w_p||
+ * ||w_q||) over the pairs of columns with ||w||^2 > live^2 max ||w||^2 of every
+ * matrix (:54-58); norms2: batch * n doubles of scratch. */
+JB_API int jb_pair_round_f64(double *Wt, double *Vt, const int32_t *cols, int64_t batch, int32_t m, int32_t n,
+                             int32_t pairs, int32_t c, double tol, int32_t max_sweeps, int32_t *status,
+                             int32_t *sweeps, void *stream);
+JB_API int jb_worst_correlation_f64(const double *Wt, int64_t batch, int32_t m, int32_t n, double live,
+                                    double *norms2, double *worst, void *stream);
+
 /* Measurement kernel for the rooflines of the FP32/FP64 Jacobi kernels (no
  * counterpart in the reference): `blocks` CTAs of 256 threads, each thread
  * 16 independent fused multiply-add chains of `iters` steps; mode 0 FP32

@@ -20,7 +20,10 @@ the other (the reference) or all at once (here) gives the same result:
     the same rotations and sweeps in exact arithmetic, far less work;
   * the rotations W[:, cols] V_ij and V[:, cols] V_ij and the convergence
     check's Gram W^H W are library GEMMs in the input dtype, as the
-    reference's matmuls are.
+    reference's matmuls are;
+  * float64 pairs of at most 128 rows and 32 columns do all of a round in one
+    launch (jb_pair_round_f64) and the convergence check in two
+    (jb_worst_correlation_f64).
 
 After a sweep the largest correlation |g_pq| / sqrt(g_pp g_qq) between live
 columns decides convergence (tol defaults to 40 eps); then the columns are
@@ -78,13 +81,16 @@ def finish_columns(w, s, complete):
     return complete(u, keep), torch.where(keep, s, torch.zeros_like(s))
 
 
-def block_jacobi(a, stats, opts, jacobi, check, complete):
+def block_jacobi(a, stats, opts, jacobi, check, complete, fused=None):
     """Block Jacobi of a batch of tall matrices a (b, m, n), m >= n, with at
     least two column groups.  `jacobi(y)` enqueues the one-sided Jacobi of a
     batch of pair subproblems and returns (_, _, v) with v (., c, c)
     orthogonal / unitary, columns by descending sigma; `check()` raises the
     errors of the solves enqueued since its last call (called once per
-    sweep); `complete(u, keep)` fills the columns of u not in keep.  Returns
+    sweep); `complete(u, keep)` fills the columns of u not in keep.  `fused`,
+    when given, takes whole rounds: `fused.takes(a, c)` for pairs of up to c
+    columns, `fused.round(wt, vt, idx)` on W and V kept transposed,
+    `fused.worst(wt, live)` for the check, enqueued before `check()`.  Returns
     U (b, m, n), sigma (b, n) descending, V (b, n, n).  Raises
     RuntimeError('block Jacobi did not converge') after max_sweeps (default
     30) sweeps (solvers.py:59-60)."""
@@ -94,9 +100,16 @@ def block_jacobi(a, stats, opts, jacobi, check, complete):
         return a.new_zeros(b, m, n), a.real.new_zeros(b, n), a.new_zeros(b, n, n)
     width = opts.get('block_size', 4)
     dev = a.device
-    rounds = schedule(n, width, dev)
-    w = a.clone()
-    v = torch.eye(n, dtype=a.dtype, device=dev).expand(b, n, n).clone()
+    if fused is not None and not fused.takes(a, min(2 * width, n)):
+        fused = None
+    rounds = schedule(n, width, dev if fused is None else 'cpu')
+    if fused is not None:
+        flat = [idx for buckets in rounds for idx in buckets]       # one copy for all
+        idx = iter(torch.cat([i.reshape(-1) for i in flat]).to(dev, torch.int32).split([i.numel() for i in flat]))
+        rounds = [[next(idx).view(i.shape) for i in buckets] for buckets in rounds]
+        w, v = a.mT.contiguous().mT, torch.eye(n, dtype=a.dtype, device=dev).expand(b, n, n).contiguous().mT
+    else:
+        w, v = a.clone(), torch.eye(n, dtype=a.dtype, device=dev).expand(b, n, n).clone()
     eps = torch.finfo(a.real.dtype).eps
     tol = opts.get('tol') or 40 * eps
     tiny = torch.finfo(a.real.dtype).tiny
@@ -106,6 +119,9 @@ def block_jacobi(a, stats, opts, jacobi, check, complete):
     for sweep in range(max_sweeps):
         for buckets in rounds:
             for idx in buckets:
+                if fused is not None:
+                    fused.round(w.mT, v.mT, idx)
+                    continue
                 k, c = idx.shape
                 flat = idx.reshape(-1)
                 wy = w[:, :, flat].reshape(b, m, k, c).permute(2, 0, 1, 3)     # (pairs, b, m, c)
@@ -117,6 +133,13 @@ def block_jacobi(a, stats, opts, jacobi, check, complete):
                 vv = vv.reshape(k, b, c, c)
                 w[:, :, flat] = (wy @ vv).permute(1, 2, 0, 3).reshape(b, m, k * c)
                 v[:, :, flat] = (vy @ vv).permute(1, 2, 0, 3).reshape(b, n, k * c)
+        if fused is not None:
+            worst = fused.worst(w.mT, eps * max(m, n))
+            check()
+            if bool(worst <= tol):
+                converged = True
+                break
+            continue
         check()
         g = w.mH @ w
         d = g.diagonal(dim1=-2, dim2=-1).real.clamp_min(0)
@@ -141,11 +164,11 @@ def block_jacobi(a, stats, opts, jacobi, check, complete):
     return u, s, v
 
 
-def raw(x, stats, opts, jacobi, check, complete):
+def raw(x, stats, opts, jacobi, check, complete, fused=None):
     """Wide input through its conjugate transpose (solvers.py:224-227).  The
     caller sends a matrix with a single column group to the plain Jacobi
     (:36-37)."""
     if x.shape[-2] < x.shape[-1]:
-        u, s, v = raw(x.mH.resolve_conj().contiguous(), stats, opts, jacobi, check, complete)
+        u, s, v = raw(x.mH.resolve_conj().contiguous(), stats, opts, jacobi, check, complete, fused)
         return v, s, u
-    return block_jacobi(x, stats, opts, jacobi, check, complete)
+    return block_jacobi(x, stats, opts, jacobi, check, complete, fused)

@@ -33,7 +33,8 @@ SYMBOLS = ("jb_version", "jb_device_sm_count", "jb_workspace_bytes", "jb_svd_bat
            "jb_eigh_f64", "jb_eigh_complex_workspace_bytes", "jb_eigh_c64", "jb_eigh_c128",
            "jb_qr_workspace_bytes", "jb_qr_f32", "jb_qr_f64", "jb_qr_c64", "jb_qr_c128",
            "jb_svd_complex_workspace_bytes", "jb_svd_batched_c64", "jb_svd_batched_c128", "jb_jacobi_rounds",
-           "jb_complete_null_workspace_bytes", "jb_complete_null", "jb_prepare", "jb_check_finite", "jb_fma_loop_flops", "jb_fma_loop",
+           "jb_complete_null_workspace_bytes", "jb_complete_null", "jb_prepare", "jb_check_finite",
+           "jb_pair_round_f64", "jb_worst_correlation_f64", "jb_fma_loop_flops", "jb_fma_loop",
            "jb_svd_batched_f32_noalloc")
 GEMM_PLAIN, GEMM_SPLIT3, GEMM_SPLIT6, GEMM_B_MN, GEMM_CHAIN128, GEMM_SYRK = 0, 1, 2, 4, 8, 16
 EIG_FP32 = 128  # JB_EIG_FP32
@@ -136,6 +137,10 @@ def _declare(l):
     l.jb_complete_null_workspace_bytes.argtypes = [I32, I64, I64, I64]
     l.jb_complete_null.restype = ctypes.c_int
     l.jb_complete_null.argtypes = [P, P, I32, I64, I64, I64, P, P, SZ, P]
+    l.jb_pair_round_f64.restype = ctypes.c_int
+    l.jb_pair_round_f64.argtypes = [P, P, P, I64, I32, I32, I32, I32, F64, I32, P, P, P]
+    l.jb_worst_correlation_f64.restype = ctypes.c_int
+    l.jb_worst_correlation_f64.argtypes = [P, I64, I32, I32, F64, P, P, P]
     l.jb_prepare.restype = ctypes.c_int
     l.jb_prepare.argtypes = [P, I32, P, I32, I32, P, P, P, I64, I32, I32, P]
     l.jb_check_finite.restype = ctypes.c_int

@@ -574,7 +574,36 @@ def _pair_solver(jopts, stats):
         pending.clear()
         raise_for_status(host[1], max_sweeps)
         stats['jacobi_sweeps'] = max(stats.get('jacobi_sweeps', 0), int(host[0].max()))
-    return solve, check
+    return solve, check, _FusedRounds(pending, tol, max_sweeps) if not flags else None
+
+
+class _FusedRounds:
+    """Whole rounds of float64 pairs (csrc/jb_rounds.cu), for
+    block_rounds.block_jacobi: up to 128 rows and 32 columns a pair, as the
+    batched float64 solve takes without a QR first."""
+
+    def __init__(self, pending, tol, max_sweeps):
+        self.pending, self.tol, self.max_sweeps = pending, tol, max_sweeps
+
+    def takes(self, a, c):
+        return a.dtype == torch.float64 and a.shape[-2] <= 128 and c <= 32
+
+    def round(self, wt, vt, idx):
+        b, n, m = wt.shape
+        k, c = idx.shape
+        info = torch.empty(2, k * b, dtype=torch.int32, device=wt.device)
+        N.check(N.lib().jb_pair_round_f64(wt.data_ptr(), vt.data_ptr(), idx.data_ptr(), b, m, n, k, c, self.tol,
+                                          self.max_sweeps, info[1].data_ptr(), info[0].data_ptr(),
+                                          torch.cuda.current_stream(wt.device).cuda_stream), 'jb_pair_round_f64')
+        self.pending.append(info)
+
+    def worst(self, wt, live):
+        b, n, m = wt.shape
+        out = torch.empty(b * n + 1, dtype=torch.float64, device=wt.device)
+        N.check(N.lib().jb_worst_correlation_f64(wt.data_ptr(), b, m, n, live, out[1:].data_ptr(), out.data_ptr(),
+                                                 torch.cuda.current_stream(wt.device).cuda_stream),
+                'jb_worst_correlation_f64')
+        return out[0]
 
 
 def _composed_svd(a, algorithm, full_matrices, values_only, return_info, rank, opts):
@@ -606,8 +635,8 @@ def _composed_svd(a, algorithm, full_matrices, values_only, return_info, rank, o
         y, scale, words = _prepare(a, False)
         if algorithm == 'block_jacobi':
             words.read()      # the rounds loop on the host: no NaN may enter them
-            pair_v, check = _pair_solver(jopts, stats)
-            u, sv, v = BR.raw(y, stats, opts, pair_v, check, _complete_null_columns)
+            pair_v, check, fused = _pair_solver(jopts, stats)
+            u, sv, v = BR.raw(y, stats, opts, pair_v, check, _complete_null_columns, fused)
         else:
             u, sv, v = Q.raw(y, algorithm, stats, opts, jacobi)
         sv = (sv * scale[:, None]).to(sv.dtype)
