@@ -18,6 +18,7 @@
 #include <stdint.h>
 #include <math.h>
 #include "jacobi_b200.h"
+#include "jb_group.cuh"
 
 namespace jb {
 namespace blk {
@@ -244,6 +245,75 @@ __global__ void __launch_bounds__(kEigThreads) eig_kernel(const float *Gin, __nv
 // sorted position of every column (pos_out[k * n + j]); q_apply_kernel then
 // forms Q^T from them on other SMs, so this latency-bound kernel issues
 // about a quarter fewer instructions per round.
+//
+// FP32 G is scaled, G = D G_s D, and Q = Q_s D, with a scale per position (FP64):
+// a rotation is then x + b y, y - a x with both scales multiplied by c, one
+// multiply-add an element instead of two (Gentleman's rotation), and c = 1 -
+// t^2 / (...) does not round the cosines of small angles to 1, always to the
+// same side (||Q^T Q - I|| of two sweeps 2.4e-5 -> 2.2e-6).  Scales below 2^-8
+// are multiplied in, once or twice in a sweep of a dense random G.  (FP64 G is
+// not scaled: the scales' own chain costs what the shorter rotations give.)  Q
+// lags one round: while the first warps form the angles of a round, the others
+// apply the previous round's to their tiles of Q.  Rows and columns that cross
+// a lane or a warp go through shared memory in 16-byte accesses (FP32: shuffles
+// took three times as long; FP64 rows by shuffles).  One SM a slot, bound by
+// the latency and the instruction issue of a round; two sweeps of n = 128, 8
+// columns a warp: FP32 G 287 us, 383 with plain rotations, shuffles and Q
+// rotated with G; FP64 G 534 (16 columns a warp), before 570.
+
+// Bytes of the write-out area (n x n FP32) and of the boundary rows (512 a column), n <= 128.
+__host__ __device__ constexpr size_t eig_reg_area_bytes(int n) { return (size_t)n * 512; }
+
+template <typename TG> struct Pair2;
+template <> struct Pair2<float> { using T = float2; };
+template <> struct Pair2<double> { using T = double2; };
+
+// N consecutive elements to and from shared memory in accesses of up to 16 bytes.
+template <typename T, int N>
+struct Run {
+    static constexpr int B = (int)sizeof(T) * N, W = B % 16 == 0 ? 16 : B % 8 == 0 ? 8 : 4, C = W / (int)sizeof(T);
+    struct alignas(W) Chunk { T v[C]; };
+    __device__ static __forceinline__ void put(T *dst, const T (&v)[N]) {
+#pragma unroll
+        for (int i = 0; i < N / C; ++i) {
+            Chunk c;
+#pragma unroll
+            for (int e = 0; e < C; ++e) c.v[e] = v[i * C + e];
+            ((Chunk *)dst)[i] = c;
+        }
+    }
+    __device__ static __forceinline__ void get(const T *src, T (&v)[N]) {
+#pragma unroll
+        for (int i = 0; i < N / C; ++i) {
+            const Chunk c = ((const Chunk *)src)[i];
+#pragma unroll
+            for (int e = 0; e < C; ++e) v[i * C + e] = c.v[e];
+        }
+    }
+};
+
+// Tangent of a live, active pair, and the cosine of a tangent.
+__device__ __forceinline__ float eig_tan(float app, float aqq, float apq) {
+    // |zeta| <= 1e18 keeps its square finite (t is then below 1e-18)
+    const float zeta = fminf(__fdividef(fabsf(aqq - app), 2.f * fabsf(apq)), 1e18f);
+    const float h = fmaf(zeta, zeta, 1.f);
+    const float t = __fdividef(1.f, zeta + h * rsqrtf(h));
+    return (aqq < app) != (apq < 0.f) ? -t : t;
+}
+__device__ __forceinline__ double eig_tan(double app, double aqq, double apq) {
+    const double d = aqq - app, a2 = 2.0 * fabs(apq);
+    const int ex = (__double2hiint(fmax(fabs(d), a2)) >> 20) & 0x7ff;
+    const double scl = __hiloint2double((2046 - ex) << 20, 0);
+    const float df = fabsf((float)(d * scl)), af = (float)(a2 * scl);
+    const float tf = __fdividef(af, df + sqrtf(df * df + af * af));
+    return (d < 0.0) != (apq < 0.0) ? -(double)tf : (double)tf;
+}
+__device__ __forceinline__ double eig_cos(float t) { return cosine(t * t); }
+__device__ __forceinline__ double eig_cos(double t) {        // FP32 estimate and one Newton step in FP64
+    const double x = 1.0 + t * t, c0 = (double)rsqrtf(1.f + (float)t * (float)t);
+    return c0 * (1.5 - 0.5 * x * c0 * c0);
+}
+
 template <int RPT, int CB, typename TG, bool DQ = false>
 __global__ void __launch_bounds__(RPT * 1024 / CB) eig_reg_kernel(const float *Gin, __nv_bfloat16 *Qt_hi,
                                                             __nv_bfloat16 *Qt_lo, __nv_bfloat16 *Qt_lo2,
@@ -251,18 +321,23 @@ __global__ void __launch_bounds__(RPT * 1024 / CB) eig_reg_kernel(const float *G
                                                             int max_sweeps, double tol, const double *live_floor_ptr,
                                                             float2 *cs_out, int *pos_out) {
     constexpr int n = 32 * RPT;
-    constexpr int NW = n / CB;                 // warps
-    static_assert(CB % 2 == 0 && NW >= RPT / 2, "columns per warp");
+    constexpr int NW = n / CB, AW = RPT / 2;   // warps; those that form the angles (the next AW the scales)
+    constexpr bool SC = sizeof(TG) == 4;       // scaled
+    using T2 = typename Pair2<TG>::T;
+    static_assert(CB % 2 == 0 && NW >= 2 * AW && RPT % 2 == 0, "columns per warp");
     extern __shared__ __align__(16) unsigned char smem[];
-    TG *sd = (TG *)smem;               // d[x] = G[x][x]
-    TG *se = sd + n;                       // e[x] = G[x][x + 1]
-    TG *sc = se + n;                       // c of the pair starting at position p, at cs_at(p)
-    TG *ss = sc + n;                       // s of the pair starting at position p, at cs_at(p)
-    TG *bg = ss + n;                       // [NW][2][RPT][32] boundary columns of G (first, last), lane-major
-    float *bq = (float *)(bg + (size_t)NW * 2 * n);  // [NW][2][RPT][32] boundary columns of Q, lane-major
+    double *scl = (double *)smem;              // scale of position x
+    T2 *sab = (T2 *)(scl + n);                 // [2][n] (a, b) of the pair starting at position p, at cs_at(p)
+    TG *sd = (TG *)(sab + 2 * n);              // d[x] = G_s[x][x]
+    TG *se = sd + n;                           // e[x] = G_s[x][x + 1]
+    T2 *sfi = (T2 *)(se + n);                  // the scale of position x and its inverse
+    TG *st = (TG *)(sfi + n);                  // tangent of pair t
+    TG *bg = st + n;                           // [NW][2][32][RPT] boundary columns of G (first, last)
+    float *bq = (float *)(bg + (size_t)NW * 2 * n);  // [NW][2][32][RPT] boundary columns of Q
     float *Qs = bq + (size_t)NW * 2 * n;       // n x n, Q[col * n + row] (write-out)
-    int *perm = (int *)(Qs + (size_t)n * n);   // n
-    __shared__ int s_any;
+    TG *br = (TG *)Qs;                         // [NW][2][CB / chunk][32][chunk] boundary rows of G (before the write-out)
+    int *perm = (int *)((unsigned char *)Qs + eig_reg_area_bytes(n));   // n
+    __shared__ int s_any, s_small;
     __shared__ double s_first_off;
     __shared__ double s_red[NW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -271,13 +346,13 @@ __global__ void __launch_bounds__(RPT * 1024 / CB) eig_reg_kernel(const float *G
     // 32 i + l, so that the 32 lanes reading "their" i-th row hit 32 consecutive words instead of
     // one bank RPT-fold; a warp-uniform row is a broadcast either way.
     auto cs_at = [](int x) { return (x % RPT) * 32 + x / RPT; };
-    auto bnd_at = [](int w, int side, int i, int l) { return ((w * 2 + side) * RPT + i) * 32 + l; };
+    auto bnd_at = [](int w, int side, int l) { return ((w * 2 + side) * 32 + l) * RPT; };
     const int k = blockIdx.x;
     const double live_floor = live_floor_ptr ? *live_floor_ptr : 0.0;
     const float *g_in = Gin + (size_t)k * n * n;
 
     TG g[RPT][CB];
-    float q[RPT][CB];
+    float2 q[RPT / 2][CB];                     // rows 2 i and 2 i + 1 of Q's tile
 #pragma unroll
     for (int i = 0; i < RPT; ++i)
 #pragma unroll
@@ -285,21 +360,102 @@ __global__ void __launch_bounds__(RPT * 1024 / CB) eig_reg_kernel(const float *G
             const int r = r0 + i, c = c0 + j;
             // symmetrise (the tensor-core Gram is symmetric up to rounding)
             g[i][j] = (TG)(0.5 * ((double)g_in[(size_t)r * n + c] + (double)g_in[(size_t)c * n + r]));
-            q[i][j] = (r == c) ? 1.f : 0.f;
+            if (i & 1) q[i / 2][j].y = (r == c) ? 1.f : 0.f;
+            else q[i / 2][j].x = (r == c) ? 1.f : 0.f;
         }
+    // d and e: rows r0.. of a lane meet this warp's columns in LB lanes (both),
+    // and in the lane before them (the e of its last row)
+    constexpr int LB = CB / RPT > 0 ? CB / RPT : 1;
+    static_assert(CB % RPT == 0 || RPT % CB == 0, "tiles");
     auto publish_de = [&]() {
+        if constexpr (CB >= RPT) {
 #pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-            const int x = r0 + i;
+            for (int b = 0; b < LB; ++b)
+                if (lane == warp * LB + b) {
 #pragma unroll
-            for (int j = 0; j < CB; ++j) {
-                if (c0 + j == x) sd[x] = g[i][j];
-                if (c0 + j == x + 1) se[x] = g[i][j];
+                    for (int i = 0; i < RPT; ++i) {
+                        sd[r0 + i] = g[i][b * RPT + i];
+                        if (b * RPT + i + 1 < CB) se[r0 + i] = g[i][b * RPT + i + 1];
+                    }
+                }
+            if (lane == warp * LB - 1) se[r0 + RPT - 1] = g[RPT - 1][0];
+        } else {
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+#pragma unroll
+                for (int j = 0; j < CB; ++j) {
+                    if (c0 + j == r0 + i) sd[r0 + i] = g[i][j];
+                    if (c0 + j == r0 + i + 1) se[r0 + i] = g[i][j];
+                }
+        }
+    };
+    // A rotation and the swap of its positions, x, y <- first(x, y), second(y, x):
+    // y + b x and x - a y of (a, b) when scaled, else s x + c y and c x - s y of (s, c).
+    // (the larger product inside the multiply-add)
+    auto first = [](TG own, TG other, T2 v) -> TG { return SC ? fma(v.y, own, other) : fma(v.y, other, v.x * own); };
+    auto second = [](TG own, TG other, T2 v) -> TG { return SC ? fma(-v.x, own, other) : fma(v.y, other, -v.x * own); };
+    auto turn = [&](TG &x, TG &y, T2 v) {
+        const TG u = x;
+        x = first(u, y, v);
+        y = second(y, u, v);
+    };
+    auto both = [](float v) { return make_float2(v, v); };
+    auto first_q = [&](float2 own, float2 other, T2 v) {
+        if constexpr (SC) return __ffma2_rn(both(v.y), own, other);
+        else return __ffma2_rn(both((float)v.y), other, __fmul2_rn(both((float)v.x), own));
+    };
+    auto second_q = [&](float2 own, float2 other, T2 v) {
+        if constexpr (SC) return __ffma2_rn(both(-v.x), own, other);
+        else return __ffma2_rn(both((float)v.y), other, __fmul2_rn(both(-(float)v.x), own));
+    };
+    auto turn_q = [&](float2 &x, float2 &y, T2 v) {
+        const float2 u = x;
+        x = first_q(u, y, v);
+        y = second_q(y, u, v);
+    };
+    // Q's column rotations of a round of parity par with the angles of buffer buf
+    auto update_q = [&](int par, int buf) {
+        const T2 *ab = sab + buf * n;
+        if (par == 0) {
+#pragma unroll
+            for (int j = 0; j < CB; j += 2) {
+                const T2 t = ab[cs_at(c0 + j)];
+#pragma unroll
+                for (int i = 0; i < RPT / 2; ++i) turn_q(q[i][j], q[i][j + 1], t);
+            }
+        } else {
+            if (warp > 0) {                    // pair (c0 - 1, c0): this warp holds the second
+                const T2 v = ab[cs_at(c0 - 1)];
+                float x[RPT];
+                Run<float, RPT>::get(bq + bnd_at(warp - 1, 1, lane), x);
+#pragma unroll
+                for (int i = 0; i < RPT / 2; ++i)
+                    q[i][0] = second_q(q[i][0], make_float2(x[2 * i], x[2 * i + 1]), v);
+            }
+            if (warp < NW - 1) {               // pair (c0 + CB - 1, c0 + CB): this warp holds the first
+                const T2 v = ab[cs_at(c0 + CB - 1)];
+                float y[RPT];
+                Run<float, RPT>::get(bq + bnd_at(warp + 1, 0, lane), y);
+#pragma unroll
+                for (int i = 0; i < RPT / 2; ++i)
+                    q[i][CB - 1] = first_q(q[i][CB - 1], make_float2(y[2 * i], y[2 * i + 1]), v);
+            }
+#pragma unroll
+            for (int j = 1; j + 1 < CB; j += 2) {
+                const T2 t = ab[cs_at(c0 + j)];
+#pragma unroll
+                for (int i = 0; i < RPT / 2; ++i) turn_q(q[i][j], q[i][j + 1], t);
             }
         }
     };
     publish_de();
-    if (threadIdx.x == 0) s_first_off = 0.0;
+    T2 one;
+    one.x = one.y = (TG)1;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        scl[i] = 1.0;
+        sfi[i] = one;
+    }
+    if (threadIdx.x == 0) { s_first_off = 0.0; s_small = 0; }
     __syncthreads();
     double dm = 0.0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) dm = fmax(dm, (double)sd[i]);
@@ -311,192 +467,256 @@ __global__ void __launch_bounds__(RPT * 1024 / CB) eig_reg_kernel(const float *G
     for (int w = 0; w < NW; ++w) gmax = fmax(gmax, s_red[w]);
     // eps of the arithmetic squared times the largest diagonal: the active floor
     constexpr double eps_g = sizeof(TG) == 8 ? 2.220446049250313e-16 : 1.1920928955078125e-07;
-    const double floor_ = eps_g * eps_g * gmax;
-    const double tol2 = tol * tol;
-    int sweep = 0;
+    const TG floor_ = (TG)(eps_g * eps_g * gmax), live = (TG)live_floor;
+    const TG tol2 = (TG)(tol * tol);
+    int sweep = 0, buf = 0;                    // buf: the angles of the round at hand
+    bool lag = false;                          // Q still lacks the previous round (odd, or even: its parity is 1 - par)
     for (sweep = 1; sweep <= max_sweeps; ++sweep) {
         if (threadIdx.x == 0) s_any = 0;
-        double offn = 0.0, offd = 1.0;
-        for (int r = 0; r < n; ++r) {
+        TG offm = 0;                           // the largest a_pq^2 / (a_pp a_qq) this thread met
+        for (int r = 0; r < n; ++r, buf ^= 1) {
             const int par = r & 1;
             __syncthreads();                   // d / e of the previous round published; s_any reset
-            if (warp < RPT / 2) {                 // one pair per lane
-                {
-                    const int t = warp * 32 + lane;
-                    if (t >= n / 2 - par) goto angles_done;
-                    const int p = 2 * t + par;
-                    const double app = sd[p], aqq = sd[p + 1], apq = se[p];
-                    TG c = 1, sn = 0;
-                    const double prod = app * aqq, apq2 = apq * apq;
-                    if (apq2 > tol2 * prod && fmin(app, aqq) > floor_) {
+            const bool small = s_small != 0;
+            if (warp < AW) {                   // the angles, a pair a lane
+                const int p = 2 * threadIdx.x + par;
+                if (p + 1 < n) {
+                    T2 fp, fq;
+                    TG app = sd[p], aqq = sd[p + 1], apq = se[p];
+                    if constexpr (SC) {
+                        fp = sfi[p];
+                        fq = sfi[p + 1];
+                        app *= fp.x * fp.x;
+                        aqq *= fq.x * fq.x;
+                        apq *= fp.x * fq.x;
+                    }
+                    const TG low = app < aqq ? app : aqq;
+                    bool on;
+                    TG ratio = 0, tt = 0;
+                    if constexpr (sizeof(TG) == 4) {         // no product of two small entries: no underflow
+                        ratio = low > floor_ ? __fdividef(apq, app) * __fdividef(apq, aqq) : 0.f;
+                        on = ratio > tol2;
+                    } else {
+                        on = apq * apq > tol2 * (app * aqq) && low > floor_;
+                        if (on && sweep == 1) ratio = apq * apq / (app * aqq);
+                    }
+                    if (on) {
                         // off over live columns only (solvers.py:55-57)
-                        if (fmin(app, aqq) > live_floor && apq2 * offd > offn * prod) { offn = apq2; offd = prod; }
-                        if constexpr (sizeof(TG) == 8) {
-                            const double d = aqq - app, a2 = 2.0 * fabs(apq);
-                            const int ex = (__double2hiint(fmax(fabs(d), a2)) >> 20) & 0x7ff;
-                            const double scl = __hiloint2double((2046 - ex) << 20, 0);
-                            const float df = fabsf((float)(d * scl)), af = (float)(a2 * scl);
-                            const float tf = __fdividef(af, df + sqrtf(df * df + af * af));
-                            const double tt = d < 0.0 ? -(double)tf : (double)tf;
-                            // c = 1 / sqrt(1 + t^2): FP32 estimate and one Newton step in FP64
-                            const double x = 1.0 + tt * tt;
-                            const double c0 = (double)rsqrtf(1.f + tf * tf);
-                            c = c0 * (1.5 - 0.5 * x * c0 * c0);
-                            sn = tt * c;
-                        } else {
-                            // FP32 G (the two-part stage): the same angle, all in FP32
-                            const float d = (float)(aqq - app), a2 = 2.f * fabsf((float)apq);
-                            const float tf = __fdividef(a2, fabsf(d) + sqrtf(d * d + a2 * a2));
-                            const float tt = d < 0.f ? -tf : tf;
-                            c = rsqrtf(1.f + tt * tt);
-                            sn = tt * c;
-                        }
-                        if (apq < 0.0) sn = -sn;
+                        if (low > live && ratio > offm) offm = ratio;
+                        tt = eig_tan(app, aqq, apq);
                         s_any = 1;
                     }
-                    sc[cs_at(p)] = c;
-                    ss[cs_at(p)] = sn;
-                    if constexpr (DQ)
-                        cs_out[(((size_t)k * max_sweeps + (sweep - 1)) * n + r) * n + p] = make_float2((float)c, (float)sn);
+                    T2 v;
+                    if constexpr (SC) {
+                        v.x = tt * (fq.x * fp.y);
+                        v.y = tt * (fp.x * fq.y);
+                        st[threadIdx.x] = tt;
+                    } else {
+                        v.y = on ? eig_cos(tt) : (TG)1;
+                        v.x = tt * v.y;
+                        if constexpr (DQ)
+                            cs_out[(((size_t)k * max_sweeps + (sweep - 1)) * n + r) * n + p] =
+                                make_float2((float)v.y, (float)v.x);
+                    }
+                    sab[buf * n + cs_at(p)] = v;
                 }
-            angles_done:;
+            } else if constexpr (!DQ) {
+                if (lag) update_q(1 - par, buf ^ 1);
             }
             __syncthreads();
-            // Rows (J^T from the left, then the swap): (x_p, x_q) <- (s x_p + c x_q, c x_p - s x_q).
+            const T2 *ab = sab + buf * n;
+            if (warp < AW) {
+                if constexpr (!DQ)
+                    if (lag) update_q(1 - par, buf ^ 1);
+            } else if (SC && warp < 2 * AW) {  // the scales, which the next round's angles need
+                const int x = threadIdx.x - 32 * AW, p = 2 * x + par;
+                if (p + 1 < n) {
+                    const TG tt = st[x];
+                    const double c = eig_cos(tt), np_ = c * scl[p + 1], nq_ = c * scl[p];
+                    T2 f, h;
+                    f.x = (TG)np_;
+                    f.y = inv_scale(f.x);
+                    h.x = (TG)nq_;
+                    h.y = inv_scale(h.x);
+                    scl[p] = np_;
+                    scl[p + 1] = nq_;
+                    sfi[p] = f;
+                    sfi[p + 1] = h;
+                    if (fmin(np_, nq_) < 0.00390625) s_small = 1;
+                    if constexpr (DQ)
+                        cs_out[(((size_t)k * max_sweeps + (sweep - 1)) * n + r) * n + p] =
+                            make_float2((float)c, (float)((double)tt * c));
+                }
+            }
+            // Rows (J^T from the left, then the swap).
             if (par == 0) {
 #pragma unroll
                 for (int i = 0; i < RPT; i += 2) {
-                    const TG c = sc[32 * i + lane], sn = ss[32 * i + lane];       // pair at row r0 + i
+                    const T2 v = ab[32 * i + lane];          // pair at row r0 + i
 #pragma unroll
-                    for (int j = 0; j < CB; ++j) {
-                        const TG x = g[i][j], y = g[i + 1][j];
-                        g[i][j] = sn * x + c * y;
-                        g[i + 1][j] = c * x - sn * y;
-                    }
+                    for (int j = 0; j < CB; ++j) turn(g[i][j], g[i + 1][j], v);
                 }
             } else {
-                const bool has_up = lane > 0, has_down = lane < 31;
-                // pairs at rows r0 - 1 (lane - 1's last row) and r0 + RPT - 1 (this lane's last row)
-                const TG cu = has_up ? sc[32 * (RPT - 1) + lane - 1] : (TG)1,
-                         su = has_up ? ss[32 * (RPT - 1) + lane - 1] : (TG)0;
-                const TG cd = has_down ? sc[32 * (RPT - 1) + lane] : (TG)1,
-                         sdn = has_down ? ss[32 * (RPT - 1) + lane] : (TG)0;
+                // pairs at rows r0 - 1 (lane - 1's last row) and r0 + RPT - 1 (this lane's last row);
+                // their other rows through shared memory (FP32) or by shuffles
+                constexpr int CH = 16 / (int)sizeof(TG) < CB ? 16 / (int)sizeof(TG) : CB;
+                TG *mine = br + (size_t)warp * 2 * CB * 32 + lane * CH;
+                if constexpr (SC) {
 #pragma unroll
-                for (int j = 0; j < CB; ++j) {
-                    const TG up = __shfl_up_sync(0xffffffffu, g[RPT - 1][j], 1);   // row r0 - 1
-                    const TG dn = __shfl_down_sync(0xffffffffu, g[0][j], 1);       // row r0 + RPT
-                    const TG first = g[0][j], last = g[RPT - 1][j];
-                    if (has_up) g[0][j] = cu * up - su * first;                         // second of pair (r0 - 1, r0)
-                    if (has_down) g[RPT - 1][j] = sdn * last + cd * dn;                 // first of pair (r0 + RPT - 1, r0 + RPT)
+                    for (int jc = 0; jc < CB / CH; ++jc) {
+                        TG f[CH], l[CH];
+#pragma unroll
+                        for (int e = 0; e < CH; ++e) {
+                            f[e] = g[0][jc * CH + e];
+                            l[e] = g[RPT - 1][jc * CH + e];
+                        }
+                        Run<TG, CH>::put(mine + jc * 32 * CH, f);
+                        Run<TG, CH>::put(mine + (CB / CH + jc) * 32 * CH, l);
+                    }
+                    __syncwarp();
+                }
+                const int up = lane > 0 ? -CH : 0, down = lane < 31 ? CH : 0;
+                T2 vu, vd;                     // no pair: the row itself, from a zero other row
+                vu.x = (TG)-1;
+                vu.y = (TG)0;
+                vd.x = vd.y = (TG)1;
+                if constexpr (!SC) vd.y = (TG)0;
+                if (lane > 0) vu = ab[32 * (RPT - 1) + lane - 1];
+                if (lane < 31) vd = ab[32 * (RPT - 1) + lane];
+                if constexpr (SC) {
+#pragma unroll
+                    for (int jc = 0; jc < CB / CH; ++jc) {
+                        TG f[CH], l[CH];
+                        Run<TG, CH>::get(mine + (CB / CH + jc) * 32 * CH + up, l);
+                        Run<TG, CH>::get(mine + jc * 32 * CH + down, f);
+#pragma unroll
+                        for (int e = 0; e < CH; ++e) {
+                            const int j = jc * CH + e;
+                            g[0][j] = second(g[0][j], lane > 0 ? l[e] : (TG)0, vu);
+                            g[RPT - 1][j] = first(g[RPT - 1][j], lane < 31 ? f[e] : (TG)0, vd);
+                        }
+                    }
+                    __syncwarp();
+                } else {
+#pragma unroll
+                    for (int j = 0; j < CB; ++j) {
+                        const TG l = __shfl_up_sync(0xffffffffu, g[RPT - 1][j], 1);      // row r0 - 1
+                        const TG f = __shfl_down_sync(0xffffffffu, g[0][j], 1);          // row r0 + RPT
+                        g[0][j] = second(g[0][j], lane > 0 ? l : (TG)0, vu);
+                        g[RPT - 1][j] = first(g[RPT - 1][j], lane < 31 ? f : (TG)0, vd);
+                    }
                 }
 #pragma unroll
                 for (int i = 1; i + 1 < RPT; i += 2) {
-                    const TG c = sc[32 * i + lane], sn = ss[32 * i + lane];       // pair at row r0 + i
+                    const T2 v = ab[32 * i + lane];          // pair at row r0 + i
 #pragma unroll
-                    for (int j = 0; j < CB; ++j) {
-                        const TG x = g[i][j], y = g[i + 1][j];
-                        g[i][j] = sn * x + c * y;
-                        g[i + 1][j] = c * x - sn * y;
-                    }
+                    for (int j = 0; j < CB; ++j) turn(g[i][j], g[i + 1][j], v);
                 }
             }
-            // Columns (J from the right, then the swap), G and Q alike.
+            // Columns (J from the right, then the swap).
             if (par == 0) {
 #pragma unroll
                 for (int j = 0; j < CB; j += 2) {
-                    const TG c = sc[cs_at(c0 + j)], sn = ss[cs_at(c0 + j)];
-                    const float fc = (float)c, fs = (float)sn;
+                    const T2 v = ab[cs_at(c0 + j)];
 #pragma unroll
-                    for (int i = 0; i < RPT; ++i) {
-                        const TG x = g[i][j], y = g[i][j + 1];
-                        g[i][j] = sn * x + c * y;
-                        g[i][j + 1] = c * x - sn * y;
-                        if constexpr (!DQ) {
-                            const float u = q[i][j], v = q[i][j + 1];
-                            q[i][j] = fs * u + fc * v;
-                            q[i][j + 1] = fc * u - fs * v;
-                        }
-                    }
+                    for (int i = 0; i < RPT; ++i) turn(g[i][j], g[i][j + 1], v);
                 }
             } else {
-                // publish this warp's first and last columns (after the row rotation)
+                // publish this warp's first and last columns (G after the row rotation, Q for update_q)
+                TG lo[RPT], hi[RPT];
 #pragma unroll
                 for (int i = 0; i < RPT; ++i) {
-                    bg[bnd_at(warp, 0, i, lane)] = g[i][0];
-                    bg[bnd_at(warp, 1, i, lane)] = g[i][CB - 1];
-                    if constexpr (!DQ) {
-                        bq[bnd_at(warp, 0, i, lane)] = q[i][0];
-                        bq[bnd_at(warp, 1, i, lane)] = q[i][CB - 1];
+                    lo[i] = g[i][0];
+                    hi[i] = g[i][CB - 1];
+                }
+                Run<TG, RPT>::put(bg + bnd_at(warp, 0, lane), lo);
+                Run<TG, RPT>::put(bg + bnd_at(warp, 1, lane), hi);
+                if constexpr (!DQ) {
+                    float qf[RPT], ql[RPT];
+#pragma unroll
+                    for (int i = 0; i < RPT; ++i) {
+                        qf[i] = i & 1 ? q[i / 2][0].y : q[i / 2][0].x;
+                        ql[i] = i & 1 ? q[i / 2][CB - 1].y : q[i / 2][CB - 1].x;
                     }
+                    Run<float, RPT>::put(bq + bnd_at(warp, 0, lane), qf);
+                    Run<float, RPT>::put(bq + bnd_at(warp, 1, lane), ql);
                 }
                 __syncthreads();
-                const bool has_left = warp > 0, has_right = warp < NW - 1;
-                const TG cl = has_left ? sc[cs_at(c0 - 1)] : (TG)1, sl = has_left ? ss[cs_at(c0 - 1)] : (TG)0;
-                const TG cr = has_right ? sc[cs_at(c0 + CB - 1)] : (TG)1,
-                         sr = has_right ? ss[cs_at(c0 + CB - 1)] : (TG)0;
+                if (warp > 0) {                // pair (c0 - 1, c0): this warp holds the second
+                    const T2 v = ab[cs_at(c0 - 1)];
+                    Run<TG, RPT>::get(bg + bnd_at(warp - 1, 1, lane), hi);
 #pragma unroll
-                for (int i = 0; i < RPT; ++i) {
-                    if (has_left) {                // pair (c0 - 1, c0): this warp holds the second
-                        const TG x = bg[bnd_at(warp - 1, 1, i, lane)];
-                        g[i][0] = cl * x - sl * g[i][0];
-                        if constexpr (!DQ) {
-                            const float u = bq[bnd_at(warp - 1, 1, i, lane)];
-                            q[i][0] = (float)cl * u - (float)sl * q[i][0];
-                        }
-                    }
-                    if (has_right) {               // pair (c0 + CB - 1, c0 + CB): this warp holds the first
-                        const TG y = bg[bnd_at(warp + 1, 0, i, lane)];
-                        g[i][CB - 1] = sr * g[i][CB - 1] + cr * y;
-                        if constexpr (!DQ) {
-                            const float v = bq[bnd_at(warp + 1, 0, i, lane)];
-                            q[i][CB - 1] = (float)sr * q[i][CB - 1] + (float)cr * v;
-                        }
-                    }
+                    for (int i = 0; i < RPT; ++i) g[i][0] = second(g[i][0], hi[i], v);
+                }
+                if (warp < NW - 1) {           // pair (c0 + CB - 1, c0 + CB): this warp holds the first
+                    const T2 v = ab[cs_at(c0 + CB - 1)];
+                    Run<TG, RPT>::get(bg + bnd_at(warp + 1, 0, lane), lo);
+#pragma unroll
+                    for (int i = 0; i < RPT; ++i) g[i][CB - 1] = first(g[i][CB - 1], lo[i], v);
                 }
 #pragma unroll
                 for (int j = 1; j + 1 < CB; j += 2) {
-                    const TG c = sc[cs_at(c0 + j)], sn = ss[cs_at(c0 + j)];
-                    const float fc = (float)c, fs = (float)sn;
+                    const T2 v = ab[cs_at(c0 + j)];
 #pragma unroll
-                    for (int i = 0; i < RPT; ++i) {
-                        const TG x = g[i][j], y = g[i][j + 1];
-                        g[i][j] = sn * x + c * y;
-                        g[i][j + 1] = c * x - sn * y;
-                        if constexpr (!DQ) {
-                            const float u = q[i][j], v = q[i][j + 1];
-                            q[i][j] = fs * u + fc * v;
-                            q[i][j + 1] = fc * u - fs * v;
-                        }
+                    for (int i = 0; i < RPT; ++i) turn(g[i][j], g[i][j + 1], v);
+                }
+            }
+            lag = true;
+            if (SC && small) {                       // read after the round's first barrier: the same in every thread
+                if constexpr (!DQ) update_q(par, buf);
+                lag = false;
+                __syncthreads();
+#pragma unroll
+                for (int j = 0; j < CB; ++j) {
+                    const double dj = scl[c0 + j];
+#pragma unroll
+                    for (int i = 0; i < RPT; ++i) g[i][j] *= (TG)(scl[r0 + i] * dj);
+#pragma unroll
+                    for (int i = 0; i < RPT / 2; ++i) {
+                        q[i][j].x *= (float)dj;
+                        q[i][j].y *= (float)dj;
                     }
                 }
+                __syncthreads();
+                for (int i = threadIdx.x; i < n; i += blockDim.x) {
+                    scl[i] = 1.0;
+                    sfi[i] = one;
+                }
+                if (threadIdx.x == 0) s_small = 0;
             }
             publish_de();
         }
-        if (sweep == 1 && warp < RPT / 2) {
+        if (sweep == 1 && warp < AW) {
             for (int o = 16; o; o >>= 1) {
-                const double on = __shfl_xor_sync(0xffffffffu, offn, o), od = __shfl_xor_sync(0xffffffffu, offd, o);
-                if (on * offd > offn * od) { offn = on; offd = od; }
+                const TG v = __shfl_xor_sync(0xffffffffu, offm, o);
+                offm = v > offm ? v : offm;
             }
-            if (lane == 0) s_red[warp] = sqrt(offn / offd);
+            if (lane == 0) s_red[warp] = sqrt((double)offm);
         }
         __syncthreads();
         if (sweep == 1 && threadIdx.x == 0) {
             double o = 0.0;
 #pragma unroll
-            for (int w = 0; w < RPT / 2; ++w) o = fmax(o, s_red[w]);
+            for (int w = 0; w < AW; ++w) o = fmax(o, s_red[w]);
             s_first_off = o;
         }
         const int any = s_any;
         __syncthreads();                       // everyone has read s_any before it is reset
         if (!any) break;
     }
-    // Q to shared memory (column-major) for the sorted write-out.
+    if constexpr (!DQ)
+        if (lag) update_q(1, buf ^ 1);         // a sweep ends on an odd round
+    // Q to shared memory (column-major) for the sorted write-out; scales back in.
     if constexpr (!DQ) {
 #pragma unroll
-        for (int i = 0; i < RPT; ++i)
+        for (int j = 0; j < CB; ++j) {
+            const double dj = scl[c0 + j];
 #pragma unroll
-            for (int j = 0; j < CB; ++j) Qs[(size_t)(c0 + j) * n + r0 + i] = q[i][j];
+            for (int i = 0; i < RPT; ++i)
+                Qs[(size_t)(c0 + j) * n + r0 + i] = (float)(dj * (double)(i & 1 ? q[i / 2][j].y : q[i / 2][j].x));
+        }
     }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) sd[i] = (TG)((double)sd[i] * scl[i] * scl[i]);
     __syncthreads();
     // Eigenvalues descending (stable), Q^T rows in that order.
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
@@ -594,8 +814,8 @@ __global__ void __launch_bounds__(256) q_apply_kernel(const float2 *cs, const in
 
 __host__ inline size_t eig_reg_smem_bytes(int n, int cb) {   // sized for FP64 G (enough for FP32)
     const int nw = n / cb;
-    return (size_t)4 * n * 8 + (size_t)nw * 2 * n * 8 + (size_t)nw * 2 * n * 4 + (size_t)n * n * 4 + (size_t)n * 4 +
-           16;
+    return (size_t)10 * n * 8 + (size_t)nw * 2 * n * 8 + (size_t)nw * 2 * n * 4 + eig_reg_area_bytes(n) +
+           (size_t)n * 4 + 16;
 }
 
 // dst row map[r] <- src row r (length L), split into hi / lo BF16.
@@ -830,20 +1050,11 @@ __host__ inline size_t eig_dq_bytes(int64_t pairs, int n, int max_sweeps) {
 }
 
 template <int RPT, int CB, typename TG>
-static int launch_eig_reg(const float *G, void *Qt_hi, void *Qt_lo, void *Qt_lo2, float *off, float *dmax,
-                          int32_t *sweeps, int64_t pairs, int32_t max_sweeps, double tol, const double *live_floor,
-                          unsigned char *dq_ws, cudaStream_t st) {
+static int launch_eig_reg_dq(const float *G, void *Qt_hi, void *Qt_lo, void *Qt_lo2, float *off, float *dmax,
+                             int32_t *sweeps, int64_t pairs, int32_t max_sweeps, double tol, const double *live_floor,
+                             unsigned char *dq_ws, cudaStream_t st) {
     constexpr int n = 32 * RPT;
     const size_t smem = eig_reg_smem_bytes(n, CB);
-    if (!dq_ws) {
-        auto kern = eig_reg_kernel<RPT, CB, TG>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return JB_ECUDA;
-        kern<<<(unsigned)pairs, 32 * (n / CB), smem, st>>>(G, (__nv_bfloat16 *)Qt_hi, (__nv_bfloat16 *)Qt_lo,
-                                                          (__nv_bfloat16 *)Qt_lo2, off, dmax, sweeps, max_sweeps, tol,
-                                                          live_floor, nullptr, nullptr);
-        return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
-    }
     float2 *cs = (float2 *)dq_ws;
     int *pos = (int *)(dq_ws + eig_dq_cs_bytes(pairs, n, max_sweeps));
     auto kern = eig_reg_kernel<RPT, CB, TG, true>;
@@ -860,6 +1071,24 @@ static int launch_eig_reg(const float *G, void *Qt_hi, void *Qt_lo, void *Qt_lo2
     return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
 }
 
+template <int RPT, int CB, typename TG>
+static int launch_eig_reg(const float *G, void *Qt_hi, void *Qt_lo, void *Qt_lo2, float *off, float *dmax,
+                          int32_t *sweeps, int64_t pairs, int32_t max_sweeps, double tol, const double *live_floor,
+                          unsigned char *dq_ws, cudaStream_t st) {
+    constexpr int n = 32 * RPT;
+    const size_t smem = eig_reg_smem_bytes(n, CB);
+    if (dq_ws)
+        return launch_eig_reg_dq<RPT, CB, TG>(G, Qt_hi, Qt_lo, Qt_lo2, off, dmax, sweeps, pairs, max_sweeps, tol,
+                                              live_floor, dq_ws, st);
+    auto kern = eig_reg_kernel<RPT, CB, TG>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return JB_ECUDA;
+    kern<<<(unsigned)pairs, 32 * (n / CB), smem, st>>>(G, (__nv_bfloat16 *)Qt_hi, (__nv_bfloat16 *)Qt_lo,
+                                                      (__nv_bfloat16 *)Qt_lo2, off, dmax, sweeps, max_sweeps, tol,
+                                                      live_floor, nullptr, nullptr);
+    return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
+}
+
 template <typename TG>
 static int dispatch_eig_reg(int n, int cb, const float *G, void *Qt_hi, void *Qt_lo, void *Qt_lo2, float *off,
                             float *dmax, int32_t *sweeps, int64_t pairs, int32_t max_sweeps, double tol,
@@ -872,7 +1101,14 @@ static int dispatch_eig_reg(int n, int cb, const float *G, void *Qt_hi, void *Qt
     JB_EIG_CASE(64, 2, 8)
     JB_EIG_CASE(64, 2, 16)
     JB_EIG_CASE(128, 4, 4)
-    JB_EIG_CASE(128, 4, 8)
+    // FP64 G with Q needs more registers than 512 threads have: 630 us two sweeps, with 256 threads 534
+    if (sizeof(TG) == 8 && n == 128 && cb == 8 && !dq_ws) cb = 16;
+    if constexpr (sizeof(TG) == 4) {
+        JB_EIG_CASE(128, 4, 8)
+    } else if (n == 128 && cb == 8) {
+        return launch_eig_reg_dq<4, 8, TG>(G, Qt_hi, Qt_lo, Qt_lo2, off, dmax, sweeps, pairs, max_sweeps, tol,
+                                           live_floor, dq_ws, st);
+    }
     JB_EIG_CASE(128, 4, 16)
 #undef JB_EIG_CASE
     return JB_EINVAL;
