@@ -1179,20 +1179,49 @@ static int launch_group_as(Params &p, int mt, int nt, cudaStream_t st) {
 // rows a lane from the shape (the registers hold 2B columns of W and V a
 // group, at most 96 of them).  Full bases fit too: at most 131 columns, 203 KB.
 // B200, ms a batch, this / one warp a block pair (jb_regblock.cuh): 1024 x
-// 64 x 32 FP64 0.72 / 2.00, 2048 x 45 x 61 FP32 1.29 / 2.15.
+// 64 x 32 FP64 0.69 / 2.00, 2048 x 45 x 61 FP32 1.29 / 2.15.  The rows a lane follow
+// the shape closely, as padding rows cost what rows cost: 2048 matrices of FP64
+// 48 x 32 0.74 ms with 48 rows, 0.94 with 64; 90 x 60 6.6 with 96, 9.8 with 128; 32 x
+// 32 0.80 and FP32 0.35 with 32, 0.95 and 0.42 with 64.  (90 x 16 gains nothing: 0.375
+// with 96, 0.369 with 128.)
 static int launch_group(Params &p, int elem, cudaStream_t st) {
     const int mt = p.um > p.un ? p.um : p.un, nt = p.um > p.un ? p.un : p.um;
     if (elem == 8) {
-        if (nt <= 16 && mt <= 32) return launch_group_as<double, 8, 2, 4, 2, 32>(p, mt, nt, st);
-        if (nt <= 16) return launch_group_as<double, 16, 2, 8, 2, 64>(p, mt, nt, st);
-        if (nt <= 32 && mt <= 64) return launch_group_as<double, 8, 2, 8, 4, 64>(p, mt, nt, st);
-        if (nt <= 32) return launch_group_as<double, 16, 2, 8, 2, 128>(p, mt, nt, st);
+        if (nt <= 16) {
+            if (mt <= 32) return launch_group_as<double, 8, 2, 4, 2, 32>(p, mt, nt, st);
+            if (mt <= 64) return launch_group_as<double, 16, 2, 4, 2, 64>(p, mt, nt, st);
+            return launch_group_as<double, 16, 2, 8, 2, 64>(p, mt, nt, st);
+        }
+        if (nt <= 32) {
+            if (mt <= 32) return launch_group_as<double, 8, 2, 4, 4, 64>(p, mt, nt, st);
+            if (mt <= 48) return launch_group_as<double, 8, 2, 6, 4, 64>(p, mt, nt, st);
+            if (mt <= 64) return launch_group_as<double, 8, 2, 8, 4, 64>(p, mt, nt, st);
+            if (mt <= 96) return launch_group_as<double, 16, 2, 6, 2, 128>(p, mt, nt, st);
+            return launch_group_as<double, 16, 2, 8, 2, 128>(p, mt, nt, st);
+        }
         if (mt <= 64) return launch_group_as<double, 16, 2, 4, 4, 256>(p, mt, nt, st);
+        if (mt <= 96) return launch_group_as<double, 16, 2, 6, 4, 256>(p, mt, nt, st);
         return launch_group_as<double, 16, 2, 8, 4, 256>(p, mt, nt, st);
     }
-    if (nt <= 16 && mt <= 32) return launch_group_as<float, 8, 2, 4, 4, 32>(p, mt, nt, st);
-    if (nt <= 32 && mt <= 64) return launch_group_as<float, 8, 2, 8, 4, 64>(p, mt, nt, st);
-    if (nt <= 32) return launch_group_as<float, 16, 2, 8, 4, 128>(p, mt, nt, st);
+    // FP32: rows by 32 (whole 16-byte chunks).  The lanes of a shape are those of
+    // group_uneven_kernel, so the sums are too (rows of padding add zeros).
+    if (nt <= 16) {
+        if (mt <= 32) return launch_group_as<float, 8, 2, 4, 4, 32>(p, mt, nt, st);
+        // 16 columns need half the threads of 32; a batch of few matrices keeps
+        // them for the loads and the epilogue (16 x 60 x 16: 57 us, 66 with half;
+        // 2048: 159 and 105)
+        const bool few = p.count <= 2 * sm_count();
+        if (mt <= 64)
+            return few ? launch_group_as<float, 8, 2, 8, 4, 64>(p, mt, nt, st)
+                       : launch_group_as<float, 8, 2, 8, 4, 32>(p, mt, nt, st);
+        return few ? launch_group_as<float, 16, 2, 8, 4, 128>(p, mt, nt, st)
+                   : launch_group_as<float, 16, 2, 8, 4, 64>(p, mt, nt, st);
+    }
+    if (nt <= 32) {
+        if (mt <= 32) return launch_group_as<float, 8, 2, 4, 4, 64>(p, mt, nt, st);
+        if (mt <= 64) return launch_group_as<float, 8, 2, 8, 4, 64>(p, mt, nt, st);
+        return launch_group_as<float, 16, 2, 8, 4, 128>(p, mt, nt, st);
+    }
     if (mt <= 64) return launch_group_as<float, 8, 2, 8, 8, 128>(p, mt, nt, st);
     return launch_group_as<float, 16, 2, 8, 4, 256>(p, mt, nt, st);
 }

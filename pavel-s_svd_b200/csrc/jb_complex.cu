@@ -338,22 +338,32 @@ static int entry(const void *A, void *U, R *S, void *Vh, int32_t *sweeps, int32_
     if (batch == 0) return JB_OK;
     const R t = tol > 0 ? (R)tol : R(10) * (sizeof(R) == 4 ? (R)1.1920928955078125e-07 : (R)2.220446049250313e-16);
     // up to 128 x 64: in registers, lanes a pair and rows a lane from the shape
-    // (at most 48 (FP32) or 96 (FP64) registers of W and V)
+    // (at most 48 (FP32) or 96 (FP64) registers of W and V).  Padding rows and
+    // columns cost what others do: 2048 matrices complex128 48 x 32 2.1 ms with 48
+    // rows, 2.6 with 64; 64 x 50 12.7 with 64, 19.2 with 128; complex64 64 x 16 0.25
+    // with 16 columns and 64 rows, 0.57 with 32 and 128.
     if (m <= 128 && n <= 64) {
 #define JB_CGROUP(GL, RW, RV, TH) \
         return launch_cgroup<R, GL, RW, RV, TH>(A, U, S, Vh, sweeps, status, batch, m, n, t, max_sweeps, \
                                                 (cudaStream_t)stream)
-        if constexpr (sizeof(R) == 4) {
-            if (n <= 16 && m <= 32) JB_CGROUP(8, 4, 2, 64);
-            if (n <= 32 && m <= 48) JB_CGROUP(8, 6, 4, 128);
-            if (n <= 32) JB_CGROUP(16, 8, 2, 256);
-            JB_CGROUP(16, 8, 4, 512);
-        } else {
-            if (n <= 16 && m <= 32) JB_CGROUP(8, 4, 2, 64);
-            if (n <= 32 && m <= 64) JB_CGROUP(8, 8, 4, 128);
-            if (n <= 32) JB_CGROUP(16, 8, 2, 256);
-            JB_CGROUP(16, 8, 4, 512);
+        if (n <= 16) {
+            if (m <= 32) JB_CGROUP(8, 4, 2, 64);
+            if (m <= 48) JB_CGROUP(8, 6, 2, 64);
+            if (m <= 64) JB_CGROUP(8, 8, 2, 64);
+            if (batch <= 2 * sm_count()) JB_CGROUP(16, 8, 2, 256);   // few matrices: threads for loads and epilogue
+            JB_CGROUP(16, 8, 2, 128);
         }
+        if (n <= 32) {
+            if (m <= 32) JB_CGROUP(8, 4, 4, 128);
+            if (m <= 48) JB_CGROUP(8, 6, 4, 128);
+            if constexpr (sizeof(R) == 8)
+                if (m <= 64) JB_CGROUP(8, 8, 4, 128);
+            if (m <= 96) JB_CGROUP(16, 6, 2, 256);
+            JB_CGROUP(16, 8, 2, 256);
+        }
+        if (m <= 64) JB_CGROUP(16, 4, 4, 512);
+        if (m <= 96) JB_CGROUP(16, 6, 4, 512);
+        JB_CGROUP(16, 8, 4, 512);
 #undef JB_CGROUP
     }
     const int np = n + (n & 1);

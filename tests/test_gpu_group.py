@@ -19,7 +19,8 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 # (m, n): edges of the tiles (16, 32, 64 columns; 32, 48, 64, 128 rows), odd sizes
 SIZES = [(1, 1), (2, 2), (5, 3), (32, 16), (31, 15), (33, 16), (128, 16), (96, 13), (17, 17), (48, 17), (48, 32),
-         (49, 32), (64, 32), (64, 31), (65, 32), (128, 32), (33, 33), (64, 33), (64, 64), (65, 64), (100, 47), (128, 64)]
+         (49, 32), (64, 32), (64, 31), (65, 32), (128, 32), (33, 33), (64, 33), (64, 64), (65, 64), (100, 47), (128, 64),
+         (32, 32), (30, 24), (47, 16), (60, 14), (64, 16), (65, 16), (96, 32), (97, 30), (60, 40), (96, 64), (97, 50)]
 
 
 @pytest.fixture(scope="module")
@@ -124,3 +125,20 @@ def test_eigen_sizes(n, dt):
     assert float(np.abs(np.conj(np.swapaxes(v, 1, 2)) @ v - np.eye(n)).max()) <= 100 * n * eps
     res = np.abs(h.astype(np.complex128) @ v - v * w[:, None, :]).max((-2, -1)) / scale
     assert float(res.max()) <= 100 * n * eps
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.complex64, np.complex128])
+@pytest.mark.parametrize("m,n", [(60, 16), (100, 16), (33, 9)])
+def test_large_batches_take_the_same_sums(pkg, m, n, dt):
+    """Up to 16 columns a large batch has half the threads a matrix: the same
+    lanes a pair, so sigma of a matrix is the same to the last rounding of its
+    norm (2 eps sigma_1) as in a batch of three."""
+    a = matrices((700, m, n), dt, m + n)
+    x = torch.from_numpy(a).to(DEV)
+    s = pkg.svd(x, precision="fp32")[1]
+    for k in (0, 350, 697):
+        u3, s3, v3 = pkg.svd(x[k:k + 3].contiguous(), precision="fp32")
+        assert float((s[k:k + 3] - s3).abs().max()) <= 2 * torch.finfo(s.dtype).eps * float(s3.max())
+        check(a[k:k + 3], u3, s3, v3)
+    u, s, vh = pkg.svd(x[:400].contiguous(), precision="fp32")
+    check(a[:400], u, s, vh)
