@@ -3,8 +3,8 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
 Workload (one step): the uneven batch of 8192 float32 matrices, n ~ U{8..64},
-m ~ U{n..2n}, entries N(0,1), seed 1, solved by ONE persistent launch
-replayed from a captured CUDA graph, in the mixed precision that meets
+m ~ U{n..2n}, entries N(0,1), seed 1, solved by one call of the library
+replayed as a captured CUDA graph, in the mixed precision that meets
 sigma-rel-err <= 1e-5 against FP64 LAPACK (checked on rank 0 after timing).
 The same batch is then timed in plain FP32 (the reference's arithmetic) for
 the mixed / plain factor.
@@ -62,16 +62,16 @@ METRIC = "Jacobi SVD matrices/s at sigma-rel-err<=1e-5 vs FP64 (uneven batch)"
 WORKLOAD = "uneven_batch_8192"
 COUNT = 8192
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one solve of
-# this workload, the four launches of the two size classes (rb32_kernel_t
-# 256- and 128-thread, rb64_kernel 512- and 256-thread), from one ncu capture
-# (those metrics only) of `bench.py --steps 1 --warmup 3 --no-cpu-baseline`.
-MEASURED_TRAFFIC_PER_SOLVE = 289.0e6
-TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the four solve launches of one step, "
-                  "captured at the library of commit 013b917 (the FP32 and FP64 solve kernels unchanged since)")
+# this workload, its five launches (factor_kernel, precondition_kernel,
+# refine_kernel, and the two that find nothing pending), from one ncu capture
+# (those metrics only) of `bench.py --steps 2 --warmup 3 --no-cpu-baseline`.
+MEASURED_TRAFFIC_PER_SOLVE = 361.0e6
+TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the five solve launches of one step, "
+                  "captured at the library of commit e7f7333")
 
 
-MIXED = ("mixed (FP32 sweeps, then FP64 sweeps from the Newton-Schulz orthogonalised V, "
-         "W = A V recomputed in FP64)")
+MIXED = ("mixed (FP32 sweeps on the Cholesky factor of the FP64 Gram, then V corrected in FP64, "
+         "W = A V from the exact input in FP64)")
 
 
 def workload_config(n_gpus, scaling="weak", precision=MIXED):
@@ -551,8 +551,8 @@ def run_ours(args, rank, world, local_rank):
             "fp_pipe": {"achieved_tflops": fp_tflops, "flop_per_launch": flop,
                         "measured_peaks": fp_peaks,
                         "frac_of_measured_fp32": fp_tflops / fp_peaks["fp32_tflops"],
-                        "note": "algorithmic flop = sum over matrices of sweeps x nt(nt-1)/2 (12 mt + 6 nt), FP32 "
-                                "and FP64 sweeps together, against the measured FP32 peak"},
+                        "note": "the reference's flop for the sweeps reported, nt(nt-1)/2 (12 mt + 6 nt) each, against "
+                                "the measured FP32 peak; the mixed solve's own sweeps run on the nt x nt factor"},
             "clocks": clocks.summary(), "gpu_launches": args.steps * plan.launches_per_solve,
             "e2e": {"value": e2e_value, "unit": "matrices/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "api": "batch.StreamedUneven (8 chunks of cost 1:2:4:4:4:4:2:1, two compute streams, copies overlapped "

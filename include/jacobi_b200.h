@@ -69,9 +69,9 @@ extern "C" {
 
 /* ---- arithmetic of the solve ------------------------------------------- */
 #define JB_PREC_NATIVE      0   /* sweeps in the input precision (f32 or f64)   */
-#define JB_PREC_MIXED       1   /* f32 input: FP32 sweeps, then Householder-QR
-                                   re-orthonormalised V and FP64 sweeps from
-                                   W = A V to the same tolerance; f64 input:
+#define JB_PREC_MIXED       1   /* f32 input: FP32 sweeps, then V corrected or
+                                   swept in FP64 from the exact input to the
+                                   same tolerance; f64 input:
                                    same as NATIVE                               */
 
 /* One matrix of an uneven batch.  A is row-major m x n at A + a_off.
@@ -120,14 +120,14 @@ JB_API int jb_svd_batched_f64(const double *A, double *U, double *S, double *Vh,
                        int32_t *sweeps, int32_t *status,
                        void *workspace, size_t workspace_bytes, void *stream);
 
-/* Uneven batch in ONE persistent launch per precision phase.  descs: `count`
+/* Uneven batch in a handful of launches.  descs: `count`
  * device descriptors; order: optional device permutation of [0, count)
  * giving the processing order (largest cost first balances the persistent
  * grid), or NULL.  max_m/max_n bound every descriptor (either orientation).
  * Workspace: jb_uneven_workspace_bytes(max_m, max_n, count, precision,
  * scratch_floats) bytes, where scratch_floats (JB_PREC_MIXED) covers every
- * descriptor's x_off + nt^2 (the FP32 V handed from the FP32 to the FP64
- * phase); a descriptor whose scratch does not fit gets JB_ST_BAD_DESC.
+ * descriptor's x_off + nt^2 (the FP32 factor and V handed between the
+ * phases); a descriptor whose scratch does not fit gets JB_ST_BAD_DESC.
  * Replaces a harness loop of svd(x, 'jacobi') over matrices of different
  * shapes. */
 JB_API size_t jb_uneven_workspace_bytes(int32_t max_m, int32_t max_n, int64_t count,

@@ -5,8 +5,8 @@ The reference can only batch equal shapes (svdbench/standalone/solvers.py:
 ``svd(x, 'jacobi')`` one call per matrix.  ``UnevenBatch`` replaces that loop:
 shapes are fixed when the plan is built (descriptors, output offsets, a
 largest-first processing order and the workspace are made once), and every
-solve is one call of ``jb_svd_uneven_f32`` -- one persistent kernel per
-precision phase and size class -- that can be captured in a CUDA graph and
+solve is one call of ``jb_svd_uneven_f32`` -- a handful of launches over the
+whole batch (launches_per_solve) -- that can be captured in a CUDA graph and
 replayed.
 """
 from __future__ import annotations

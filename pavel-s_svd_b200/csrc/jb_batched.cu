@@ -1,9 +1,11 @@
-// jb_batched.cu - persistent batched one-sided Jacobi SVD for sm_100a and
-// the C-ABI entry points declared in include/jacobi_b200.h.
+// jb_batched.cu - batched one-sided Jacobi SVD for sm_100a and the C-ABI
+// entry points declared in include/jacobi_b200.h.  (float64 and plain FP32:
+// group_kernel, jb_group.cuh; float32 in mixed precision: jb_mixed.cuh, then
+// the register kernels here for what that hands on.)
 //
 // One CTA solves one matrix at a time and then takes the next one from a
 // work list (an atomic ticket for uneven batches, a grid stride for equal
-// shapes), so an uneven batch of thousands of matrices is ONE launch and can
+// shapes), so an uneven batch of thousands of matrices is a few launches and can
 // be captured in a CUDA graph.  Everything of svd(a, 'jacobi') for one matrix
 // happens inside the CTA: finiteness scan, exact power-of-two scaling,
 // wide->tall transposition, sweeps with per-matrix convergence (no host

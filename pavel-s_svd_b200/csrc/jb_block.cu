@@ -233,12 +233,12 @@ __global__ void __launch_bounds__(kEigThreads) eig_kernel(const float *Gin, __nv
 // has met exactly once (the swaps reverse the order).  With positions fixed,
 // G and Q stay in registers: lane l holds rows RPT l .. RPT l + RPT - 1 and
 // warp w columns CB w .. CB w + CB - 1 (CB even: 4, 8 or 16 columns per warp,
-// n / CB warps; the outputs do not depend on CB).  Row pairs that straddle two lanes use warp
-// shuffles, column pairs that straddle two warps (odd rounds) one exchange
-// through shared memory.  Per round: warp 0 forms the angles from the
-// diagonal d and superdiagonal e (published in shared memory by their
-// owners), one barrier, rotations, (odd rounds: boundary exchange, one
-// barrier), new d / e, one barrier.
+// n / CB warps; the outputs do not depend on CB).  Row pairs that straddle two
+// lanes and column pairs that straddle two warps (odd rounds) are exchanged.
+// Per round: the first warps form the angles from the diagonal d and
+// superdiagonal e (published in shared memory by their owners), one barrier,
+// rotations, (odd rounds: boundary exchange, one barrier), new d / e, one
+// barrier.
 // DQ (deferred Q): Q is not accumulated here.  The angle threads record every
 // applied (c, s) as FP32 pairs, cs_out[(k * max_sweeps + sweep) * n + r][p]
 // by the pair's first position p, and the kernel writes the eigenvalues'

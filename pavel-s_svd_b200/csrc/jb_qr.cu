@@ -9,7 +9,7 @@
 //
 // All kernels compute in the input type, as the reference does.
 //
-// qr_panel_kernel: a cluster of 1 to 8 CTAs a matrix, each with a panel of rows
+// qr_panel_kernel: a cluster of 1 to 16 CTAs a matrix, each with a panel of rows
 // in shared memory.  Per column j one reduction over the rows gives ||x||^2 and
 // x^H y_c for all later columns at once (v = x / (alpha - beta), so v^H y_c =
 // y_jc + x^H y_c / (alpha - beta)): one cluster barrier a column, every CTA
@@ -20,7 +20,7 @@
 // CTAs 0.05 ms, 1.62 ms by one CTA through global memory; 256 x (256 x 16) FP32
 // 0.02 ms, 0.07 ms.
 //
-// qr_kernel, cqr_kernel (matrices whose panels do not fit 8 SMs): one CTA per
+// qr_kernel, cqr_kernel (matrices whose panels do not fit 16 SMs): one CTA per
 // matrix (grid-stride over the batch).  The work area is the matrix (m x n,
 // column-major: a warp walks a column with unit stride) whose lower part
 // keeps the reflectors, and Q (m x n, column-major); in shared memory when

@@ -6,8 +6,8 @@ and messages, same output contract (U (...,m,k), s (...,k), Vh (...,k,n);
 ``None`` for U and Vh with ``values_only``; the info dict with ``return_info``).
 For 'jacobi' the numeric work is ONE call of the sm_100a batched solver
 (``jb_svd_batched_f32`` / ``_f64``, ``_c64`` / ``_c128`` for complex input:
-one persistent kernel, two for the FP32 and FP64 phases of the mixed
-precision); the host reads back only the per-matrix status and sweep words
+one kernel, or the factor, precondition and refine kernels of the mixed
+precision with two more for the matrices these hand on); the host reads back only the per-matrix status and sweep words
 to raise the reference's errors.
 
 Differences, by design:
@@ -16,8 +16,8 @@ Differences, by design:
     (svdbench/algorithms.py:12-13) instead of running elsewhere: there is no
     CPU fallback.
   * ``precision`` option for float32 input: ``'mixed'`` (default) runs FP32
-    sweeps and then FP64 sweeps from the Householder re-orthonormalised V, so
-    singular values meet a 1e-5 relative bound against FP64 LAPACK even where
+    sweeps on the Cholesky factor of the FP64 Gram and corrects V in FP64
+    from the exact input until the reference's test passes, so singular values meet a 1e-5 relative bound against FP64 LAPACK even where
     FP32 arithmetic alone does not; ``'fp32'`` is the plain FP32 Jacobi of the
     reference.  float64 input always runs in FP64.
   * Scaling by a power of two (exact) instead of max|a| (solvers.py:294-295).
@@ -303,8 +303,8 @@ def _qr_first(a):
 
 
 def _tall_svd(a, full_matrices, values_only, return_info, rank, precision, opts):
-    """'jacobi' on matrices taller than the register and large-tile kernels
-    (real) or the shared-memory work area (complex) take (QR_FIRST_ROWS).  A
+    """'jacobi' on matrices taller than the register kernels take
+    (QR_FIRST_ROWS).  A
     one-sided Jacobi sees its matrix only through the column Gram W^H W, and
     R^H R of a QR equals it, so the Jacobi of the small factor R rotates as
     the Jacobi of A would: the same V, sigma and sweeps in exact arithmetic,
@@ -315,8 +315,9 @@ def _tall_svd(a, full_matrices, values_only, return_info, rank, precision, opts)
         tall view (the conjugate transpose of a wide matrix), in FP64 for
         the mixed precision of float32 input (the 1e-5 sigma bound of that
         mode rests on FP64 arithmetic from the exact input); a batch of
-        fewer large matrices than SMs runs it as TSQR (qr.tsqr: row tiles in
-        parallel, about one per SM, then the reduction tree; TSQR_WORK);
+        fewer matrices than SMs that are too large for its on-chip panels
+        runs it as TSQR (qr.tsqr: row tiles in parallel, about one per SM,
+        then the reduction tree; TSQR_WORK);
       * the Jacobi of R by the batched kernels, with the input dtype's
         tolerance (10 eps, primitives.py:325); for mixed float32 with more
         than 64 columns R is rounded to FP32 and solved in the mixed mode,
