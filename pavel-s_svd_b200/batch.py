@@ -202,13 +202,15 @@ class UnevenBatch:
         # and FP64 register kernels for what these leave) after the factor
         # kernel (one CTA a matrix), an FP32 one two when the batch is wider
         # than 32 (widths above and up to 32 columns run in CTAs of different
-        # sizes).  launches_per_solve counts every kernel.
+        # sizes).  launches_per_solve counts every kernel (a mixed batch of more
+        # than two matrices an SM refines widths above and up to 32 in a launch each).
         phases = 2 if self.precision == N.PREC_MIXED else 1
         register = (not self.launch_choice.flags & (N.ROUND_ROBIN | N.BLOCK_WIDTH_8) and self.max_m <= 128
                     and self.max_n <= 64)
         split = self.max_n > 32 and not self.launch_choice.flags & N.ONE_SIZE_CLASS
         self.kernels_per_solve = phases * (2 if register and (phases == 2 or split) else 1)
-        self.launches_per_solve = self.kernels_per_solve + (1 if register and phases == 2 else 0)
+        both = split and self.count > 2 * lib.jb_device_sm_count()
+        self.launches_per_solve = self.kernels_per_solve + (1 + both if register and phases == 2 else 0)
 
     # -- solving ----------------------------------------------------------------
     def launch(self, a_flat: torch.Tensor, stream=None):

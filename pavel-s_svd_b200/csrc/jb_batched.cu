@@ -1284,7 +1284,7 @@ static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsign
         p.n_pending = (int *)ws + 4;
         p.maxd = pl.d32;
         p.region_cap = pl.reg32;
-        const size_t s0 = fac_smem<64>(pl.d.mt, pl.d.nt), s1 = pre_smem(pl.d.nt), s2 = ref_smem(pl.d.mt, pl.d.nt);
+        const size_t s0 = fac_smem<64>(pl.d.mt, pl.d.nt), s1 = pre_smem(pl.d.nt);
         // one CTA a matrix, largest first: no state is kept from one to the next
         if ((rc = occupancy_grid(factor_kernel<kFacT>, kFacT, s0, p.count, grid))) return rc;
         factor_kernel<kFacT><<<(unsigned)(p.count < kMaxGrid ? p.count : kMaxGrid), kFacT, s0, st>>>(p);
@@ -1292,9 +1292,28 @@ static int launch_reg(Params &p, const Plan &pl, int elem, int precision, unsign
         if ((rc = occupancy_grid(precondition_kernel<kPreT>, kPreT, s1, p.count, grid))) return rc;
         precondition_kernel<kPreT><<<(unsigned)grid, kPreT, s1, st>>>(p);
         if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
-        if ((rc = occupancy_grid(refine_kernel, kRefT, s2, p.count, grid))) return rc;
-        refine_kernel<<<(unsigned)grid, kRefT, s2, st>>>(p);
-        if (cudaGetLastError() != cudaSuccess) return JB_ECUDA;
+        auto refine = [&](auto kern, int threads, int nt, int cls, int counter) -> int {
+            const size_t smem = ref_smem(pl.d.mt, nt);
+            if ((rc = occupancy_grid(kern, threads, smem, p.count, grid))) return rc;
+            p.cls = cls;
+            p.counter2 = (int *)ws + counter;
+            kern<<<(unsigned)grid, threads, smem, st>>>(p);
+            p.cls = 0;
+            return cudaGetLastError() == cudaSuccess ? JB_OK : JB_ECUDA;
+        };
+        // At most 32 columns: half the threads and a third of the shared memory, so
+        // more matrices an SM (2048 matrices, us: 16 x 8 73 -> 46, 32 x 16 100 -> 68, 64 x
+        // 32 169 -> 141, 128 x 32 229 -> 206).  Few matrices keep the threads, tall ones
+        // longer (300 of 100 x 20: 39 us, 41 with half; of 32 x 16 28 and 23).  An uneven
+        // batch gives each width class its launch (8192 matrices, the whole solve: 2.175
+        // -> 2.150 ms).
+        const int64_t sms = sm_count();
+        const bool narrow = pl.d.nt <= kNarrowN && p.count > (pl.d.mt <= 64 ? 2 : 8) * sms;
+        const bool both = split && p.count > 2 * sms;
+        if (narrow) rc = refine(refine_kernel<kRefNarrowT>, kRefNarrowT, pl.d.nt, 0, 1);
+        else rc = refine(refine_kernel<kRefT>, kRefT, pl.d.nt, both ? 1 : 0, 1);
+        if (!rc && both) rc = refine(refine_kernel<kRefNarrowT>, kRefNarrowT, kNarrowN, 2, 3);
+        if (rc) return rc;
         p.pending = 1;
         p.counter = (int *)ws + 5;
         p.counter2 = (int *)ws + 6;

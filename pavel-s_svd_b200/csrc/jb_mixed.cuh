@@ -40,7 +40,7 @@ namespace jb {
 
 constexpr int kPending = -1;   // status: left to the register kernels
 constexpr int kHanded = -2;    // status: FP32 sweeps done by rb32, FP64 phase due
-constexpr int kFacT = 128, kPreT = 64, kRefT = 256;
+constexpr int kFacT = 128, kPreT = 64, kRefT = 256, kRefNarrowT = 128;
 // A pivot below kPivotCut times the largest diagonal of G (a singular value
 // ratio of about 3e-6) is left to the register kernels: FP64 rounding of G
 // no longer resolves it well enough for a start.
@@ -697,7 +697,7 @@ __host__ __device__ inline size_t ref_smem(int mt, int nt) {
 // x[i * sr + k * sk], Y(k, j) at y[j * ldy + k].  C is written once every
 // warp is done reading: it may take X's or Y's place.  Rows and columns of a
 // block past the end repeat the last tile; their results are not stored.
-template <int NB, int S, bool ADD, typename TX>
+template <int NB, int S, int NW, bool ADD, typename TX>
 __device__ __forceinline__ void ref_mul(const TX *x, int sr, int sk, const double *y, int ldy, double *C, int ldc,
                                         int k8, int mt8, int nt8) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
@@ -705,7 +705,7 @@ __device__ __forceinline__ void ref_mul(const TX *x, int sr, int sk, const doubl
     double acc[S][2][NB][2];
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-        const int blk = warp + 8 * s;
+        const int blk = warp + NW * s;
 #pragma unroll
         for (int b = 0; b < NB; ++b)
             acc[s][0][b][0] = acc[s][0][b][1] = acc[s][1][b][0] = acc[s][1][b][1] = 0.0;
@@ -731,7 +731,7 @@ __device__ __forceinline__ void ref_mul(const TX *x, int sr, int sk, const doubl
     __syncthreads();
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-        const int blk = warp + 8 * s;
+        const int blk = warp + NW * s;
         if (blk < blocks) {
             const int tr = 2 * (blk % bm), tc = NB * (blk / bm);
 #pragma unroll
@@ -748,14 +748,14 @@ __device__ __forceinline__ void ref_mul(const TX *x, int sr, int sk, const doubl
 }
 // W = A V with A staged in W's place, and V <- V + V N, with the block width
 // (3 or 4 column tiles) that leaves the fewest idle.
-template <int NB>
+template <int NB, int NW>
 __device__ __forceinline__ void ref_w(const float *As, Stage st, const double *V, int ldv, double *W, int ldw, int mt8,
                                       int nt8) {
-    ref_mul<NB, 2, false>(As, st.sr, st.sk, V, ldv, W, ldw, 8 * nt8, mt8, nt8);
+    ref_mul<NB, 2, NW, false>(As, st.sr, st.sk, V, ldv, W, ldw, 8 * nt8, mt8, nt8);
 }
-template <int NB>
+template <int NB, int NW>
 __device__ __forceinline__ void ref_v(double *V, int ldv, const double *Nm, int nt8) {
-    ref_mul<NB, 1, true>(V, 1, ldv, Nm, ldv, V, ldv, 8 * nt8, nt8, nt8);
+    ref_mul<NB, 1, NW, true>(V, 1, ldv, Nm, ldv, V, ldv, 8 * nt8, nt8, nt8);
 }
 __device__ __forceinline__ bool ref_three(int nt8) { return nt8 == 3 || nt8 == 5 || nt8 == 6; }
 
@@ -796,7 +796,11 @@ __device__ __forceinline__ double ref_angle(double d, double a) {
     return d < 0.0 ? -(double)t : (double)t;
 }
 
-__global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
+// THREADS 256 (two matrices an SM at 128 x 64), or 128 for matrices of at most 32
+// columns (four or more an SM).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) refine_kernel(Params p) {
+    constexpr int NW = THREADS / 32;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_idx;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
@@ -810,6 +814,7 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
         bool wide;
         {
             const jb_matrix_desc d = desc_of(p, mat);
+            if (!class_takes(d, p.cls)) continue;   // the other size class's launch refines it
             wide = d.m < d.n;
             mt = wide ? d.n : d.m;
             nt = wide ? d.m : d.n;
@@ -825,7 +830,7 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
         const Stage sg = stage_of(wide, g.m8, g.n8);
         {
             const float *x = p.x32 + desc_of(p, mat).x_off;
-            for (int c = warp; c < g.n8; c += kRefT / 32)
+            for (int c = warp; c < g.n8; c += NW)
                 for (int i = lane; i < g.n8; i += 32)
                     V[c * ldv + i] = (c < nt && i < nt) ? (double)x[c * nt + i] : 0.0;
         }
@@ -836,16 +841,16 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
         for (; pass <= most; ++pass) {
             {
                 const jb_matrix_desc d = desc_of(p, mat);
-                stage_tall((const float *)p.A + d.a_off, d, g.m8, g.n8, sg, As, kRefT);
+                stage_tall((const float *)p.A + d.a_off, d, g.m8, g.n8, sg, As, THREADS);
             }
             __syncthreads();
-            if (ref_three(nt8)) ref_w<3>(As, sg, V, ldv, W, ldw, mt8, nt8);
-            else ref_w<4>(As, sg, V, ldv, W, ldw, mt8, nt8);
+            if (ref_three(nt8)) ref_w<3, NW>(As, sg, V, ldv, W, ldw, mt8, nt8);
+            else ref_w<4, NW>(As, sg, V, ldv, W, ldw, mt8, nt8);
             __syncthreads();
             double h[3][2][2], e[3][2][2];
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
-                const int job = warp + 8 * s;
+                const int job = warp + NW * s;
                 if (job >= jobs) continue;
                 int tr, tc;
                 job_place(job, tr, tc);
@@ -869,7 +874,7 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
             int need = 0;
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
-                const int job = warp + 8 * s;
+                const int job = warp + NW * s;
                 if (job >= jobs) continue;
                 int tr, tc;
                 job_place(job, tr, tc);
@@ -893,7 +898,7 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
             int wild = 0;
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
-                const int job = warp + 8 * s;
+                const int job = warp + NW * s;
                 if (job >= jobs) continue;
                 int tr, tc;
                 job_place(job, tr, tc);
@@ -923,7 +928,7 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
             if (__syncthreads_or(wild)) { pass = most; break; }
             // second-order term on the diagonal: -sum_i K_ij^2 / 2 (an isolated
             // close pair has an angle far above all others)
-            for (int j = warp; j < nt; j += kRefT / 32) {
+            for (int j = warp; j < nt; j += NW) {
                 double sum = 0.0;
                 for (int i = lane; i < nt; i += 32) {
                     const double k = 0.5 * (Nm[j * ldv + i] - Nm[i * ldv + j]);
@@ -933,8 +938,8 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
                 if (lane == 0) Nm[j * ldv + j] -= 0.5 * sum;
             }
             __syncthreads();
-            if (ref_three(nt8)) ref_v<3>(V, ldv, Nm, nt8);
-            else ref_v<4>(V, ldv, Nm, nt8);
+            if (ref_three(nt8)) ref_v<3, NW>(V, ldv, Nm, nt8);
+            else ref_v<4, NW>(V, ldv, Nm, nt8);
         }
         // sigma, the stable descending order and the cut (primitives.py:356-366)
         int st = JB_ST_OK;
@@ -983,7 +988,7 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
                 const double *X = wide ? V : W;
                 const int ldl = wide ? ldv : ldw, rows = wide ? nt : mt;
                 const int r8 = (d.rank + 7) >> 3;
-                for (int blk = warp; blk < ((rows + 3) >> 2) * r8; blk += kRefT / 32) {
+                for (int blk = warp; blk < ((rows + 3) >> 2) * r8; blk += NW) {
                     const int r = (blk % r8) * 8 + (lane & 7), i = (blk / r8) * 4 + (lane >> 3);
                     if (r < d.rank && i < rows) {
                         const int c = perm[r];
@@ -994,7 +999,7 @@ __global__ void __launch_bounds__(kRefT, 2) refine_kernel(Params p) {
                 }
                 const double *Y = wide ? W : V;
                 const int ldr = wide ? ldw : ldv, cols = wide ? mt : nt;
-                for (int r = warp; r < d.rank; r += kRefT / 32) {
+                for (int r = warp; r < d.rank; r += NW) {
                     const int c = perm[r];
                     const double f = wide ? dh[c] : 1.0;
                     for (int i = lane; i < cols; i += 32) {
@@ -1130,7 +1135,7 @@ __global__ void __launch_bounds__(kRefT, 1) refine_large_kernel(Params p) {
             }
             asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
             __syncthreads();
-            ref_mul<4, 1, false>(As, sg.sr, sg.sk, V, ldv, W, ldw, g.n8, kLgRows / 8, nt8);
+            ref_mul<4, 1, kRefT / 32, false>(As, sg.sr, sg.sk, V, ldv, W, ldw, g.n8, kLgRows / 8, nt8);
             __syncthreads();
             if (rows > 0) {
                 double *mine = part + (size_t)rank * nblk * 256;

@@ -119,3 +119,40 @@ def test_errors(pkg):
         with pytest.raises(ValueError, match="NaN or infinity"):
             pkg.svd(b)
     assert bool(torch.isfinite(pkg.svd(a)[1]).all())
+
+
+@pytest.mark.parametrize("n,m", [(1, 1), (8, 17), (16, 16), (17, 64), (20, 65), (24, 100), (31, 33), (32, 64), (32, 128)])
+@pytest.mark.parametrize("wide", [False, True], ids=["tall", "wide"])
+def test_large_batches_of_narrow_matrices(pkg, n, m, wide):
+    """At most 32 columns in a batch of many matrices an SM: the refinement
+    with half the threads, at the edges of its tiles; the same sums, so sigma is
+    that of a batch of three to its rounding."""
+    rng = np.random.default_rng(n + m)
+    a = rng.standard_normal((1300, m, n)).astype(np.float32)
+    if wide:
+        a = np.ascontiguousarray(np.swapaxes(a, 1, 2))
+    x = torch.from_numpy(a).to(DEV)
+    u, s, vh = pkg.svd(x)
+    pick = list(range(0, 1300, 61))
+    check(a[pick], u[pick], s[pick], vh[pick])
+    s3 = pkg.svd(x[610:613].contiguous())[1]
+    assert float(((s[610:613] - s3).abs() / s3[:, :1]).max()) <= 2.0 ** -23
+
+
+def test_uneven_width_classes(B):
+    """An uneven batch of more than two matrices an SM: widths above and up to 32
+    are refined by launches of their own; every matrix once."""
+    rng = np.random.default_rng(12)
+    n = rng.integers(1, 65, 700)
+    m = np.minimum(n * rng.integers(1, 3, 700) + rng.integers(0, 3, 700), 128)
+    m = np.maximum(m, n)
+    plan = B.UnevenBatch(m, n, DEV)
+    mats = [rng.standard_normal((int(p), int(q))).astype(np.float32) for p, q in zip(m, n)]
+    flat = np.zeros(max(int(o) + t.size for t, o in zip(mats, plan.a_off)), np.float32)
+    for t, o in zip(mats, plan.a_off):
+        flat[int(o):int(o) + t.size] = t.ravel()
+    plan.launch(torch.from_numpy(flat).to(DEV))
+    torch.cuda.synchronize()
+    assert int(plan.info[1].abs().max()) == 0
+    for i in range(0, 700, 9):
+        check(mats[i], *plan.result(i))
